@@ -134,6 +134,7 @@ struct StepBuffers {
     float* potential;        // walk potential by body id (GBH_FLAG_STORE_POTENTIAL)
     uint32_t prec;           // 1: this step runs the precision form
     uint32_t merge;          // 1: this step emits merge tasks (mode GBH_MODE_MERGE)
+    uint32_t collide;        // 1: this step resolves contacts in the walk (mode GBH_MODE_COLLISION)
     // compaction scratch
     uint32_t* tile_dead;
     float* tile_aabb;

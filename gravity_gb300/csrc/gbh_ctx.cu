@@ -95,6 +95,7 @@ StepBuffers ctx_buffers(const gbh_ctx* c) {
     b.potential = c->potential;
     b.prec = (c->params_valid && c->params_host.precision_mode == GBH_PRECISION_COMPENSATED && c->pos64[0]) ? 1u : 0u;
     b.merge = (c->params_valid && c->params_host.merging_collision_or_neither == GBH_MODE_MERGE) ? 1u : 0u;
+    b.collide = (c->params_valid && c->params_host.merging_collision_or_neither == GBH_MODE_COLLISION) ? 1u : 0u;
     b.tile_dead = c->tile_dead;
     b.tile_aabb = c->tile_aabb;
     b.hist = c->hist;

@@ -5,25 +5,458 @@
 // thread per body with a private 64-entry stack, a full 80-byte node gather per
 // visit and a global atomic per opened node.
 //
-// Here a warp walks for 32 consecutive bodies of the Morton order (spatial
-// neighbours) with ONE shared stack.  Each stack entry carries the mask of
-// lanes that opened its parent; a lane evaluates only the entries that carry
-// its bit, so every lane visits exactly the nodes its own reference walk would
-// visit, in the same depth-first order (childB evaluated before childA), and
-// accumulates its terms in that order.
+// Both kernels here give a warp 32 consecutive bodies of the Morton order
+// (spatial neighbours) and ONE shared stack of (node, mask of the lanes whose
+// own walk opened the node), so every lane interacts with exactly the nodes
+// that its own reference walk would interact with.  The children of an opened
+// node come as one 64-byte ChildPair record.
 //
-// Node data travel with the traversal: opening a node reads its ChildPair
-// (the 32-byte records of both children, one 64-byte warp-uniform load);
-// childB is evaluated next straight from registers and childA is pushed, with
-// its record, on the warp's shared-memory stack.  A visit therefore costs no
-// global load of its own, and one load serves two visits.  The per-node debug
-// atomic of the reference (bh_force.comp:72) becomes one add per warp.
+//   k_walk_plain     gravity and merges, FP32 and the precision form.  Up to 16
+//                    opened nodes are popped at once and their children, one
+//                    per lane, classified against the box of the
+//                    warp's bodies; only the children whose acceptance differs
+//                    inside the box get the per-body test.
+//   k_walk_collide   collision mode, where a contact changes the body (position
+//                    and velocity) in the reference's depth-first order, which
+//                    the next tests and forces use: one node at a time in that
+//                    order (childB before childA).
 //
 // Arithmetic: the MAC is the reference's (half side * invDist < theta, with
 // invDist from the softened distance); the force sum uses fused multiply-adds
 // (G m inv^3 r accumulated with FMA), which is within 1e-7 relative of the
 // reference's operation order.
 #include "gbh_common.cuh"
+
+// ---- gravity and merges ----------------------------------------------------------
+//
+// What bounds it: instruction issue.  A walk of one node at a time per warp
+// (the collision kernel below) spends about 46 instructions on every node that
+// any of its 32 bodies meets, with the 20-30% of the lanes active whose own
+// walk meets it: 66,600 instructions per warp on a 4,194,304-body mixture.  Of
+// the nodes that a warp meets (976 on a 1,048,576-body mixture at theta 0.5)
+// two thirds are accepted or opened by all of the warp's bodies alike, which
+// one lane can tell from the box of the 32 bodies.  So a round pops up to 16
+// opened nodes and classifies their 32 children, one per lane (about 60
+// instructions for all of them); the force of a node on the bodies of its
+// mask then takes 17 instructions, and a node that the box leaves undecided
+// 23, force included.  A finer box (per 16, 8 or 4 bodies) leaves 309, 290 or
+// 267 of the 327 undecided nodes of a warp and was not worth its tests; 64
+// bodies per warp leave more undecided tests per body (485 against 654 for two
+// warps of 32, at twice the work each).
+// Walk stage, ms, before and after: 4,194,301-body mixture at theta 0.5 8.04 ->
+// 3.14; 2,097,152-body galaxy pair, precision form, 6.43 -> 2.50; 65,536-body
+// Plummer sphere 0.289 -> 0.092; 1,024 bodies 0.131 -> 0.045; 1,048,576-body
+// merge state at theta 0.7 0.457 -> 0.352.  Popping 32 nodes and classifying
+// both children of each in turn: 4.12 ms on the mixture.
+
+#define PW_THREADS 128
+#define PW_WARPS (PW_THREADS / 32)
+#define PW_LIST 64     // below 32 entries wait, one append adds up to 32
+#define PW_LOW 120     // above this many stack entries the walk turns depth-first
+#define PW_STACK 288   // PW_LOW + 63 (one batch) + 96 (a depth-first descent: 63 key + 30 tie-break levels)
+#define PW_BLOCKS 8     // resident blocks per SM (64 registers): 3.14 ms where 6 take 3.28, 5 3.62, 10 3.20
+
+enum PlainForm { PF_FP32 = 0, PF_PREC = 1, PF_MERGE = 2 };
+
+// per-warp shared memory
+template <int FORM>
+struct PlainSmem {
+    float4 a_cm[PW_LIST];     // entries every lane of the mask interacts with: centre of mass, G x mass
+    float4 x_cm[PW_LIST];     // nodes to test body by body
+    uint2 x_half_mask[PW_LIST];
+    uint32_t x_id[PW_LIST];
+    uint32_t a_mask[PW_LIST];
+    uint2 stack[PW_STACK];    // (opened node's internal index, lanes that opened it)
+    // merge and precision forms: leaves apart (mask; radius and slot, or residual)
+    float4 l_cm[FORM == PF_FP32 ? 1 : PW_LIST];
+    float4 l_lo[FORM == PF_PREC ? PW_LIST : 1];
+    uint32_t l_mask[FORM == PF_FP32 ? 1 : PW_LIST];
+    float l_rad[FORM == PF_MERGE ? PW_LIST : 1];
+    uint32_t l_id[FORM == PF_MERGE ? PW_LIST : 1];
+};
+
+// PREC: the precision form.  Offsets are formed from the FP32 position and
+// its FP32 residual (leaf_lo), r = (x_j - x_b) + (lo_j - lo_b) for a leaf and
+// (com - x_b) - lo_b for a node, and the leaf terms are summed with Kahan
+// compensation apart from the node terms.  Gravity only.
+template <int FORM>
+__global__ __launch_bounds__(PW_THREADS, PW_BLOCKS) void k_walk_plain(StepBuffers b) {
+    constexpr bool PREC = FORM == PF_PREC;
+    constexpr bool MERGE = FORM == PF_MERGE;
+    __shared__ PlainSmem<FORM> s_warp[PW_WARPS];
+    __shared__ unsigned long long s_inter, s_opened;
+    __shared__ uint32_t s_depth;
+    const uint32_t n = b.st->n_new;
+    const uint32_t N = b.N;
+    const uint32_t lane = lane_id(), w = threadIdx.x >> 5;
+    const uint32_t base = (blockIdx.x * PW_WARPS + w) * 32;
+    const uint32_t g = base + lane;
+    if (blockIdx.x == 0 && threadIdx.x == 0) b.st->sorted_valid = 1u;  // the update below fills sorted_pm
+    uint32_t s_lo, s_hi;
+    shard_slots(b, n, s_lo, s_hi);
+    const uint32_t block_first = blockIdx.x * PW_THREADS;
+    if (block_first >= n || block_first + PW_THREADS <= s_lo || block_first >= s_hi) return;
+    if (threadIdx.x == 0) {
+        s_inter = s_opened = 0ull;
+        s_depth = 0u;
+    }
+    __syncthreads();
+    // every live body of the warp walks, so that a body's sums do not depend on
+    // the sharding; only the shard's own bodies count, merge and are updated
+    const bool active = g < n;
+    const bool owned = active && g >= s_lo && g < s_hi;
+    const uint32_t everyone = __ballot_sync(0xffffffffu, active);
+    const uint32_t owners = __ballot_sync(0xffffffffu, owned);
+    const gbh_step_params* P = b.params;
+    const gbh_sim_values* sim = b.sim;
+    const float G = sim->gravitational_constant;
+    const float soft = P->softening, theta = P->theta;
+    PlainSmem<FORM>& S = s_warp[w];
+    const uint32_t bit = 1u << lane;
+
+    const uint32_t bi = active ? b.idx_in[g] : 0u;
+    const float4 pm = active ? b.leaf_pm[g] : make_float4(0.f, 0.f, 0.f, 0.f);
+    const float my_rad = (MERGE && active) ? b.leaf_rad[g] : 0.0f;
+    const float4 lo_b = (PREC && active) ? b.leaf_lo[g] : make_float4(0.f, 0.f, 0.f, 0.f);
+    const bool want_pot = (P->flags & GBH_FLAG_STORE_POTENTIAL) && b.potential;
+
+    // box of the warp's bodies; `boxed` is false when it cannot speak for all
+    // of them (positions that are not finite, parameters outside the range the
+    // margins below are made for): then every node is tested body by body
+    float mnx = active ? pm.x : 3.0e38f, mny = active ? pm.y : 3.0e38f, mnz = active ? pm.z : 3.0e38f;
+    float mxx = active ? pm.x : -3.0e38f, mxy = active ? pm.y : -3.0e38f, mxz = active ? pm.z : -3.0e38f;
+    float grp_rad = my_rad;
+    float res = PREC ? fmaxf(fabsf(lo_b.x), fmaxf(fabsf(lo_b.y), fabsf(lo_b.z))) : 0.0f;
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) {
+        mnx = fminf(mnx, __shfl_xor_sync(0xffffffffu, mnx, o));
+        mny = fminf(mny, __shfl_xor_sync(0xffffffffu, mny, o));
+        mnz = fminf(mnz, __shfl_xor_sync(0xffffffffu, mnz, o));
+        mxx = fmaxf(mxx, __shfl_xor_sync(0xffffffffu, mxx, o));
+        mxy = fmaxf(mxy, __shfl_xor_sync(0xffffffffu, mxy, o));
+        mxz = fmaxf(mxz, __shfl_xor_sync(0xffffffffu, mxz, o));
+        if (MERGE) grp_rad = fmaxf(grp_rad, __shfl_xor_sync(0xffffffffu, grp_rad, o));
+        if (PREC) res = fmaxf(res, __shfl_xor_sync(0xffffffffu, res, o));
+    }
+    if (PREC) {
+        // the bodies' residuals, and the rounding of the widened corners
+        const float pad = 2.0f * res + 2.4e-7f * fmaxf(fmaxf(fmaxf(fabsf(mnx), fabsf(mxx)), fmaxf(fabsf(mny), fabsf(mxy))),
+                                                       fmaxf(fabsf(mnz), fabsf(mxz)));
+        mnx = mnx - pad;
+        mny = mny - pad;
+        mnz = mnz - pad;
+        mxx = mxx + pad;
+        mxy = mxy + pad;
+        mxz = mxz + pad;
+    }
+    const bool boxed = !__any_sync(0xffffffffu, active && !(finite3(pm.x, pm.y, pm.z) && finite3(lo_b.x, lo_b.y, lo_b.z))) &&
+                       theta >= 1e-3f && theta <= 1e3f && soft >= 0.0f && soft <= 1e30f;
+    // theta^2 with margins of 1e-5: the body's own test (a reciprocal square
+    // root of at most 2 ulp error and six more roundings, together below 1e-6)
+    // decides the same way wherever the box test decides
+    const float t2_accept = theta * theta * 0.99999f, t2_open = theta * theta * 1.00001f;
+
+    float ax = 0.0f, ay = 0.0f, az = 0.0f, pot = 0.0f;
+    float nx_ = 0.0f, ny_ = 0.0f, nz_ = 0.0f, np_ = 0.0f;  // PREC: leaf terms (Kahan)
+    float cx_ = 0.0f, cy_ = 0.0f, cz_ = 0.0f, cp_ = 0.0f;
+    uint32_t inter = 0, opened = 0;  // this lane's share of the warp's counts
+    uint32_t sp = 0, max_sp = 0, an = 0, xn = 0, ln = 0;
+    bool overflow = false;
+
+    // push the opened nodes of the lanes with mask != 0 (warp-collective)
+    auto push = [&](uint32_t id, uint32_t mask) {
+        const uint32_t bo = __ballot_sync(0xffffffffu, mask != 0u);
+        const uint32_t cnt = __popc(bo);
+        if (sp + cnt > PW_STACK) {
+            overflow = true;
+            return;
+        }
+        if (mask) S.stack[sp + __popc(bo & lanemask_lt())] = make_uint2(id - N, mask);
+        opened += __popc(mask & owners);
+        sp += cnt;
+    };
+    // forces of list A's last `cnt` entries on the lanes of each entry's mask
+    auto flush_a = [&](uint32_t cnt) {
+        __syncwarp();
+        an -= cnt;
+        const float4* cmv = S.a_cm + an;
+        const uint32_t* mv = S.a_mask + an;
+        if (want_pot) {
+            for (uint32_t j = 0; j < cnt; ++j) {
+                const float4 c = cmv[j];
+                float rx = c.x - pm.x, ry = c.y - pm.y, rz = c.z - pm.z;
+                if (PREC) rx = rx - lo_b.x, ry = ry - lo_b.y, rz = rz - lo_b.z;
+                const float inv = rsqrtf(__fmaf_rn(rz, rz, __fmaf_rn(ry, ry, __fmaf_rn(rx, rx, soft))));
+                if (mv[j] & bit) {
+                    const float f = c.w * (inv * inv * inv);
+                    ax = __fmaf_rn(f, rx, ax);
+                    ay = __fmaf_rn(f, ry, ay);
+                    az = __fmaf_rn(f, rz, az);
+                    pot = __fmaf_rn(-c.w, inv, pot);
+                }
+            }
+        } else {
+#pragma unroll 4
+            for (uint32_t j = 0; j < cnt; ++j) {
+                const float4 c = cmv[j];
+                float rx = c.x - pm.x, ry = c.y - pm.y, rz = c.z - pm.z;
+                if (PREC) rx = rx - lo_b.x, ry = ry - lo_b.y, rz = rz - lo_b.z;
+                const float inv = rsqrtf(__fmaf_rn(rz, rz, __fmaf_rn(ry, ry, __fmaf_rn(rx, rx, soft))));
+                const float f = c.w * (inv * inv * inv);
+                if (mv[j] & bit) {
+                    ax = __fmaf_rn(f, rx, ax);
+                    ay = __fmaf_rn(f, ry, ay);
+                    az = __fmaf_rn(f, rz, az);
+                }
+            }
+        }
+        __syncwarp();
+    };
+    // the same for the leaves of the merge and precision forms
+    auto flush_l = [&](uint32_t cnt) {
+        __syncwarp();
+        ln -= cnt;
+        for (uint32_t j = 0; j < cnt; ++j) {
+            const float4 c = S.l_cm[ln + j];
+            const bool me = S.l_mask[ln + j] & bit;
+            float rx = c.x - pm.x, ry = c.y - pm.y, rz = c.z - pm.z;
+            if (PREC) {
+                const float4 lo_j = S.l_lo[ln + j];
+                rx = rx + (lo_j.x - lo_b.x);
+                ry = ry + (lo_j.y - lo_b.y);
+                rz = rz + (lo_j.z - lo_b.z);
+            }
+            const float inv = rsqrtf(__fmaf_rn(rz, rz, __fmaf_rn(ry, ry, __fmaf_rn(rx, rx, soft))));
+            const float f = c.w * (inv * inv * inv);
+            if (me) {
+                if (PREC) {
+                    kahan_add(nx_, cx_, f * rx);
+                    kahan_add(ny_, cy_, f * ry);
+                    kahan_add(nz_, cz_, f * rz);
+                    if (want_pot) kahan_add(np_, cp_, -c.w * inv);
+                } else {
+                    ax = __fmaf_rn(f, rx, ax);
+                    ay = __fmaf_rn(f, ry, ay);
+                    az = __fmaf_rn(f, rz, az);
+                    if (want_pot) pot = __fmaf_rn(-c.w, inv, pot);
+                }
+            }
+        }
+        if (MERGE) {
+            // lane j screens leaf j: within reach of the box (its radius plus
+            // the warp's largest, a margin for rounding)?  Only those get the
+            // per-body overlap test (bh_force.comp:109-112).
+            bool near = false;
+            if (lane < cnt) {
+                const float4 c = S.l_cm[ln + lane];
+                const float dx = fmaxf(fmaxf(mnx - c.x, c.x - mxx), 0.0f);
+                const float dy = fmaxf(fmaxf(mny - c.y, c.y - mxy), 0.0f);
+                const float dz = fmaxf(fmaxf(mnz - c.z, c.z - mxz), 0.0f);
+                const float reach = S.l_rad[ln + lane] + grp_rad;
+                near = dx * dx + dy * dy + dz * dz <= 1.001f * (reach * reach);
+            }
+            uint32_t m = __ballot_sync(0xffffffffu, near);
+            while (m) {
+                const uint32_t j = ln + __ffs(m) - 1;
+                m &= m - 1;
+                if (!(owned && (S.l_mask[j] & bit))) continue;
+                const float4 c = S.l_cm[j];
+                const uint32_t slot_j = S.l_id[j];
+                const float rx = c.x - pm.x, ry = c.y - pm.y, rz = c.z - pm.z;
+                const float dist = sqrtf(rx * rx + ry * ry + rz * rz);
+                const float pen = my_rad + S.l_rad[j] - dist;
+                if (pen > 0.0f) {
+                    const uint32_t oi = b.idx_in[slot_j];
+                    if (bi < oi) {
+                        const uint32_t slot = atomicAdd(&b.mq->tail, 1u);
+                        if (slot < N) {
+                            // the reference's walk meets a body's leaves in
+                            // descending slot order (childB before childA)
+                            b.mq->pairs[slot] = make_uint2(bi, oi);
+                            b.mkeys[slot] = ((unsigned long long)g << 32) | (N - 1u - slot_j);
+                            b.mslots[slot] = slot_j;
+                        }
+                    }
+                }
+            }
+        }
+        __syncwarp();
+    };
+    // list X's last `cnt` nodes, body by body: the accepting lanes take the
+    // force, the others' mask goes on the stack
+    auto test_x = [&](uint32_t cnt) {
+        __syncwarp();
+        xn -= cnt;
+        const float4* cmv = S.x_cm + xn;
+        const uint2* hv = S.x_half_mask + xn;
+        uint32_t mine = 0u;
+#pragma unroll 4
+        for (uint32_t j = 0; j < cnt; ++j) {
+            const float4 c = cmv[j];
+            const uint2 hm = hv[j];
+            float rx = c.x - pm.x, ry = c.y - pm.y, rz = c.z - pm.z;
+            if (PREC) rx = rx - lo_b.x, ry = ry - lo_b.y, rz = rz - lo_b.z;
+            const float rr = __fmaf_rn(rz, rz, __fmaf_rn(ry, ry, rx * rx));
+            const float inv = rsqrtf(rr + soft);
+            const bool accept = __uint_as_float(hm.x) * inv < theta;
+            const bool me = hm.y & bit;
+            const float f = c.w * (inv * inv * inv);
+            if (me && accept) {
+                ax = __fmaf_rn(f, rx, ax);
+                ay = __fmaf_rn(f, ry, ay);
+                az = __fmaf_rn(f, rz, az);
+                if (want_pot) pot = __fmaf_rn(-c.w, inv, pot);
+            }
+            const uint32_t om = __ballot_sync(0xffffffffu, me && !accept);
+            if (lane == j) mine = om;
+        }
+        uint32_t id = 0u;
+        if (lane < cnt) {
+            id = S.x_id[xn + lane];
+            inter += __popc(hv[lane].y & ~mine & owners);
+        }
+        push(id, mine);
+    };
+    // one candidate per lane (`m`: the lanes whose walk reached it): leaves
+    // and nodes that every body of the box accepts to list A (leaves to L in
+    // the merge and precision forms), nodes that every body opens to the
+    // stack, the others to list X (warp-collective)
+    auto classify = [&](bool has, float4 cm, float half, uint32_t id, uint32_t m) {
+        const bool leaf = has && id < N;
+        bool accept = false, open = false;
+        if (has && !leaf) {
+            const float ux = mnx - cm.x, uy = mny - cm.y, uz = mnz - cm.z;
+            const float vx = cm.x - mxx, vy = cm.y - mxy, vz = cm.z - mxz;
+            const float lx = fmaxf(fmaxf(ux, vx), 0.0f), ly = fmaxf(fmaxf(uy, vy), 0.0f), lz = fmaxf(fmaxf(uz, vz), 0.0f);
+            const float hx = fminf(ux, vx), hy = fminf(uy, vy), hz = fminf(uz, vz);
+            const float near2 = __fmaf_rn(lz, lz, __fmaf_rn(ly, ly, __fmaf_rn(lx, lx, soft)));
+            const float far2 = __fmaf_rn(hz, hz, __fmaf_rn(hy, hy, __fmaf_rn(hx, hx, soft)));
+            // a centre of mass that is not finite has no far2 below 1e30; the
+            // small constants leave squares that lose bits to underflow to X
+            const float h2 = half * half;
+            const bool ok = boxed && far2 < 1e30f;
+            accept = ok && h2 < __fmaf_rn(t2_accept, near2, -1e-33f);
+            open = ok && h2 >= __fmaf_rn(t2_open, far2, 1e-33f);
+        }
+        uint32_t take = m;
+        if (leaf) {
+            const uint32_t own = id - base;  // the body's own leaf, bh_force.comp:76-78
+            if (own < 32u) take &= ~(1u << own);
+        }
+        if (leaf || accept) inter += __popc(take & owners);
+        const bool to_a = accept || (FORM == PF_FP32 && leaf);
+        const uint32_t ba = __ballot_sync(0xffffffffu, to_a);
+        if (to_a) {
+            const uint32_t pos = an + __popc(ba & lanemask_lt());
+            S.a_cm[pos] = make_float4(cm.x, cm.y, cm.z, G * cm.w);
+            S.a_mask[pos] = take;
+        }
+        an += __popc(ba);
+        const bool to_x = has && !leaf && !accept && !open;
+        const uint32_t bx = __ballot_sync(0xffffffffu, to_x);
+        if (to_x) {
+            const uint32_t pos = xn + __popc(bx & lanemask_lt());
+            S.x_cm[pos] = make_float4(cm.x, cm.y, cm.z, G * cm.w);
+            S.x_half_mask[pos] = make_uint2(__float_as_uint(half), m);
+            S.x_id[pos] = id;
+        }
+        xn += __popc(bx);
+        if (FORM != PF_FP32) {
+            const uint32_t bl = __ballot_sync(0xffffffffu, leaf);
+            if (leaf) {
+                const uint32_t pos = ln + __popc(bl & lanemask_lt());
+                S.l_cm[pos] = make_float4(cm.x, cm.y, cm.z, G * cm.w);
+                S.l_mask[pos] = take;
+                if (PREC) S.l_lo[pos] = b.leaf_lo[id];
+                if (MERGE) {
+                    S.l_rad[pos] = b.leaf_rad[id];
+                    S.l_id[pos] = id;
+                }
+            }
+            ln += __popc(bl);
+            if (ln >= 32) flush_l(32);
+        }
+        push(id, open ? m : 0u);
+        if (an >= 32) flush_a(32);
+        if (xn >= 32) test_x(32);
+    };
+
+    if (n > 1 && owners) {
+        const WalkRec root = *b.root_rec;  // bh_force.comp:53
+        classify(lane == 0, root.cm, root.half_side, N, everyone);
+        for (;;) {
+            // the undecided nodes before a pop when the stack is empty (the
+            // opened ones refill it) and, above PW_LOW entries, always: the
+            // walk then takes one node at a time, depth-first, so the stack
+            // holds what a tree of any height needs.  Testing them earlier,
+            // from 8 to 24 waiting ones at 8 to 48 stack entries, changed
+            // nothing (3.26 to 3.29 ms).
+            const bool low = sp > PW_LOW;
+            if (xn && (sp == 0 || low)) {
+                test_x(min(xn, 32u));
+                continue;
+            }
+            if (sp == 0) break;
+            max_sp = max(max_sp, sp);
+            const uint32_t k = low ? 1u : min(sp, 16u);
+            sp -= k;
+            const bool has = lane < 2 * k;
+            uint32_t m = 0u;
+            float4 cm = make_float4(0.f, 0.f, 0.f, 0.f);
+            uint2 meta = make_uint2(0u, 0u);
+            __syncwarp();
+            if (has) {  // lane l: child l & 1 of popped node l / 2
+                const uint2 e = S.stack[sp + (lane >> 1)];
+                const float4* q = reinterpret_cast<const float4*>(b.pairs + e.x) + 2 * (lane & 1u);
+                m = e.y;
+                cm = __ldg(q);
+                meta = __ldg(reinterpret_cast<const uint2*>(q + 1));
+            }
+            __syncwarp();
+            classify(has, cm, __uint_as_float(meta.x), meta.y, m);
+        }
+        if (an) flush_a(an);
+        if (FORM != PF_FP32 && ln) flush_l(ln);
+    }
+    if (overflow && lane == 0) set_error(b.st, GBH_DEVERR_WALK_STACK);
+
+    // counters: one add per block (the whole grid adds to the same words)
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) {
+        inter += __shfl_xor_sync(0xffffffffu, inter, o);
+        opened += __shfl_xor_sync(0xffffffffu, opened, o);
+    }
+    if (lane == 0) {
+        atomicAdd(&s_inter, (unsigned long long)inter);
+        atomicAdd(&s_opened, (unsigned long long)opened);
+        atomicMax(&s_depth, max_sp + 1);
+    }
+    if (owned) {
+        if (PREC) {
+            ax = ax + (nx_ - cx_);
+            ay = ay + (ny_ - cy_);
+            az = az + (nz_ - cz_);
+            pot = pot + (np_ - cp_);
+        }
+        const float4 vd = ld_vel_density(b.bodies_in, bi);
+        if (b.accel && (P->flags & GBH_FLAG_STORE_ACCEL)) b.accel[bi] = make_float4(ax, ay, az, 0.0f);
+        if (b.accel_mag) b.accel_mag[bi] = sqrtf(ax * ax + ay * ay + az * az);
+        if (want_pot) b.potential[bi] = pot;
+        if (PREC)
+            walk_update_fp64(b, P, sim, g, bi, pm, vd, ax, ay, az);
+        else
+            walk_update(b, P, sim, g, bi, pm, vd, ax, ay, az);
+    }
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        atomicAdd(&b.st->interactions, s_inter);
+        atomicAdd(&b.st->opened, s_opened);
+        atomicAdd(&b.sim->uint_debug[0], (uint32_t)s_opened);
+        atomicMax(&b.st->max_stack, s_depth);
+    }
+}
+
+// ---- collision mode ----------------------------------------------------------------
 
 #define WALK_THREADS 256
 #define WALK_WARPS (WALK_THREADS / 32)
@@ -37,12 +470,7 @@ struct __align__(16) StackEntry {
     uint32_t pad;
 };
 
-// PREC: the precision form.  Offsets are formed from the FP32 position and
-// its FP32 residual (leaf_lo), r = (x_j - x_b) + (lo_j - lo_b) for a leaf and
-// (com - x_b) - lo_b for a node, and the leaf terms are summed with Kahan
-// compensation apart from the node terms.  Gravity only.
-template <bool PREC>
-__global__ __launch_bounds__(WALK_THREADS) void k_walk_plain(StepBuffers b) {
+__global__ __launch_bounds__(WALK_THREADS) void k_walk_collide(StepBuffers b) {
     __shared__ StackEntry s_stack[WALK_WARPS][WALK_STACK];
     const uint32_t n = b.st->n_new;
     const uint32_t N = b.N;
@@ -59,20 +487,16 @@ __global__ __launch_bounds__(WALK_THREADS) void k_walk_plain(StepBuffers b) {
     const gbh_sim_values* sim = b.sim;
     const float G = sim->gravitational_constant;
     const float soft = P->softening, theta = P->theta;
-    const uint32_t mode = P->merging_collision_or_neither;
     const ChildPair* __restrict__ pairs = b.pairs;
     StackEntry* stk = s_stack[w];
 
     const uint32_t bi = active ? b.idx_in[g] : 0u;
     float4 pm = active ? b.leaf_pm[g] : make_float4(0.f, 0.f, 0.f, 0.f);
     float4 vd = active ? ld_vel_density(b.bodies_in, bi) : make_float4(0.f, 0.f, 0.f, 0.f);
-    const float my_rad = (active && mode != GBH_MODE_NEITHER) ? b.leaf_rad[g] : 0.0f;
-    const float4 lo_b = (PREC && active) ? b.leaf_lo[g] : make_float4(0.f, 0.f, 0.f, 0.f);
+    const float my_rad = active ? b.leaf_rad[g] : 0.0f;
     const bool want_pot = (P->flags & GBH_FLAG_STORE_POTENTIAL) && b.potential;
     float ax = 0.0f, ay = 0.0f, az = 0.0f, pot = 0.0f;
-    float nx_ = 0.0f, ny_ = 0.0f, nz_ = 0.0f, np_ = 0.0f;  // PREC: leaf terms (Kahan)
-    float cx_ = 0.0f, cy_ = 0.0f, cz_ = 0.0f, cp_ = 0.0f;
-    uint32_t inter = 0, seq = 0;
+    uint32_t inter = 0;
     uint32_t opened = 0;
     uint32_t sp = 0, max_sp = 0;
     bool overflow = false;
@@ -91,14 +515,7 @@ __global__ __launch_bounds__(WALK_THREADS) void k_walk_plain(StepBuffers b) {
     const bool walk = n > 1;
     while (walk) {
         const bool me = (cur_mask >> lane) & 1u;
-        float rx = cur_cm.x - pm.x, ry = cur_cm.y - pm.y, rz = cur_cm.z - pm.z;
-        if (PREC) {
-            float4 lo_j = make_float4(0.f, 0.f, 0.f, 0.f);
-            if (cur_id < N) lo_j = b.leaf_lo[cur_id];
-            rx = rx + (lo_j.x - lo_b.x);
-            ry = ry + (lo_j.y - lo_b.y);
-            rz = rz + (lo_j.z - lo_b.z);
-        }
+        const float rx = cur_cm.x - pm.x, ry = cur_cm.y - pm.y, rz = cur_cm.z - pm.z;
         const float rr = __fmaf_rn(rz, rz, __fmaf_rn(ry, ry, rx * rx));
         const float inv = rsqrtf(rr + soft);
         bool open = false, interact;
@@ -111,24 +528,17 @@ __global__ __launch_bounds__(WALK_THREADS) void k_walk_plain(StepBuffers b) {
         }
         if (interact) {
             const float f = G * cur_cm.w * (inv * inv * inv);
-            if (PREC && cur_id < N) {
-                kahan_add(nx_, cx_, f * rx);
-                kahan_add(ny_, cy_, f * ry);
-                kahan_add(nz_, cz_, f * rz);
-                if (want_pot) kahan_add(np_, cp_, -(G * cur_cm.w) * inv);
-            } else {
-                ax = __fmaf_rn(f, rx, ax);
-                ay = __fmaf_rn(f, ry, ay);
-                az = __fmaf_rn(f, rz, az);
-                if (want_pot) pot = __fmaf_rn(-(G * cur_cm.w), inv, pot);
-            }
+            ax = __fmaf_rn(f, rx, ax);
+            ay = __fmaf_rn(f, ry, ay);
+            az = __fmaf_rn(f, rz, az);
+            if (want_pot) pot = __fmaf_rn(-(G * cur_cm.w), inv, pot);
             ++inter;
-            if (!PREC && mode != GBH_MODE_NEITHER && cur_id < N) {
+            if (cur_id < N) {
                 const uint32_t oi = b.idx_in[cur_id];
                 const float orad = b.leaf_rad[cur_id];
                 const float dist = sqrtf(rx * rx + ry * ry + rz * rz);
                 const float pen = my_rad + orad - dist;
-                if (mode == GBH_MODE_COLLISION && pen > 0.0f) {
+                if (pen > 0.0f) {
                     // bh_force.comp:93-107, in the reference's operation order
                     const float ow = cur_cm.w;
                     const float4 ov = ld_vel_density(b.bodies_in, oi);
@@ -146,16 +556,6 @@ __global__ __launch_bounds__(WALK_THREADS) void k_walk_plain(StepBuffers b) {
                     pm.x -= sc * nx;
                     pm.y -= sc * ny;
                     pm.z -= sc * nz;
-                }
-                if (mode == GBH_MODE_MERGE && pen > 0.0f && bi < oi) {
-                    // bh_force.comp:109-112, plus an ordering key for merge resolution
-                    const uint32_t slot = atomicAdd(&b.mq->tail, 1u);
-                    if (slot < N) {
-                        b.mq->pairs[slot] = make_uint2(bi, oi);
-                        b.mkeys[slot] = ((unsigned long long)g << 32) | seq;
-                        b.mslots[slot] = cur_id;
-                    }
-                    ++seq;
                 }
             }
         }
@@ -207,25 +607,20 @@ __global__ __launch_bounds__(WALK_THREADS) void k_walk_plain(StepBuffers b) {
         atomicMax(&b.st->max_stack, max_sp + 1);
     }
     if (!active) return;
-    if (PREC) {
-        ax = ax + (nx_ - cx_);
-        ay = ay + (ny_ - cy_);
-        az = az + (nz_ - cz_);
-        pot = pot + (np_ - cp_);
-    }
     if (b.accel && (P->flags & GBH_FLAG_STORE_ACCEL)) b.accel[bi] = make_float4(ax, ay, az, 0.0f);
     if (b.accel_mag) b.accel_mag[bi] = sqrtf(ax * ax + ay * ay + az * az);
     if (want_pot) b.potential[bi] = pot;
-    if (PREC)
-        walk_update_fp64(b, P, sim, g, bi, pm, vd, ax, ay, az);
-    else
-        walk_update(b, P, sim, g, bi, pm, vd, ax, ay, az);
+    walk_update(b, P, sim, g, bi, pm, vd, ax, ay, az);
 }
 
 void launch_walk_plain(const StepBuffers& b, cudaStream_t s) {
-    const uint32_t blocks = (b.N + WALK_THREADS - 1) / WALK_THREADS;
-    if (b.prec)
-        k_walk_plain<true><<<blocks, WALK_THREADS, 0, s>>>(b);
+    const uint32_t blocks = (b.N + PW_THREADS - 1) / PW_THREADS;
+    if (b.collide)
+        k_walk_collide<<<(b.N + WALK_THREADS - 1) / WALK_THREADS, WALK_THREADS, 0, s>>>(b);
+    else if (b.prec)
+        k_walk_plain<PF_PREC><<<blocks, PW_THREADS, 0, s>>>(b);
+    else if (b.merge)
+        k_walk_plain<PF_MERGE><<<blocks, PW_THREADS, 0, s>>>(b);
     else
-        k_walk_plain<false><<<blocks, WALK_THREADS, 0, s>>>(b);
+        k_walk_plain<PF_FP32><<<blocks, PW_THREADS, 0, s>>>(b);
 }

@@ -1,0 +1,66 @@
+"""The plain walk's box classification against the oracle's per-body walk: the
+same interactions for every warp shape, for parameters outside the range its
+margins cover, for positions that are not finite, and for a walk that opens
+everything (the stack's depth-first mode)."""
+import numpy as np
+import pytest
+
+from gravity_gb300 import BarnesHut, abi
+
+from .helpers import bounds_of, make_pair, plummer_case, rel_err
+
+pytestmark = pytest.mark.gpu
+
+
+def _walk(g, o, p):
+    for x in (g, o):
+        x.stage_reset(p)
+        x.stage_prepare(p)
+        x.stage_sort()
+        x.stage_build()
+        x.stage_fill()
+        x.stage_walk(p)
+    assert g.read_stats().error_word == 0
+    return g.read_accel()[:, :3], o.read_accel()[:, :3]
+
+
+@pytest.mark.parametrize("n", [2, 3, 31, 32, 33, 127, 129, 4097])
+@pytest.mark.parametrize("theta,soft", [(0.5, 1e-4), (0.5, 0.0), (0.0, 1e-4), (5e-4, 1e-6), (3.0, 1e-2), (2e3, 1e-4)])
+def test_walk_forms_match_oracle(gbh_lib, oracle_mod, n, theta, soft):
+    b = plummer_case(n, seed=n)
+    g, o = make_pair(oracle_mod, BarnesHut, b, bounds_of(b))
+    ag, ao = _walk(g, o, abi.step_params(theta=theta, softening=soft, flags=abi.FLAG_STORE_ACCEL))
+    # a node exactly at the threshold may fall either way (rsqrtf against
+    # 1/sqrtf): 1e-4 of the interactions, as in the parity tests
+    ig, io = g.read_stats().interactions, o.read_stats().interactions
+    assert abs(int(ig) - int(io)) <= 1e-4 * io
+    if theta == 0.0:
+        assert ig == n * (n - 1)  # every leaf of every other body
+    assert np.median(rel_err(ag, ao)) < 1e-5
+
+
+@pytest.mark.parametrize("bad", [np.nan, np.inf])
+def test_walk_with_positions_not_finite(gbh_lib, oracle_mod, bad):
+    b = plummer_case(2000, seed=3)
+    b["pos_mass"][[7, 900], 0] = bad
+    g, o = make_pair(oracle_mod, BarnesHut, b, bounds_of(b))
+    ag, ao = _walk(g, o, abi.step_params(theta=0.5, softening=1e-4, flags=abi.FLAG_STORE_ACCEL))
+    ig, io = g.read_stats().interactions, o.read_stats().interactions
+    assert abs(int(ig) - int(io)) <= 1e-4 * io
+    assert np.array_equal(np.isnan(ag), np.isnan(ao))
+
+
+def test_walk_of_a_tall_tree(gbh_lib, oracle_mod):
+    # bodies halving their distance to a corner (one tree level each) and
+    # coinciding bodies (levels of the index tie-break)
+    k = np.arange(1, 21)
+    line = np.repeat((0.5 ** k)[:, None], 3, axis=1)
+    pos = np.concatenate([line, np.zeros((300, 3)), np.ones((4, 3))]).astype(np.float32)
+    b = plummer_case(len(pos), seed=1)
+    b["pos_mass"][:, :3] = pos
+    g, o = make_pair(oracle_mod, BarnesHut, b, bounds_of(b))
+    for theta in (0.0, 0.5):
+        ag, ao = _walk(g, o, abi.step_params(theta=theta, softening=1e-3, flags=abi.FLAG_STORE_ACCEL))
+        assert abs(int(g.read_stats().interactions) - int(o.read_stats().interactions)) <= 2
+        far = np.linalg.norm(ao, axis=1) > 0
+        assert np.median(rel_err(ag[far], ao[far])) < 1e-5
