@@ -67,7 +67,6 @@ struct DevState {
     uint32_t num_groups;               // body groups of the group walk
     uint32_t group_next;               // the next group a warp of the group walk takes (ticket)
     uint32_t frontier_saturated;       // group walks that accepted instead of opening (full stack)
-    uint32_t fill_frontier;            // nodes handed from the tiled fill to the top-tree fill
     uint32_t sorted_valid;             // sorted_pm holds the current positions in index order
     uint32_t view_count;               // records of the last node selection (gbh_select_*)
     uint32_t shard_lo, shard_hi;       // sorted slots a sharded walk updated [lo, hi)
@@ -115,7 +114,7 @@ struct StepBuffers {
     // writes whole 80-byte nodes (no partial-sector writes to the node arrays)
     uint2* topo_kids;      // (childA, childB) per internal node
     uint32_t* topo_cnt;    // bodiesContained per internal node
-    uint32_t* fill_ready;  // arrival counters of the fill's climb across tiles
+    uint32_t* fill_ready;  // arrival counters of the fill's climb above the groups
     uint32_t* parent_int;  // parentId per internal node
     uint32_t* parent_leaf; // parentId per leaf
     uint2* groups;        // (first slot, body count) of the group walk's body groups
@@ -125,8 +124,6 @@ struct StepBuffers {
     // its ancestors (k_group_paths)
     uint32_t* group_path;
     uint32_t group_path_cap;
-    uint2* fill_frontier; // (node, bodies) handed from the tiled fill to the top-tree fill
-    uint32_t fill_frontier_cap;
     // precision form (GBH_PRECISION_COMPENSATED); null until first used
     const double* pos64_in;  // [N][4] FP64 positions (x, y, z, 0) by body id, current state
     double* pos64_out;       // the next state's

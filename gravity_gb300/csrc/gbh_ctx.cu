@@ -85,10 +85,6 @@ StepBuffers ctx_buffers(const gbh_ctx* c) {
     b.group_node = c->group_node;
     b.group_path = c->group_path;
     b.group_path_cap = c->group_path_cap;
-    // the fill's frontier lives in the sort's spare key buffer (free once the
-    // sorted keys are back in keys_in, until the next step's encode)
-    b.fill_frontier = reinterpret_cast<uint2*>(c->keys[1 - c->iin]);
-    b.fill_frontier_cap = c->N;
     b.pos64_in = c->pos64[c->bin];
     b.pos64_out = c->pos64[1 - c->bin];
     b.leaf_lo = c->leaf_lo;

@@ -8,10 +8,11 @@
 //   written in part.  The stage entry point gbh_stage_build also writes the
 //   reference's intermediate topology words into the nodes (k_build_nodes).
 // Fill: treeInitLeafNodesKernel (bh_tree.comp:140-175) + 64 launches of
-//   treePropagateNodesKernel (bh_tree.comp:183-259) become one kernel: each
-//   leaf thread initialises its leaf and climbs; at every internal node an
-//   atomic on readyChildren lets the second arriving child finish the node
-//   (Karras 2012 / Apetrei 2014).  There is no pass limit, so trees taller
+//   treePropagateNodesKernel (bh_tree.comp:183-259) become two kernels: one
+//   warp per body group (a subtree of at most 96 bodies) initialises its
+//   leaves and finishes its nodes, and one thread per group climbs above the
+//   groups, where an atomic on an arrival counter lets the second child finish
+//   a node (Karras 2012 / Apetrei 2014).  There is no pass limit, so trees taller
 //   than 64 levels are filled completely, and the queue-reset race of the
 //   reference (bh_tree.comp:188-193) does not exist.
 #include "gbh_common.cuh"
@@ -199,7 +200,7 @@ void launch_build(const StepBuffers& b, cudaStream_t s) {
 
 // ---------------------------------------------------------------------------
 // getStarColor, common.glsl:232-276
-__device__ void star_color(float mass, float density, float rgb[3]) {
+__device__ __noinline__ float3 star_color_hot(float mass, float density) {
     const float e = 0.875f - 1.0f / 6.0f;
     float t = 5.95589e-19f * powf(mass, e);
     t = t * powf(density, 1.0f / 6.0f);
@@ -220,9 +221,21 @@ __device__ void star_color(float mass, float density, float rgb[3]) {
     } else {
         bl = 138.5177312231f * logf(gmax(temp - 10.0f, 1e-3f)) - 305.0447927307f;
     }
-    rgb[0] = gclamp(r, 0.0f, 255.0f) / 255.0f;
-    rgb[1] = gclamp(g, 0.0f, 255.0f) / 255.0f;
-    rgb[2] = gclamp(bl, 0.0f, 255.0f) / 255.0f;
+    return make_float3(gclamp(r, 0.0f, 255.0f) / 255.0f, gclamp(g, 0.0f, 255.0f) / 255.0f,
+                       gclamp(bl, 0.0f, 255.0f) / 255.0f);
+}
+
+__device__ __forceinline__ float3 star_color(float mass, float density) {
+    // below these bounds the temperature is at most 0.23: red saturates and
+    // both logarithms are negative before their clamps, so the colour is
+    // exactly (1, 0, 0)
+    if (mass <= 1e22f && density <= 1e24f) return make_float3(1.0f, 0.0f, 0.0f);
+    return star_color_hot(mass, density);
+}
+
+// out of line: the fill's code has to stay in the instruction cache
+__device__ __noinline__ float fill_radius(float body_len_const, float m, float rho) {
+    return body_radius(body_len_const, m, rho);
 }
 
 struct NodeVals {
@@ -265,6 +278,40 @@ __device__ __forceinline__ WalkRec make_rec(const NodeVals& v, uint32_t id, uint
     return r;
 }
 
+// a / m, correctly rounded, from inv = 1 / m correctly rounded (Markstein 1990):
+// a quotient within one unit in the last place, corrected by its exact
+// remainder times the correctly rounded reciprocal, rounds as a / m does.  The
+// first correction brings the product a inv within that unit, the second
+// applies the theorem.  Holds where no remainder underflows: see div3.
+__device__ __forceinline__ float div_by(float a, float m, float inv) {
+    float q = a * inv;
+    q = __fmaf_rn(__fmaf_rn(-q, m, a), inv, q);
+    return __fmaf_rn(__fmaf_rn(-q, m, a), inv, q);
+}
+
+__device__ __noinline__ float3 div3_slow(float x, float y, float z, float m) {
+    return make_float3(x / m, y / m, z / m);
+}
+
+// (x, y, z) / m as IEEE divisions.  One reciprocal serves the three: a node's
+// centre of mass is a link of the fill's dependent chain, and three separate
+// divisions take most of its instructions.
+__device__ __forceinline__ void div3(float x, float y, float z, float m, float inv, float4& out) {
+    const float lo = fminf(fabsf(x), fminf(fabsf(y), fabsf(z))), hi = fmaxf(fabsf(x), fmaxf(fabsf(y), fabsf(z)));
+    // numerators in [2^-80, 2^80] and m in [2^-60, 2^60]: quotients and
+    // remainders (above 2^-128) stay normal; NaN and zeros divide below
+    if (lo >= 8.2718061e-25f && hi <= 1.2089258e24f && m >= 8.6736174e-19f && m <= 1.1529215e18f) {
+        out.x = div_by(x, m, inv);
+        out.y = div_by(y, m, inv);
+        out.z = div_by(z, m, inv);
+    } else {
+        const float3 v = div3_slow(x, y, z, m);
+        out.x = v.x;
+        out.y = v.y;
+        out.z = v.z;
+    }
+}
+
 // One internal node from its two children (bh_tree.comp:223-246); L is
 // childA's values, R childB's.
 __device__ __forceinline__ NodeVals combine(const NodeVals& L, const NodeVals& R) {
@@ -272,11 +319,9 @@ __device__ __forceinline__ NodeVals combine(const NodeVals& L, const NodeVals& R
     const float M = lw + rw;
     NodeVals out;
     if (M > 0.0f) {
-        out.cm.x = (lw * L.cm.x + rw * R.cm.x) / M;
-        out.cm.y = (lw * L.cm.y + rw * R.cm.y) / M;
-        out.cm.z = (lw * L.cm.z + rw * R.cm.z) / M;
-        // the colour (render-only, compared with a tolerance) by one reciprocal
         const float inv_m = 1.0f / M;
+        div3(lw * L.cm.x + rw * R.cm.x, lw * L.cm.y + rw * R.cm.y, lw * L.cm.z + rw * R.cm.z, M, inv_m, out.cm);
+        // the colour (render-only, compared with a tolerance) by the reciprocal
         out.col.x = (lw * L.col.x + rw * R.col.x) * inv_m;
         out.col.y = (lw * L.col.y + rw * R.col.y) * inv_m;
         out.col.z = (lw * L.col.z + rw * R.col.z) * inv_m;
@@ -321,170 +366,258 @@ __device__ __forceinline__ void store_internal(const StepBuffers& b, uint32_t i,
     }
 }
 
-// Node values kept in shared memory by the tiled fill (64 bytes)
-struct TileVals {
-    float4 cm;
-    float4 col;
-    float4 box03;
-    float box4, box5;
-    uint32_t depth, pad;
+// Values of a group's leaves and finished nodes in shared memory.
+struct FillSmem {
+    float4 leaf_cm[GBH_GROUP_MAX];
+    float4 leaf_col[GBH_GROUP_MAX];     // rgb; w: the parent's id
+    float4 node_cm[GBH_GROUP_MAX];
+    float4 node_box03[GBH_GROUP_MAX];
+    float4 node_box45[GBH_GROUP_MAX];   // aabb[4..5], height, bodies
+    float4 node_col[GBH_GROUP_MAX];     // rgb; w: the parent's id
+    uint8_t kid_a[GBH_GROUP_MAX];       // children: slot in the group, + FILL_NODE for a node
+    uint8_t kid_b[GBH_GROUP_MAX];
+    uint8_t list[GBH_GROUP_MAX];        // nodes to finish in this round
 };
+#define FILL_NODE 128u
+#define FILL_WARPS 4
+#define FILL_THREADS (32 * FILL_WARPS)
+#define FILL_SLOTS (GBH_GROUP_MAX / 32)
+#define FILL_BLOCKS 5  // resident blocks per SM
+static_assert(GBH_GROUP_MAX == 96, "the masks of a group's nodes below are three words");
 
-__device__ __forceinline__ TileVals to_tile(const NodeVals& v) {
-    TileVals t;
-    t.cm = v.cm;
-    t.col = v.col;
-    t.box03 = make_float4(v.box[0], v.box[1], v.box[2], v.box[3]);
-    t.box4 = v.box[4];
-    t.box5 = v.box[5];
-    t.depth = v.depth;
-    t.pad = 0;
-    return t;
-}
-
-__device__ __forceinline__ NodeVals from_tile(const TileVals& t) {
+__device__ __forceinline__ NodeVals fill_vals(const FillSmem& S, uint32_t kid) {
     NodeVals v;
-    v.cm = t.cm;
-    v.col = t.col;
-    v.box[0] = t.box03.x;
-    v.box[1] = t.box03.y;
-    v.box[2] = t.box03.z;
-    v.box[3] = t.box03.w;
-    v.box[4] = t.box4;
-    v.box[5] = t.box5;
-    v.depth = t.depth;
+    if (kid < FILL_NODE) {
+        v.cm = S.leaf_cm[kid];
+        v.col = S.leaf_col[kid];
+        v.box[0] = v.box[3] = v.cm.x;
+        v.box[1] = v.box[4] = v.cm.y;
+        v.box[2] = v.box[5] = v.cm.z;
+        v.depth = 0;
+    } else {
+        const uint32_t t = kid - FILL_NODE;
+        v.cm = S.node_cm[t];
+        v.col = S.node_col[t];
+        const float4 a = S.node_box03[t], c = S.node_box45[t];
+        v.box[0] = a.x;
+        v.box[1] = a.y;
+        v.box[2] = a.z;
+        v.box[3] = a.w;
+        v.box[4] = c.x;
+        v.box[5] = c.y;
+        v.depth = __float_as_uint(c.z);
+    }
     return v;
 }
 
-// block-scope release/acquire add on a shared-memory counter
-__device__ __forceinline__ uint32_t atomic_add_acq_rel_cta(uint32_t* p, uint32_t v) {
-    uint32_t old;
-    const uint32_t a = (uint32_t)__cvta_generic_to_shared(p);
-    asm volatile("atom.acq_rel.cta.shared::cta.add.u32 %0, [%1], %2;" : "=r"(old) : "r"(a), "r"(v) : "memory");
-    return old;
-}
-
-#ifndef FILL_TILE
-#define FILL_TILE 512
-#endif
-
-// Tiled fill.  Block k owns the sorted slots [k T, k T + T) (T = FILL_TILE).
-// Phase 1: every thread initialises its leaf and keeps its values in shared
-// memory.  Phase 2: the leaf threads climb while the node's leaf range lies
-// inside the tile; the second child to arrive (a shared-memory counter)
-// combines the children from shared memory.  A thread whose next node crosses
-// a tile boundary hands its node to k_fill_top through a frontier list and
-// ends, so no block waits on a long climb.  The arithmetic of a node depends
-// only on its two children, so the result is the same in any schedule.
-__global__ __launch_bounds__(FILL_TILE) void k_fill(StepBuffers b) {
+// Fill of the body groups, one warp each (persistent: each warp takes every
+// W-th group).  A group is a subtree, so no node of it depends on another
+// warp, and the nodes above the groups (one per group) are left to k_fill_top.
+//   1. Every lane initialises its leaves and keeps their values in shared
+//      memory, beside its nodes' children.
+//   2. Rounds: the nodes whose children are finished (masks of finished
+//      nodes, held by every lane) are listed and finished by consecutive lanes.
+//   3. The warp writes the group's leaf and internal nodes, consecutive lanes
+//      consecutive 16-byte words.
+// The arithmetic of a node depends only on its two children, so the result is
+// the same in any schedule.
+//
+// What bounds it: each round is a dependent chain (children's words, three
+// divisions by one mass, store) of a few lanes, about 10 rounds per group, and
+// before them a gather of the bodies through the index.  So the work of
+// different groups has to overlap: 20 warps per SM (5 blocks of 4 warps at 96
+// registers and 40 KB; 4 or 3 blocks: 2.14 and 2.63 ms), all loads of a group
+// issued together and the next group's ids loaded during the rounds (1.84 ->
+// 1.43 ms).  A subtree per warp needs no block barrier and leaves 1.7% of the
+// nodes to k_fill_top, where tiles of 64 or 512 consecutive slots leave 9% or
+// 2%, in chains as long as the tree is high.  Unrolling the output loops
+// overflows the instruction cache (1.58 ms); so do the star colour and the
+// plain divisions inlined.
+// Fill stage, ms, before (512-slot tiles, threads climbing from their leaves)
+// and after: 16,777,216-body mixture 1.99 -> 1.43; 8,388,608 bodies in clusters 1.12 -> 0.78; 4,194,301
+// bodies with the plain walk's records 0.63 -> 0.46; 65,536 bodies 0.094 -> 0.070.
+__global__ __launch_bounds__(FILL_THREADS, FILL_BLOCKS) void k_fill(StepBuffers b) {
     extern __shared__ __align__(16) unsigned char fill_smem[];
-    TileVals* s_leaf = reinterpret_cast<TileVals*>(fill_smem);  // [FILL_TILE]
-    TileVals* s_node = s_leaf + FILL_TILE;                       // [FILL_TILE]
-    uint4* s_topo = reinterpret_cast<uint4*>(s_node + FILL_TILE);  // childA, childB, first slot, bodies
-    uint32_t* s_parent = reinterpret_cast<uint32_t*>(s_topo + FILL_TILE);
-    uint32_t* s_ready = s_parent + FILL_TILE;  // arrival counters of the tile's internal nodes
+    const uint32_t lane = lane_id(), w = threadIdx.x >> 5;
+    FillSmem& S = reinterpret_cast<FillSmem*>(fill_smem)[w];
     const uint32_t n = b.st->n_new;
     const uint32_t N = b.N;
-    const uint32_t base = blockIdx.x * FILL_TILE;
-    const uint32_t t = threadIdx.x;
-    const uint32_t g = base + t;
-    if (base >= n) return;
+    if (n == 0) return;
     const gbh_sim_values* sim = b.sim;
-    s_ready[t] = 0u;
-    if (g + 1 < n) {
-        // topology of internal node g (written by the build), read once
-        const uint2 kids = b.topo_kids[g];
-        s_topo[t] = make_uint4(kids.x, kids.y, b.node_lo[g], b.topo_cnt[g]);
-        s_parent[t] = b.parent_int[g];
-    }
-    NodeVals own;
-    uint32_t parent0 = GBH_NONE;
-    if (g < n) {
-        const uint32_t bi = b.idx_in[g];
-        const float4 pm = ld_pos_mass(b.bodies_in, bi);
-        const float4 vd = ld_vel_density(b.bodies_in, bi);
-        // leaf init, bh_tree.comp:153-166
-        gbh_node* lf = &b.leaf[g];
-        float4* lp = reinterpret_cast<float4*>(lf);
-        parent0 = b.parent_leaf[g];
-        own.cm = pm;
-        own.box[0] = own.box[3] = pm.x;
-        own.box[1] = own.box[4] = pm.y;
-        own.box[2] = own.box[5] = pm.z;
-        own.col = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-        own.depth = 0;
-        if (pm.w > 0.0f && vd.w > 0.0f) {
-            float rgb[3];
-            star_color(pm.w * sim->unit_mass, vd.w * sim->unit_density, rgb);
-            own.col = make_float4(rgb[0], rgb[1], rgb[2], 0.0f);
+    const uint32_t groups = b.st->num_groups;
+    const bool radii = b.params->merging_collision_or_neither != GBH_MODE_NEITHER;
+    const bool pairs = b.params->mac_mode == GBH_MAC_PLAIN;
+    const uint32_t stride = gridDim.x * FILL_WARPS;
+    uint32_t gi = blockIdx.x * FILL_WARPS + w;
+    // one group ahead: its range, and (from the rounds on) its body ids
+    uint2 grp = gi < groups ? b.groups[gi] : make_uint2(0u, 0u);
+    uint32_t bi[FILL_SLOTS];
+#pragma unroll
+    for (int q = 0; q < FILL_SLOTS; ++q) bi[q] = lane + 32 * q < grp.y ? b.idx_in[grp.x + lane + 32 * q] : 0u;
+    for (; gi < groups; gi += stride) {
+        const uint32_t base = grp.x, count = grp.y;
+        // every load of the group at once: bodies, topology (written by the build)
+        float4 pm[FILL_SLOTS];
+        float density[FILL_SLOTS];
+        uint2 kids[FILL_SLOTS];
+        uint32_t first[FILL_SLOTS], bodies[FILL_SLOTS], parent[FILL_SLOTS], leaf_parent[FILL_SLOTS];
+#pragma unroll
+        for (int q = 0; q < FILL_SLOTS; ++q) {
+            const uint32_t t = lane + 32 * q, g = base + t;
+            pm[q] = make_float4(0.f, 0.f, 0.f, 0.f);
+            density[q] = 0.0f;
+            kids[q] = make_uint2(0u, 0u);
+            first[q] = bodies[q] = parent[q] = leaf_parent[q] = 0u;
+            if (t < count) {
+                pm[q] = ld_pos_mass(b.bodies_in, bi[q]);
+                density[q] = b.bodies_in[bi[q]].vel_density[3];
+                leaf_parent[q] = b.parent_leaf[g];
+                if (g + 1 < n) {
+                    kids[q] = b.topo_kids[g];
+                    first[q] = b.node_lo[g];
+                    bodies[q] = b.topo_cnt[g];
+                    parent[q] = b.parent_int[g];
+                }
+            }
         }
-        lp[0] = pm;
-        lp[1] = make_float4(pm.x, pm.y, pm.z, pm.x);
-        reinterpret_cast<uint4*>(lp)[2] = make_uint4(__float_as_uint(pm.y), __float_as_uint(pm.z), GBH_NONE, GBH_NONE);
-        reinterpret_cast<uint4*>(lp)[3] = make_uint4(0u, 0u, GBH_NONE, parent0);
-        lp[4] = own.col;
-        b.leaf_pm[g] = pm;
-        if (b.params->merging_collision_or_neither != GBH_MODE_NEITHER)
-            b.leaf_rad[g] = body_radius(sim->body_length_constant, pm.w, vd.w);
-        if (b.prec) {
-            // precision form: the FP32 residual of the FP64 position
-            const double2 xy = reinterpret_cast<const double2*>(b.pos64_in)[2 * (size_t)bi];
-            const double z = b.pos64_in[4 * (size_t)bi + 2];
-            b.leaf_lo[g] = make_float4((float)(xy.x - (double)pm.x), (float)(xy.y - (double)pm.y),
-                                       (float)(z - (double)pm.z), 0.0f);
+        grp = gi + stride < groups ? b.groups[gi + stride] : make_uint2(0u, 0u);
+        uint32_t in_mask[FILL_SLOTS], done[FILL_SLOTS], need[FILL_SLOTS][FILL_SLOTS];
+        __syncwarp();  // the last group's words are written out
+#pragma unroll
+        for (int q = 0; q < FILL_SLOTS; ++q) {
+            // internal node g is inside the group, or (at most one index) an
+            // ancestor of it
+            const uint32_t t = lane + 32 * q;
+            in_mask[q] = done[q] = 0u;
+            if (32u * q >= count) continue;  // (uniform) no bodies in this slot
+            const bool inside = t < count && base + t + 1 < n && first[q] >= base && first[q] + bodies[q] <= base + count;
+#pragma unroll
+            for (int k = 0; k < FILL_SLOTS; ++k) need[q][k] = 0u;
+            if (inside) {
+                const bool a_leaf = kids[q].x < N, c_leaf = kids[q].y < N;
+                const uint32_t a = kids[q].x - base - (a_leaf ? 0u : N), c = kids[q].y - base - (c_leaf ? 0u : N);
+                S.kid_a[t] = (uint8_t)(a_leaf ? a : a + FILL_NODE);
+                S.kid_b[t] = (uint8_t)(c_leaf ? c : c + FILL_NODE);
+                S.node_box45[t].w = __uint_as_float(bodies[q]);
+                S.node_col[t].w = __uint_as_float(parent[q]);
+#pragma unroll
+                for (int k = 0; k < FILL_SLOTS; ++k) {
+                    if (!a_leaf && a / 32 == k) need[q][k] |= 1u << (a & 31u);
+                    if (!c_leaf && c / 32 == k) need[q][k] |= 1u << (c & 31u);
+                }
+            }
+            in_mask[q] = __ballot_sync(0xffffffffu, inside);
+            if (t >= count) continue;
+            // leaf init, bh_tree.comp:153-166
+            const uint32_t g = base + t;
+            float3 rgb = make_float3(0.0f, 0.0f, 0.0f);
+            if (pm[q].w > 0.0f && density[q] > 0.0f)
+                rgb = star_color(pm[q].w * sim->unit_mass, density[q] * sim->unit_density);
+            S.leaf_cm[t] = pm[q];
+            S.leaf_col[t] = make_float4(rgb.x, rgb.y, rgb.z, __uint_as_float(leaf_parent[q]));
+            b.leaf_pm[g] = pm[q];
+            if (radii) b.leaf_rad[g] = fill_radius(sim->body_length_constant, pm[q].w, density[q]);
+            if (b.prec) {
+                // precision form: the FP32 residual of the FP64 position
+                const double2 xy = reinterpret_cast<const double2*>(b.pos64_in)[2 * (size_t)bi[q]];
+                const double z = b.pos64_in[4 * (size_t)bi[q] + 2];
+                b.leaf_lo[g] = make_float4((float)(xy.x - (double)pm[q].x), (float)(xy.y - (double)pm[q].y),
+                                           (float)(z - (double)pm[q].z), 0.0f);
+            }
         }
-        s_leaf[t] = to_tile(own);
-    }
-    __syncthreads();
-    if (g >= n) return;
-    const uint32_t tile_end = min(base + FILL_TILE, n);
+#pragma unroll
+        for (int q = 0; q < FILL_SLOTS; ++q) bi[q] = lane + 32 * q < grp.y ? b.idx_in[grp.x + lane + 32 * q] : 0u;
+        for (;;) {
+            uint32_t m[FILL_SLOTS], c = 0;
+#pragma unroll
+            for (int q = 0; q < FILL_SLOTS; ++q) {
+                m[q] = 0u;
+                if (in_mask[q] == done[q]) continue;  // (uniform) nothing left in this slot
+                bool ready = ((in_mask[q] & ~done[q]) >> lane) & 1u;
+#pragma unroll
+                for (int k = 0; k < FILL_SLOTS; ++k) ready = ready && (done[k] & need[q][k]) == need[q][k];
+                m[q] = __ballot_sync(0xffffffffu, ready);
+                if (ready) S.list[c + __popc(m[q] & lanemask_lt())] = (uint8_t)(lane + 32 * q);
+                c += __popc(m[q]);
+            }
+            __syncwarp();
+            if (!c) break;
+            for (uint32_t k = lane; k < c; k += 32) {
+                const uint32_t i = S.list[k];
+                const NodeVals out = combine(fill_vals(S, S.kid_a[i]), fill_vals(S, S.kid_b[i]));
+                S.node_cm[i] = out.cm;
+                S.node_box03[i] = make_float4(out.box[0], out.box[1], out.box[2], out.box[3]);
+                S.node_box45[i].x = out.box[4];
+                S.node_box45[i].y = out.box[5];
+                S.node_box45[i].z = __uint_as_float(out.depth);
+                S.node_col[i].x = out.col.x;
+                S.node_col[i].y = out.col.y;
+                S.node_col[i].z = out.col.z;
+            }
+#pragma unroll
+            for (int q = 0; q < FILL_SLOTS; ++q) done[q] |= m[q];
+            __syncwarp();
+        }
+        // the whole tree is one group: its root is finished here
+        if (n > 1 && count == n) {
+            for (uint32_t i = lane; i < n - 1; i += 32)
+                if (__float_as_uint(S.node_col[i].w) == GBH_NONE) {
+                    const NodeVals out = fill_vals(S, i + FILL_NODE);
+                    b.st->tree_height = out.depth;
+                    *b.root_rec = make_rec(out, base + i + N, n, false);
+                }
+        }
 
-    uint32_t self = g;  // global id of the node whose values are in `own`
-    uint32_t self_count = 1;
-    uint32_t node = parent0;
-    // phase 2: nodes inside the tile (never for a single-body tree, whose root
-    // has one child)
-    while (n > 1 && node != GBH_NONE) {
-        const uint32_t i = node - N;
-        if (i < base || i >= tile_end) break;
-        const uint4 topo = s_topo[i - base];  // childA, childB, first slot, bodies
-        if (topo.z < base || topo.z + topo.w > tile_end) break;
-        if (atomic_add_acq_rel_cta(&s_ready[i - base], 1u) == 0u) return;
-        const bool self_is_a = topo.x == self;
-        const uint32_t sib = self_is_a ? topo.y : topo.x;
-        // the sibling lies inside the tile too
-        uint32_t sib_count = 1;
-        NodeVals S;
-        if (sib < N) {
-            S = from_tile(s_leaf[sib - base]);
-        } else {
-            S = from_tile(s_node[sib - N - base]);
-            sib_count = s_topo[sib - N - base].w;
+        // the group's nodes, whole: Node words (reference layout,
+        // common.glsl:40-58) including the topology ones, readyChildren claimed
+        // (0xFFFFFFFF, bh_tree.comp:200)
+        float4* leaf_words = reinterpret_cast<float4*>(b.leaf + base);
+        float4* node_words = reinterpret_cast<float4*>(b.internal + base);
+        const float none = __uint_as_float(GBH_NONE);
+        auto id_of = [&](uint32_t kid) { return kid < FILL_NODE ? base + kid : base + kid - FILL_NODE + N; };
+        const uint32_t in0 = in_mask[0], in1 = in_mask[1], in2 = in_mask[2];
+        auto is_in = [=](uint32_t i) { return ((i < 32 ? in0 : i < 64 ? in1 : in2) >> (i & 31u)) & 1u; };
+#pragma unroll 1
+        for (uint32_t q = lane; q < 5 * count; q += 32) {
+            const uint32_t i = q / 5, part = q - 5 * i;
+            float4 v = (part < 3 ? S.leaf_cm : S.leaf_col)[i];
+            if (part == 1) v.w = v.x;
+            if (part == 2) v = make_float4(v.y, v.z, none, none);
+            if (part == 3) v = make_float4(0.0f, 0.0f, none, v.w);
+            if (part == 4) v.w = 0.0f;
+            leaf_words[q] = v;
+            if (is_in(i)) {
+                const float4* words = part == 0 ? S.node_cm : part == 1 ? S.node_box03 : part == 4 ? S.node_col : S.node_box45;
+                float4 x = words[i];
+                if (part == 2) x = make_float4(x.x, x.y, __uint_as_float(id_of(S.kid_a[i])), __uint_as_float(id_of(S.kid_b[i])));
+                if (part == 3) x = make_float4(x.z, x.w, none, S.node_col[i].w);
+                if (part == 4) x.w = 0.0f;
+                node_words[q] = x;
+            }
         }
-        const NodeVals& L = self_is_a ? own : S;
-        const NodeVals& R = self_is_a ? S : own;
-        const NodeVals out = combine(L, R);
-        const uint32_t a_id = self_is_a ? self : sib, b_id = self_is_a ? sib : self;
-        store_internal(b, i, out, L, R, a_id, b_id, self_is_a ? self_count : sib_count,
-                       self_is_a ? sib_count : self_count, topo.w, s_parent[i - base]);
-        s_node[i - base] = to_tile(out);
-        self = node;
-        self_count += sib_count;
-        own = out;
-        node = s_parent[i - base];
-        if (node == GBH_NONE) {
-            b.st->tree_height = out.depth;
-            *b.root_rec = make_rec(out, self, self_count, false);
-            return;
+        // the children's walk records feed the plain walk only
+        if (pairs) {
+            float4* pair_words = reinterpret_cast<float4*>(b.pairs + base);
+#pragma unroll 1
+            for (uint32_t q = lane; q < 4 * count; q += 32) {
+                const uint32_t i = q >> 2;
+                if (!is_in(i)) continue;
+                const uint32_t kid = (q & 2u) ? S.kid_b[i] : S.kid_a[i];
+                const bool leaf = kid < FILL_NODE;
+                float4 v = leaf ? S.leaf_cm[kid] : S.node_cm[kid - FILL_NODE];
+                if (q & 1u) {
+                    float half = 0.0f, bodies = __uint_as_float(1u);
+                    if (!leaf) {
+                        const float4 b03 = S.node_box03[kid - FILL_NODE], b45 = S.node_box45[kid - FILL_NODE];
+                        const float box[6] = {b03.x, b03.y, b03.z, b03.w, b45.x, b45.y};
+                        half = half_side(box);
+                        bodies = b45.w;
+                    }
+                    v = make_float4(half, __uint_as_float(id_of(kid)), bodies, 0.0f);
+                }
+                pair_words[q] = v;
+            }
         }
-    }
-    // the next node crosses a tile boundary: hand over
-    if (node != GBH_NONE) {
-        const uint32_t slot = atomicAdd(&b.st->fill_frontier, 1u);
-        if (slot < b.fill_frontier_cap)
-            b.fill_frontier[slot] = make_uint2(self, self_count);
-        else
-            set_error(b.st, GBH_DEVERR_FILL_SPIN);
     }
 }
 
@@ -496,14 +629,17 @@ __device__ void climb_global(const StepBuffers& b, uint32_t self, uint32_t self_
     const uint32_t N = b.N;
     while (node != GBH_NONE) {
         const uint32_t i = node - N;
+        // the topology does not depend on the count: loaded beside it
+        const uint2 kids = b.topo_kids[i];
+        const uint32_t bodies = b.topo_cnt[i];
+        const uint32_t parent = b.parent_int[i];
         // release: own node's writes before the count; acquire: the sibling's writes after it
         const uint32_t old = atomic_add_acq_rel(&b.fill_ready[i], 1u);
         if (old == 0u) return;
-        const uint2 kids = b.topo_kids[i];
         const bool self_is_a = kids.x == self;
         const uint32_t sib = self_is_a ? kids.y : kids.x;
         NodeVals S;
-        uint32_t sib_count = 1;
+        uint32_t sib_count = bodies - self_count;
         if (sib == GBH_NONE) {  // single-body tree: the missing child contributes nothing
             S.cm = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
             S.col = S.cm;
@@ -511,19 +647,15 @@ __device__ void climb_global(const StepBuffers& b, uint32_t self, uint32_t self_
             S.box[3] = S.box[4] = S.box[5] = -1e38f;
             S.depth = 0;
             sib_count = 0;
-        } else if (sib < N) {
-            S = load_node_cg(&b.leaf[sib]);
         } else {
-            S = load_node_cg(&b.internal[sib - N]);
-            sib_count = b.topo_cnt[sib - N];
+            S = load_node_cg(sib < N ? &b.leaf[sib] : &b.internal[sib - N]);
         }
         const NodeVals& L = self_is_a ? own : S;
         const NodeVals& R = self_is_a ? S : own;
         const NodeVals out = combine(L, R);
         const uint32_t a_id = self_is_a ? self : sib, b_id = self_is_a ? sib : self;
-        const uint32_t parent = b.parent_int[i];
         store_internal(b, i, out, L, R, a_id, b_id, self_is_a ? self_count : sib_count,
-                       self_is_a ? sib_count : self_count, b.topo_cnt[i], parent);
+                       self_is_a ? sib_count : self_count, bodies, parent);
         self = node;
         self_count = self_count + sib_count;
         own = out;
@@ -536,25 +668,30 @@ __device__ void climb_global(const StepBuffers& b, uint32_t self, uint32_t self_
     }
 }
 
-// Top-tree fill: the nodes that cross tile boundaries (about 2 N / FILL_TILE),
-// climbing from the frontier the tiled fill left.
+// Fill of the nodes above the body groups: one thread per group climbs from
+// its subtree's root.
 __global__ __launch_bounds__(256) void k_fill_top(StepBuffers b) {
-    const uint32_t count = min(b.st->fill_frontier, b.fill_frontier_cap);
+    const uint32_t groups = b.st->num_groups;
     const uint32_t N = b.N;
-    for (uint32_t e = blockIdx.x * blockDim.x + threadIdx.x; e < count; e += gridDim.x * blockDim.x) {
-        const uint2 fr = b.fill_frontier[e];
-        const gbh_node* nd = fr.x < N ? &b.leaf[fr.x] : &b.internal[fr.x - N];
-        climb_global(b, fr.x, fr.y, load_node_cg(nd), fr.x < N ? b.parent_leaf[fr.x] : b.parent_int[fr.x - N]);
+    for (uint32_t e = blockIdx.x * blockDim.x + threadIdx.x; e < groups; e += gridDim.x * blockDim.x) {
+        const uint32_t id = b.group_node[e];
+        const gbh_node* nd = id < N ? &b.leaf[id] : &b.internal[id - N];
+        const uint32_t parent = id < N ? b.parent_leaf[id] : b.parent_int[id - N];
+        // a single body's group is named by the root, whose one child it is
+        if (b.st->n_new == 1)
+            climb_global(b, 0u, 1u, load_node_cg(&b.leaf[0]), N);
+        else if (parent != GBH_NONE)
+            climb_global(b, id, b.groups[e].y, load_node_cg(nd), parent);
     }
 }
 
-#define FILL_SMEM (FILL_TILE * (2 * sizeof(TileVals) + sizeof(uint4) + 2 * sizeof(uint32_t)))
-
 void fill_setup() {
-    cudaFuncSetAttribute(k_fill, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)FILL_SMEM);
+    cudaFuncSetAttribute(k_fill, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)(FILL_WARPS * sizeof(FillSmem)));
 }
 
 void launch_fill(const StepBuffers& b, cudaStream_t s) {
-    k_fill<<<(b.N + FILL_TILE - 1) / FILL_TILE, FILL_TILE, FILL_SMEM, s>>>(b);
+    // persistent: the blocks that fit at once, no more than the groups need
+    const uint32_t blocks = min(b.num_sms * FILL_BLOCKS, (b.N + FILL_WARPS - 1) / FILL_WARPS);
+    k_fill<<<blocks, FILL_THREADS, FILL_WARPS * sizeof(FillSmem), s>>>(b);
     k_fill_top<<<b.num_sms * 4, 256, 0, s>>>(b);
 }
