@@ -63,7 +63,12 @@ struct GroupShape {
 template <int STACK, int GW_WARPS>
 struct GroupSmem {
     uint32_t stack[GW_WARPS][STACK];
-    float4 list_cm[GW_WARPS][GW_LIST];  // centre of mass, G x mass
+    // the interaction list by component (the force loop takes two entries per
+    // packed instruction): centre of mass, G x mass
+    alignas(16) float list_x[GW_WARPS][GW_LIST];
+    alignas(16) float list_y[GW_WARPS][GW_LIST];
+    alignas(16) float list_z[GW_WARPS][GW_LIST];
+    alignas(16) float list_w[GW_WARPS][GW_LIST];
     uint32_t list_id[GW_WARPS][GW_LIST];
     float list_rad[GW_WARPS][GW_LIST];  // merge form: the leaf entries' body radii
     // merge form: each group body's radius and task counter (slot q * 32 +
@@ -153,7 +158,14 @@ __global__ __launch_bounds__(GroupShape<MODE>::threads, GroupMinBlocks<MODE, FOR
     const float G = sim->gravitational_constant;
     const float soft = P->softening, theta = P->theta, tol = P->mac_tolerance;
     uint32_t* stk = S.stack[w];
-    float4* lcm = S.list_cm[w];
+    float *lx = S.list_x[w], *ly = S.list_y[w], *lz = S.list_z[w], *lw = S.list_w[w];
+    auto entry = [&](uint32_t j) { return make_float4(lx[j], ly[j], lz[j], lw[j]); };
+    auto set_entry = [&](uint32_t j, float4 c) {
+        lx[j] = c.x;
+        ly[j] = c.y;
+        lz[j] = c.z;
+        lw[j] = c.w;
+    };
     uint32_t* lid = S.list_id[w];
     float* lrad = S.list_rad[w];
 
@@ -293,7 +305,7 @@ __global__ __launch_bounds__(GroupShape<MODE>::threads, GroupMinBlocks<MODE, FOR
             // check, merge tasks
 #pragma unroll 2
             for (uint32_t j = 0; j < cnt; ++j) {
-                const float4 c = lcm[j];
+                const float4 c = entry(j);
                 const uint32_t lj = lid[j];
 #pragma unroll
                 for (int q = 0; q < GW_BPL; ++q) {
@@ -320,7 +332,7 @@ __global__ __launch_bounds__(GroupShape<MODE>::threads, GroupMinBlocks<MODE, FOR
         } else if (self_check) {
 #pragma unroll 2
             for (uint32_t j = 0; j < cnt; ++j) {
-                const float4 c = lcm[j];
+                const float4 c = entry(j);
                 const uint32_t lj = lid[j];
 #pragma unroll
                 for (int q = 0; q < GW_BPL; ++q) {
@@ -334,29 +346,64 @@ __global__ __launch_bounds__(GroupShape<MODE>::threads, GroupMinBlocks<MODE, FOR
                 }
             }
         } else {
-            // one loop per number of slots in use (warp-uniform), unrolled
-            // over a constant
+            // Two entries per packed instruction, four per iteration; a partial
+            // list is padded with massless copies of its first entry.  A packed
+            // instruction occupies the FMA pipe for two cycles, so the loop's
+            // bound stays (63% of the pipe's cycles in the group-theta walk),
+            // but it takes 14 issue slots per two entries where single
+            // instructions take 26.  One loop per slot reads the list once per
+            // slot: 7.59 against 7.35 ms (16.8M mixture, learned), and two
+            // iterations unrolled 7.43.
+            const uint32_t pad = (cnt + 3u) & ~3u;
+            if (pad != cnt) {
+                __syncwarp();
+                const float4 c = entry(0);
+                if (lane < pad - cnt) set_entry(cnt + lane, make_float4(c.x, c.y, c.z, 0.0f));
+                __syncwarp();
+            }
+            const float2 soft2 = make_float2(soft, soft);
+            // one loop per number of slots in use (warp-uniform)
             auto slots = [&](auto qn) {
                 constexpr int Q = decltype(qn)::value;
-#pragma unroll 2
-                for (uint32_t j = 0; j < cnt; ++j) {
-                    const float4 c = lcm[j];
+                float2 px[Q], py[Q], pz[Q], sx[Q], sy[Q], sz[Q];
 #pragma unroll
-                    for (int q = 0; q < Q; ++q) {
-                        const float rx = c.x - pw[q].x, ry = c.y - pw[q].y, rz = c.z - pw[q].z;
-                        const float rr = __fmaf_rn(rz, rz, __fmaf_rn(ry, ry, __fmaf_rn(rx, rx, soft)));
-                        const float inv = rsqrtf(rr);
-                        const float f = c.w * (inv * inv * inv);
-                        ax[q] = __fmaf_rn(f, rx, ax[q]);
-                        ay[q] = __fmaf_rn(f, ry, ay[q]);
-                        az[q] = __fmaf_rn(f, rz, az[q]);
+                for (int q = 0; q < Q; ++q) {
+                    px[q] = make_float2(-pw[q].x, -pw[q].x);
+                    py[q] = make_float2(-pw[q].y, -pw[q].y);
+                    pz[q] = make_float2(-pw[q].z, -pw[q].z);
+                    sx[q] = sy[q] = sz[q] = make_float2(0.f, 0.f);
+                }
+#pragma unroll 1
+                for (uint32_t j = 0; j < pad; j += 4) {
+                    const float4 x = *reinterpret_cast<const float4*>(lx + j), y = *reinterpret_cast<const float4*>(ly + j),
+                                 z = *reinterpret_cast<const float4*>(lz + j), m = *reinterpret_cast<const float4*>(lw + j);
+#pragma unroll
+                    for (int h = 0; h < 2; ++h) {
+                        const float2 x2 = h ? make_float2(x.z, x.w) : make_float2(x.x, x.y);
+                        const float2 y2 = h ? make_float2(y.z, y.w) : make_float2(y.x, y.y);
+                        const float2 z2 = h ? make_float2(z.z, z.w) : make_float2(z.x, z.y);
+                        const float2 m2 = h ? make_float2(m.z, m.w) : make_float2(m.x, m.y);
+#pragma unroll
+                        for (int q = 0; q < Q; ++q) {
+                            const float2 rx = __fadd2_rn(x2, px[q]), ry = __fadd2_rn(y2, py[q]), rz = __fadd2_rn(z2, pz[q]);
+                            const float2 rr = __ffma2_rn(rz, rz, __ffma2_rn(ry, ry, __ffma2_rn(rx, rx, soft2)));
+                            const float2 inv = make_float2(rsqrtf(rr.x), rsqrtf(rr.y));
+                            const float2 f = __fmul2_rn(m2, __fmul2_rn(__fmul2_rn(inv, inv), inv));
+                            sx[q] = __ffma2_rn(f, rx, sx[q]);
+                            sy[q] = __ffma2_rn(f, ry, sy[q]);
+                            sz[q] = __ffma2_rn(f, rz, sz[q]);
+                        }
                     }
                 }
+#pragma unroll
+                for (int q = 0; q < Q; ++q) {
+                    ax[q] += sx[q].x + sx[q].y;
+                    ay[q] += sy[q].x + sy[q].y;
+                    az[q] += sz[q].x + sz[q].y;
+                }
             };
-            if (nq >= GW_BPL)
-                slots(std::integral_constant<int, GW_BPL>{});
-            else if (GW_BPL > 3 && nq == 3)
-                slots(std::integral_constant<int, (GW_BPL > 3 ? 3 : 1)>{});
+            if (nq > 2)
+                slots(std::integral_constant<int, 3>{});
             else if (nq == 2)
                 slots(std::integral_constant<int, 2>{});
             else
@@ -372,7 +419,7 @@ __global__ __launch_bounds__(GroupShape<MODE>::threads, GroupMinBlocks<MODE, FOR
             for (uint32_t j0 = 0; j0 < cnt; j0 += 32) {
                 bool near = false;
                 if (j0 + lane < cnt && lid[j0 + lane] < N) {
-                    const float4 c = lcm[j0 + lane];
+                    const float4 c = entry(j0 + lane);
                     const float dx = fmaxf(fmaxf(bmn.x - c.x, c.x - bmx.x), 0.0f);
                     const float dy = fmaxf(fmaxf(bmn.y - c.y, c.y - bmx.y), 0.0f);
                     const float dz = fmaxf(fmaxf(bmn.z - c.z, c.z - bmx.z), 0.0f);
@@ -383,7 +430,7 @@ __global__ __launch_bounds__(GroupShape<MODE>::threads, GroupMinBlocks<MODE, FOR
                 while (m) {
                     const uint32_t j = j0 + __ffs(m) - 1;
                     m &= m - 1;
-                    const float4 c = lcm[j];
+                    const float4 c = entry(j);
                     const uint32_t lj = lid[j];
                     const float lr = lrad[j];
 #pragma unroll
@@ -407,9 +454,9 @@ __global__ __launch_bounds__(GroupShape<MODE>::threads, GroupMinBlocks<MODE, FOR
         if (kind == 1) {
             const uint32_t pos = ln + __popc(bl & lanemask_lt());
             if (PREC)
-                lcm[pos] = make_float4((cm.x - gg.cx) + lo.x, (cm.y - gg.cy) + lo.y, (cm.z - gg.cz) + lo.z, G * cm.w);
+                set_entry(pos, make_float4((cm.x - gg.cx) + lo.x, (cm.y - gg.cy) + lo.y, (cm.z - gg.cz) + lo.z, G * cm.w));
             else
-                lcm[pos] = make_float4(cm.x, cm.y, cm.z, G * cm.w);
+                set_entry(pos, make_float4(cm.x, cm.y, cm.z, G * cm.w));
             lid[pos] = id;
             if (merging) lrad[pos] = lo.x;  // the leaf's radius, read at the pop (0 for nodes)
         }
@@ -422,147 +469,148 @@ __global__ __launch_bounds__(GroupShape<MODE>::threads, GroupMinBlocks<MODE, FOR
         sp += 2 * __popc(bo);
         opened += __popc(bo);
         __syncwarp();
-        if (ln >= 32) {
-            flush(32);
-            ln -= 32;
+    };
+
+    // One site each for the flush, the network and the commit: inlined at
+    // every place that can call for them (four flushes, two networks), they
+    // overflowed the instruction cache.  Walk stage, ms, with the packed force
+    // loop, before and after: learned with merges on 8.4M bodies in clusters
+    // 7.08 -> 4.20, learned on the 16.8M mixture 7.73 -> 7.35, group theta on a
+    // 2.0M mixture 1.50 -> 1.45.
+    for (;;) {
+        if (ln >= 32 || (ln > 0 && sp == 0 && np == 0)) {
+            const uint32_t cnt = min(ln, 32u);
+            flush(cnt);
+            ln -= cnt;
             __syncwarp();
             if (lane < ln) {  // move the remaining entries to the front
-                lcm[lane] = lcm[32 + lane];
+                set_entry(lane, entry(32 + lane));
                 lid[lane] = lid[32 + lane];
                 if (merging) lrad[lane] = lrad[32 + lane];
             }
             __syncwarp();
-        }
-    };
-
-    // decide the first `cnt` (<= 32) queued band candidates with one MLP pass
-    // and move the rest of the queue to the front
-    auto decide_queue = [&](uint32_t cnt) {
-        // features of queue rows [0, cnt), one per lane, then one MLP pass
-        float feat[MAC_FEATURES];
-#pragma unroll
-        for (int q = 0; q < MAC_FEATURES; ++q) feat[q] = 0.0f;
-        if (lane < cnt) {
-            NodeGeom ng;
-            ng.cm = S.pend_cm[w][lane];
-            const float4 b0 = S.pend_b0[w][lane];
-            const float4 b1 = S.pend_b1[w][lane];
-            ng.bmin = make_float3(b0.x, b0.y, b0.z);
-            ng.bmax = make_float3(b1.x, b1.y, b1.z);
-            ng.count = __float_as_uint(b0.w);
-            mac_features(S.geom[w], ng, feat);
-        }
-        mac_stage_features(mw, w, lane, feat);
-        const float pred = mac_infer_warp(mw, w, lane);
-        evals += cnt;
-        // the row's node, read back after the network (fewer live registers)
-        uint32_t kind = 0, id = 0, ca = 0, cb = 0;
-        float4 cm = make_float4(0.f, 0.f, 0.f, 0.f);
-        if (lane < cnt) {
-            kind = pred < tol ? 1u : 2u;
-            cm = S.pend_cm[w][lane];
-            id = __float_as_uint(S.pend_b1[w][lane].w);
-            const uint2 kids = S.pend_kids[w][lane];
-            ca = kids.x;
-            cb = kids.y;
-        }
-        const uint32_t rest = np - cnt;
-        __syncwarp();
-        if (lane < rest) {
-            S.pend_cm[w][lane] = S.pend_cm[w][32 + lane];
-            S.pend_b0[w][lane] = S.pend_b0[w][32 + lane];
-            S.pend_b1[w][lane] = S.pend_b1[w][32 + lane];
-            S.pend_kids[w][lane] = S.pend_kids[w][32 + lane];
-        }
-        np = rest;
-        __syncwarp();
-        commit(kind, id, cm, ca, cb, make_float4(0.f, 0.f, 0.f, 0.f));
-    };
-
-    while (sp > 0 || np > 0) {
-        // the network decides the queue before a pop when the stack holds
-        // fewer than GW_DECIDE_SP nodes and GW_DECIDE_NP or more rows wait:
-        // its opened nodes refill the stack, so pops run fuller (a decision
-        // does not depend on the batch)
-        if (MODE == GM_LEARNED && (sp == 0 || (sp < GW_DECIDE_SP && np >= GW_DECIDE_NP))) {
-            decide_queue(min(np, 32u));
             continue;
         }
-        const uint32_t k = min(sp, 32u);
-        sp -= k;
-        const bool has = lane < k;
-        const uint32_t id = has ? stk[sp + lane] : 0u;
-        __syncwarp();
+        if (sp == 0 && np == 0) break;
         uint32_t kind = 0;  // 0 nothing, 1 list, 2 open, 3 queued for the network
-        float4 cm = make_float4(0.f, 0.f, 0.f, 0.f);
-        float4 qb0 = cm, qb1 = cm, lo = cm;
-        uint32_t ca = 0, cb = 0, qcount = 0;
-        if (has) {
-            if (id < N) {
-                cm = b.leaf_pm[id];
-                if (PREC) lo = b.leaf_lo[id];
-                if (merging) lo.x = b.leaf_rad[id];
-                kind = 1;
-            } else {
-                const gbh_node* nd = &b.internal[id - N];
-                const float4* q = reinterpret_cast<const float4*>(nd);
-                cm = __ldg(q + 0);
-                qb0 = __ldg(q + 1);
-                qb1 = __ldg(q + 2);  // aabb4, aabb5, childA, childB
-                ca = __float_as_uint(qb1.z);
-                cb = __float_as_uint(qb1.w);
-                qcount = __ldg(&nd->bodies_contained);
-                NodeGeom ng;
-                ng.cm = cm;
-                ng.bmin = make_float3(qb0.x, qb0.y, qb0.z);
-                ng.bmax = make_float3(qb0.w, qb1.x, qb1.y);
-                ng.count = qcount;
-                if (MODE == GM_LEARNED) {
-                    // the network decides the band between a rule that is
-                    // safe to accept (band_lo, default theta_g = 0.25) and one
-                    // that must open (band_hi, default theta_g = 4): it never
-                    // accepts a node the group reaches
-                    const float rho = group_rho(S.geom[w], ng);  // shared copy: fewer live registers
-                    kind = rho < band_lo ? 1u : rho < band_hi ? 3u : 2u;
-                } else {
-                    kind = group_theta_accept(gg, ng, theta) ? 1 : 2;
-                    // training pairs: the band the network decides (see GM_LEARNED)
-                    if (MODE == GM_RECORD && ng.count <= mw.rec_max_bodies &&
-                        hash32(id ^ hash32(grp.x + mw.rec_seed)) <= mw.rec_keep &&
-                        group_rho(gg, ng) < band_hi && !(group_rho(gg, ng) < band_lo)) {
-                        const uint32_t slot = atomicAdd(mw.rec_count, 1u);
-                        if (slot < mw.rec_cap) {
-                            float f[MAC_FEATURES];
-                            mac_features(gg, ng, f);
-                            mw.rec_pairs[slot] = make_uint2(gi, id);
+        uint32_t id = 0, ca = 0, cb = 0;
+        float4 cm = make_float4(0.f, 0.f, 0.f, 0.f), lo = cm;
+        // the network decides the queue when a full batch waits, and before a
+        // pop when the stack holds fewer than GW_DECIDE_SP nodes and
+        // GW_DECIDE_NP or more rows wait: its opened nodes refill the stack, so
+        // pops run fuller (a decision does not depend on the batch)
+        if (MODE == GM_LEARNED && (np >= 32 || sp == 0 || (sp < GW_DECIDE_SP && np >= GW_DECIDE_NP))) {
+            // the first rows of the queue, one MLP pass; the rest moves to the front
+            const uint32_t cnt = min(np, 32u);
+            // features of queue rows [0, cnt), one per lane, then one MLP pass
+            float feat[MAC_FEATURES];
 #pragma unroll
-                            for (int q = 0; q < MAC_FEATURES; ++q) mw.rec_feats[(size_t)slot * MAC_FEATURES + q] = f[q];
+            for (int q = 0; q < MAC_FEATURES; ++q) feat[q] = 0.0f;
+            if (lane < cnt) {
+                NodeGeom ng;
+                ng.cm = S.pend_cm[w][lane];
+                const float4 b0 = S.pend_b0[w][lane];
+                const float4 b1 = S.pend_b1[w][lane];
+                ng.bmin = make_float3(b0.x, b0.y, b0.z);
+                ng.bmax = make_float3(b1.x, b1.y, b1.z);
+                ng.count = __float_as_uint(b0.w);
+                mac_features(S.geom[w], ng, feat);
+            }
+            mac_stage_features(mw, w, lane, feat);
+            const float pred = mac_infer_warp(mw, w, lane);
+            evals += cnt;
+            // the row's node, read back after the network (fewer live registers)
+            if (lane < cnt) {
+                kind = pred < tol ? 1u : 2u;
+                cm = S.pend_cm[w][lane];
+                id = __float_as_uint(S.pend_b1[w][lane].w);
+                const uint2 kids = S.pend_kids[w][lane];
+                ca = kids.x;
+                cb = kids.y;
+            }
+            const uint32_t rest = np - cnt;
+            __syncwarp();
+            if (lane < rest) {
+                S.pend_cm[w][lane] = S.pend_cm[w][32 + lane];
+                S.pend_b0[w][lane] = S.pend_b0[w][32 + lane];
+                S.pend_b1[w][lane] = S.pend_b1[w][32 + lane];
+                S.pend_kids[w][lane] = S.pend_kids[w][32 + lane];
+            }
+            np = rest;
+            __syncwarp();
+        } else {
+            const uint32_t k = min(sp, 32u);
+            sp -= k;
+            const bool has = lane < k;
+            id = has ? stk[sp + lane] : 0u;
+            __syncwarp();
+            float4 qb0 = cm, qb1 = cm;
+            uint32_t qcount = 0;
+            if (has) {
+                if (id < N) {
+                    cm = b.leaf_pm[id];
+                    if (PREC) lo = b.leaf_lo[id];
+                    if (merging) lo.x = b.leaf_rad[id];
+                    kind = 1;
+                } else {
+                    const gbh_node* nd = &b.internal[id - N];
+                    const float4* q = reinterpret_cast<const float4*>(nd);
+                    cm = __ldg(q + 0);
+                    qb0 = __ldg(q + 1);
+                    qb1 = __ldg(q + 2);  // aabb4, aabb5, childA, childB
+                    ca = __float_as_uint(qb1.z);
+                    cb = __float_as_uint(qb1.w);
+                    qcount = __ldg(&nd->bodies_contained);
+                    NodeGeom ng;
+                    ng.cm = cm;
+                    ng.bmin = make_float3(qb0.x, qb0.y, qb0.z);
+                    ng.bmax = make_float3(qb0.w, qb1.x, qb1.y);
+                    ng.count = qcount;
+                    if (MODE == GM_LEARNED) {
+                        // the network decides the band between a rule that is
+                        // safe to accept (band_lo, default theta_g = 0.25) and one
+                        // that must open (band_hi, default theta_g = 4): it never
+                        // accepts a node the group reaches
+                        const float rho = group_rho(S.geom[w], ng);  // shared copy: fewer live registers
+                        kind = rho < band_lo ? 1u : rho < band_hi ? 3u : 2u;
+                    } else {
+                        kind = group_theta_accept(gg, ng, theta) ? 1 : 2;
+                        // training pairs: the band the network decides (see GM_LEARNED)
+                        if (MODE == GM_RECORD && ng.count <= mw.rec_max_bodies &&
+                            hash32(id ^ hash32(grp.x + mw.rec_seed)) <= mw.rec_keep &&
+                            group_rho(gg, ng) < band_hi && !(group_rho(gg, ng) < band_lo)) {
+                            const uint32_t slot = atomicAdd(mw.rec_count, 1u);
+                            if (slot < mw.rec_cap) {
+                                float f[MAC_FEATURES];
+                                mac_features(gg, ng, f);
+                                mw.rec_pairs[slot] = make_uint2(gi, id);
+#pragma unroll
+                                for (int q = 0; q < MAC_FEATURES; ++q) mw.rec_feats[(size_t)slot * MAC_FEATURES + q] = f[q];
+                            }
                         }
                     }
                 }
             }
-        }
-        if (MODE == GM_LEARNED) {
-            // queue band candidates with their geometry; the network decides
-            // them 32 at a time
-            const uint32_t bq = __ballot_sync(0xffffffffu, kind == 3);
-            if (kind == 3) {
-                const uint32_t row = np + __popc(bq & lanemask_lt());
-                S.pend_cm[w][row] = cm;
-                S.pend_b0[w][row] = make_float4(qb0.x, qb0.y, qb0.z, __uint_as_float(qcount));
-                S.pend_b1[w][row] = make_float4(qb0.w, qb1.x, qb1.y, __uint_as_float(id));
-                S.pend_kids[w][row] = make_uint2(ca, cb);
-                kind = 0;
+            if (MODE == GM_LEARNED) {
+                // queue band candidates with their geometry; the network decides
+                // them 32 at a time
+                const uint32_t bq = __ballot_sync(0xffffffffu, kind == 3);
+                if (kind == 3) {
+                    const uint32_t row = np + __popc(bq & lanemask_lt());
+                    S.pend_cm[w][row] = cm;
+                    S.pend_b0[w][row] = make_float4(qb0.x, qb0.y, qb0.z, __uint_as_float(qcount));
+                    S.pend_b1[w][row] = make_float4(qb0.w, qb1.x, qb1.y, __uint_as_float(id));
+                    S.pend_kids[w][row] = make_uint2(ca, cb);
+                    kind = 0;
+                }
+                np += __popc(bq);
+                __syncwarp();
+            } else {
+                evals += __popc(__ballot_sync(0xffffffffu, has && id >= N));
             }
-            np += __popc(bq);
-            __syncwarp();
-        } else {
-            evals += __popc(__ballot_sync(0xffffffffu, has && id >= N));
         }
         commit(kind, id, cm, ca, cb, lo);
-        if (MODE == GM_LEARNED && np >= 32) decide_queue(32);
     }
-    if (ln) flush(ln);
     (void)saturated;
 
     // counters: interactions count the group's bodies for every list entry
