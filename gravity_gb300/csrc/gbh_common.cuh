@@ -237,6 +237,22 @@ __device__ __forceinline__ uint32_t atomic_add_acq_rel(uint32_t* p, uint32_t v) 
     return old;
 }
 
+// 1/sqrt(x) and log2(x) as the hardware gives them, one instruction each.
+// rsqrtf and __log2f are the same instruction between a test and two
+// multiplications for subnormal x, so for x that is not subnormal (NaN,
+// infinities and negative x included) the results are the same bits.
+__device__ __forceinline__ float rsqrt_normal(float x) {
+    float y;
+    asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
+    return y;
+}
+__device__ __forceinline__ float log2_normal(float x) {
+    float y;
+    asm("lg2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
+    return y;
+}
+#define GBH_MIN_NORMAL 1.17549435e-38f
+
 __device__ __forceinline__ uint32_t lane_id() { return threadIdx.x & 31u; }
 __device__ __forceinline__ uint32_t lanemask_lt() {
     uint32_t m;

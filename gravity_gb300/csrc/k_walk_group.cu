@@ -39,17 +39,16 @@
 #define GW_LIST 64
 #define GW_QUEUE 64  // queued band candidates per warp: a full MLP batch + one pop
 #define GW_BPL (GBH_GROUP_MAX / 32)  // bodies per lane
-#ifndef GW_DECIDE_SP
-#define GW_DECIDE_SP 64u  // learned walk: decide the queue early below this stack depth...
-#endif
-#ifndef GW_DECIDE_NP
-#define GW_DECIDE_NP 16u  // ...when at least this many rows wait
-#endif
+
+// FORM: the arithmetic form and the step's extra work, fixed per instance so
+// that the common case keeps its registers: FORM_FP32, FORM_PREC (precision
+// form), FORM_MERGE (merge tasks from the leaf entries).
+enum GroupForm { FORM_FP32 = 0, FORM_PREC = 1, FORM_MERGE = 2 };
 
 enum GroupMode { GM_THETA = 0, GM_LEARNED = 1, GM_RECORD = 2 };
 
 // Block shape per mode.  The learned walk runs 4-warp blocks, five per SM
-// (96 registers, 44 KB of shared memory each): 20 warps per SM, where 8-warp
+// (96 registers, 37 KB of shared memory each): 20 warps per SM, where 8-warp
 // blocks fit two (16 warps).  The others run 8-warp blocks.
 template <int MODE>
 struct GroupShape {
@@ -60,7 +59,7 @@ struct GroupShape {
 // shared memory: the stacks and lists first, the network's tiles last (only
 // the learned walk allocates them).  The learned walk's stacks are shorter so
 // that more blocks fit on an SM.
-template <int STACK, int GW_WARPS>
+template <int STACK, int GW_WARPS, bool MERGE>
 struct GroupSmem {
     uint32_t stack[GW_WARPS][STACK];
     // the interaction list by component (the force loop takes two entries per
@@ -70,29 +69,32 @@ struct GroupSmem {
     alignas(16) float list_z[GW_WARPS][GW_LIST];
     alignas(16) float list_w[GW_WARPS][GW_LIST];
     uint32_t list_id[GW_WARPS][GW_LIST];
-    float list_rad[GW_WARPS][GW_LIST];  // merge form: the leaf entries' body radii
-    // merge form: each group body's radius and task counter (slot q * 32 +
-    // lane), the group's largest radius
-    float body_rad[GW_WARPS][GBH_GROUP_MAX];
-    uint32_t body_seq[GW_WARPS][GBH_GROUP_MAX];
+    // merge form: the leaf entries' body radii, each group body's radius and
+    // task counter (slot q * 32 + lane), the group's largest radius
+    float list_rad[MERGE ? GW_WARPS : 1][MERGE ? GW_LIST : 1];
+    float body_rad[MERGE ? GW_WARPS : 1][MERGE ? GBH_GROUP_MAX : 1];
+    uint32_t body_seq[MERGE ? GW_WARPS : 1][MERGE ? GBH_GROUP_MAX : 1];
     float grp_rad[GW_WARPS];
     // queued band candidates of the learned walk: centre of mass, box and
-    // count, box and id, children
+    // count, box and id, children.  A row's boxes turn into its features when
+    // it is decided: words 0 to 3 in pend_b0, 4 and 5 in pend_b1's first two.
+    // With a feature tile of their own, and the merge form's arrays in every
+    // form, the blocks took 228 KB of an SM's 256 KB; now they fit in 196 KB,
+    // and the rest is L1 (7.00 -> 6.67 ms, 16.8M mixture).
     float4 pend_cm[GW_WARPS][GW_QUEUE];
     float4 pend_b0[GW_WARPS][GW_QUEUE];
     float4 pend_b1[GW_WARPS][GW_QUEUE];
     uint2 pend_kids[GW_WARPS][GW_QUEUE];
     GroupGeom geom[GW_WARPS];  // the group's geometry and feature terms
     alignas(16) uint32_t frag[MAC_SMEM_FRAG_WORDS];
-    __nv_bfloat16 x[GW_WARPS * 32 * 16];  // feature tile of the batch being decided
 };
 #ifndef GW_STACK_LEARNED
 #define GW_STACK_LEARNED 640
 #endif
-template <int MODE>
+template <int MODE, int FORM>
 struct GroupCfg {
     static constexpr int stack = MODE == GM_LEARNED ? GW_STACK_LEARNED : GW_STACK;
-    using Smem = GroupSmem<stack, GroupShape<MODE>::warps>;
+    using Smem = GroupSmem<stack, GroupShape<MODE>::warps, FORM == FORM_MERGE>;
     static constexpr size_t smem = MODE == GM_LEARNED ? sizeof(Smem) : offsetof(Smem, pend_cm);
 };
 
@@ -100,10 +102,6 @@ struct GroupCfg {
 // relative to the group centre c_g: (x - c_g) + lo for a leaf (lo its FP32
 // residual), com - c_g for a node; leaf terms are summed with Kahan
 // compensation apart from the node terms.
-// FORM: the arithmetic form and the step's extra work, fixed per instance so
-// that the common case keeps its registers: FORM_FP32, FORM_PREC (precision
-// form), FORM_MERGE (merge tasks from the leaf entries).
-enum GroupForm { FORM_FP32 = 0, FORM_PREC = 1, FORM_MERGE = 2 };
 
 // resident blocks per SM each instance is compiled for: the learned FP32 walk
 // five 4-warp blocks, its precision and merge forms four (their registers
@@ -119,10 +117,12 @@ template <int MODE, int FORM>
 __global__ __launch_bounds__(GroupShape<MODE>::threads, GroupMinBlocks<MODE, FORM>::value) void k_walk_group(
     StepBuffers b, MacDeviceWeights mw) {
     constexpr bool PREC = FORM == FORM_PREC;
+    // merging (bh_force.comp:109-112): every leaf entry is tested for overlap
+    constexpr bool merging = FORM == FORM_MERGE;
     extern __shared__ __align__(16) unsigned char smem_raw[];
-    using Cfg = GroupCfg<MODE>;
+    using Cfg = GroupCfg<MODE, FORM>;
     typename Cfg::Smem& S = *reinterpret_cast<typename Cfg::Smem*>(smem_raw);
-    if (MODE == GM_LEARNED) mac_load_frag(mw, S.frag, S.x);
+    if (MODE == GM_LEARNED) mac_load_frag(mw, S.frag, nullptr);
     // the updates below fill sorted_pm (the recording walk updates nothing the
     // step keeps)
     if (MODE != GM_RECORD && blockIdx.x == 0 && threadIdx.x == 0) b.st->sorted_valid = 1u;
@@ -167,7 +167,7 @@ __global__ __launch_bounds__(GroupShape<MODE>::threads, GroupMinBlocks<MODE, FOR
         lw[j] = c.w;
     };
     uint32_t* lid = S.list_id[w];
-    float* lrad = S.list_rad[w];
+    float* lrad = S.list_rad[merging ? w : 0];
 
     // group box (inactive slots repeat the first body)
     float4 pmq[GW_BPL];
@@ -221,11 +221,9 @@ __global__ __launch_bounds__(GroupShape<MODE>::threads, GroupMinBlocks<MODE, FOR
         }
     }
     const bool want_pot = (P->flags & GBH_FLAG_STORE_POTENTIAL) && b.potential;
-    // merging (bh_force.comp:109-112): every leaf entry is tested for overlap
-    constexpr bool merging = FORM == FORM_MERGE;
     // the merge state lives in shared memory: the tests are rare (screened)
-    float* my_rad = S.body_rad[w];
-    uint32_t* seq = S.body_seq[w];
+    float* my_rad = S.body_rad[merging ? w : 0];
+    uint32_t* seq = S.body_seq[merging ? w : 0];
     if (merging) {
         float gr = 0.0f;
 #pragma unroll
@@ -387,7 +385,7 @@ __global__ __launch_bounds__(GroupShape<MODE>::threads, GroupMinBlocks<MODE, FOR
                         for (int q = 0; q < Q; ++q) {
                             const float2 rx = __fadd2_rn(x2, px[q]), ry = __fadd2_rn(y2, py[q]), rz = __fadd2_rn(z2, pz[q]);
                             const float2 rr = __ffma2_rn(rz, rz, __ffma2_rn(ry, ry, __ffma2_rn(rx, rx, soft2)));
-                            const float2 inv = make_float2(rsqrtf(rr.x), rsqrtf(rr.y));
+                            const float2 inv = make_float2(rsqrt_normal(rr.x), rsqrt_normal(rr.y));
                             const float2 f = __fmul2_rn(m2, __fmul2_rn(__fmul2_rn(inv, inv), inv));
                             sx[q] = __ffma2_rn(f, rx, sx[q]);
                             sy[q] = __ffma2_rn(f, ry, sy[q]);
@@ -476,18 +474,13 @@ __global__ __launch_bounds__(GroupShape<MODE>::threads, GroupMinBlocks<MODE, FOR
     // overflowed the instruction cache.  Walk stage, ms, with the packed force
     // loop, before and after: learned with merges on 8.4M bodies in clusters
     // 7.08 -> 4.20, learned on the 16.8M mixture 7.73 -> 7.35, group theta on a
-    // 2.0M mixture 1.50 -> 1.45.
+    // 2.0M mixture 1.50 -> 1.45; with one instruction per reciprocal square root
+    // (rsqrt_normal) 3.99, 7.05 and 1.24.  The whole list is flushed and the
+    // queue's last rows are decided, so nothing is moved to the front.
     for (;;) {
         if (ln >= 32 || (ln > 0 && sp == 0 && np == 0)) {
-            const uint32_t cnt = min(ln, 32u);
-            flush(cnt);
-            ln -= cnt;
-            __syncwarp();
-            if (lane < ln) {  // move the remaining entries to the front
-                set_entry(lane, entry(32 + lane));
-                lid[lane] = lid[32 + lane];
-                if (merging) lrad[lane] = lrad[32 + lane];
-            }
+            flush(ln);
+            ln = 0;
             __syncwarp();
             continue;
         }
@@ -495,48 +488,50 @@ __global__ __launch_bounds__(GroupShape<MODE>::threads, GroupMinBlocks<MODE, FOR
         uint32_t kind = 0;  // 0 nothing, 1 list, 2 open, 3 queued for the network
         uint32_t id = 0, ca = 0, cb = 0;
         float4 cm = make_float4(0.f, 0.f, 0.f, 0.f), lo = cm;
-        // the network decides the queue when a full batch waits, and before a
-        // pop when the stack holds fewer than GW_DECIDE_SP nodes and
-        // GW_DECIDE_NP or more rows wait: its opened nodes refill the stack, so
-        // pops run fuller (a decision does not depend on the batch)
-        if (MODE == GM_LEARNED && (np >= 32 || sp == 0 || (sp < GW_DECIDE_SP && np >= GW_DECIDE_NP))) {
-            // the first rows of the queue, one MLP pass; the rest moves to the front
+        // the network decides the queue when a full batch waits or the stack is
+        // empty.  Deciding fewer rows early to refill a short stack (a decision
+        // does not depend on its batch) makes pops fuller, but a batch costs the
+        // same for any number of rows: from 16, 20, 24 or 28 rows on below 64
+        // stack entries 6.67, 6.60, 6.53 and 6.47 ms, never 6.33 (16.8M mixture).
+        if (MODE == GM_LEARNED && (np >= 32 || sp == 0)) {
+            // features of the queue's last rows, one per lane, then one MLP pass
             const uint32_t cnt = min(np, 32u);
-            // features of queue rows [0, cnt), one per lane, then one MLP pass
+            np -= cnt;
+            const uint32_t row = np + lane;
             float feat[MAC_FEATURES];
 #pragma unroll
             for (int q = 0; q < MAC_FEATURES; ++q) feat[q] = 0.0f;
             if (lane < cnt) {
                 NodeGeom ng;
-                ng.cm = S.pend_cm[w][lane];
-                const float4 b0 = S.pend_b0[w][lane];
-                const float4 b1 = S.pend_b1[w][lane];
+                ng.cm = S.pend_cm[w][row];
+                const float4 b0 = S.pend_b0[w][row];
+                const float4 b1 = S.pend_b1[w][row];
                 ng.bmin = make_float3(b0.x, b0.y, b0.z);
                 ng.bmax = make_float3(b1.x, b1.y, b1.z);
                 ng.count = __float_as_uint(b0.w);
                 mac_features(S.geom[w], ng, feat);
             }
-            mac_stage_features(mw, w, lane, feat);
-            const float pred = mac_infer_warp(mw, w, lane);
+            S.pend_b0[w][row] = make_float4(__uint_as_float(pack_bf16x2(feat[0], feat[1])),
+                                            __uint_as_float(pack_bf16x2(feat[2], feat[3])),
+                                            __uint_as_float(pack_bf16x2(feat[4], feat[5])),
+                                            __uint_as_float(pack_bf16x2(feat[6], feat[7])));
+            *reinterpret_cast<float2*>(&S.pend_b1[w][row]) =
+                make_float2(__uint_as_float(pack_bf16x2(feat[8], feat[9])), __uint_as_float(pack_bf16x2(feat[10], feat[11])));
+            const uint32_t* x0 = reinterpret_cast<const uint32_t*>(&S.pend_b0[w][np]);
+            const uint32_t* x1 = reinterpret_cast<const uint32_t*>(&S.pend_b1[w][np]);
+            const float pred = mac_forward_rows<false>(
+                mw, lane,
+                [=](uint32_t r, uint32_t k) { return k < 4 ? x0[4 * r + k] : k < 6 ? x1[4 * r + k - 4] : 0u; }, nullptr);
             evals += cnt;
             // the row's node, read back after the network (fewer live registers)
             if (lane < cnt) {
                 kind = pred < tol ? 1u : 2u;
-                cm = S.pend_cm[w][lane];
-                id = __float_as_uint(S.pend_b1[w][lane].w);
-                const uint2 kids = S.pend_kids[w][lane];
+                cm = S.pend_cm[w][row];
+                id = __float_as_uint(S.pend_b1[w][row].w);
+                const uint2 kids = S.pend_kids[w][row];
                 ca = kids.x;
                 cb = kids.y;
             }
-            const uint32_t rest = np - cnt;
-            __syncwarp();
-            if (lane < rest) {
-                S.pend_cm[w][lane] = S.pend_cm[w][32 + lane];
-                S.pend_b0[w][lane] = S.pend_b0[w][32 + lane];
-                S.pend_b1[w][lane] = S.pend_b1[w][32 + lane];
-                S.pend_kids[w][lane] = S.pend_kids[w][32 + lane];
-            }
-            np = rest;
             __syncwarp();
         } else {
             const uint32_t k = min(sp, 32u);
@@ -645,20 +640,16 @@ __global__ __launch_bounds__(GroupShape<MODE>::threads, GroupMinBlocks<MODE, FOR
     }  // groups
 }
 
-static size_t group_smem(int mode) {
-    return mode == GM_LEARNED ? GroupCfg<GM_LEARNED>::smem : mode == GM_RECORD ? GroupCfg<GM_RECORD>::smem
-                                                                              : GroupCfg<GM_THETA>::smem;
-}
-
 // resident blocks per SM of each instance (set up once per process)
 static int g_blocks_per_sm[3][3];
 
 template <int MODE, int FORM>
 static void set_smem() {
-    cudaFuncSetAttribute(k_walk_group<MODE, FORM>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)group_smem(MODE));
+    cudaFuncSetAttribute(k_walk_group<MODE, FORM>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                         (int)GroupCfg<MODE, FORM>::smem);
     int nb = 0;
     if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, k_walk_group<MODE, FORM>, GroupShape<MODE>::threads,
-                                                      group_smem(MODE)) !=
+                                                      GroupCfg<MODE, FORM>::smem) !=
             cudaSuccess ||
         nb < 1)
         nb = 1;
@@ -686,7 +677,7 @@ static void launch_mode(const StepBuffers& b, const MacDeviceWeights& mw, cudaSt
     const uint32_t need = (b.N + threads - 1) / threads + 1;
     uint32_t blocks = b.num_sms * (uint32_t)g_blocks_per_sm[MODE][FORM];
     if (blocks > need) blocks = need;
-    k_walk_group<MODE, FORM><<<blocks, threads, group_smem(MODE), s>>>(b, mw);
+    k_walk_group<MODE, FORM><<<blocks, threads, GroupCfg<MODE, FORM>::smem, s>>>(b, mw);
 }
 
 template <int MODE>

@@ -112,7 +112,8 @@ __device__ __forceinline__ float box_gap2(const GroupGeom& g, const NodeGeom& n)
 __device__ __forceinline__ float group_soft_dist2(const GroupGeom& g, const NodeGeom& n) {
     const float dx = n.cm.x - g.cx, dy = n.cm.y - g.cy, dz = n.cm.z - g.cz;
     const float D2 = dx * dx + dy * dy + dz * dz;
-    const float D = D2 > 0.0f ? D2 * rsqrtf(D2) : 0.0f;
+    // a squared distance below the normal numbers counts as (less than) 1e-19
+    const float D = D2 * rsqrt_normal(fmaxf(D2, GBH_MIN_NORMAL));
     const float d = fmaxf(D - g.R, 0.0f);
     return d * d + g.soft;
 }
@@ -133,7 +134,7 @@ __device__ __forceinline__ bool group_theta_accept(const GroupGeom& g, const Nod
 // band's two thetas.
 __device__ __forceinline__ float group_rho(const GroupGeom& g, const NodeGeom& n) {
     const float den2 = group_soft_dist2(g, n);
-    return (den2 > 0.0f && box_gap2(g, n) > 0.0f) ? node_half(n) * rsqrtf(den2) : __int_as_float(0x7f800000);
+    return (den2 > 0.0f && box_gap2(g, n) > 0.0f) ? node_half(n) * rsqrt_normal(fmaxf(den2, GBH_MIN_NORMAL)) : __int_as_float(0x7f800000);
 }
 
 __device__ __forceinline__ float clampf(float x, float lo, float hi) { return fminf(fmaxf(x, lo), hi); }
@@ -165,10 +166,10 @@ __device__ __forceinline__ void mac_features(const GroupGeom& g, const NodeGeom&
     const float h = fmaxf(0.5f * emax, 1e-30f);
     const float dx = n.cm.x - g.cx, dy = n.cm.y - g.cy, dz = n.cm.z - g.cz;
     const float d2 = fmaxf(dx * dx + dy * dy + dz * dz, 1e-36f);
-    const float inv_d = rsqrtf(d2);
-    const float l_d2 = __log2f(d2);
+    const float inv_d = rsqrt_normal(d2);
+    const float l_d2 = log2_normal(d2);
     const float l_d = 0.5f * l_d2;
-    const float l_h = __log2f(h);
+    const float l_h = log2_normal(h);
     const float l_R = fmaxf(g.l_R, l_d - 19.931568f);  // R >= 1e-6 d
     const float R = fmaxf(g.R, 1e-6f * d2 * inv_d);
     const float inv_h = __fdividef(1.0f, h);
@@ -176,18 +177,18 @@ __device__ __forceinline__ void mac_features(const GroupGeom& g, const NodeGeom&
     const float oy = n.cm.y - 0.5f * (n.bmin.y + n.bmax.y);
     const float oz = n.cm.z - 0.5f * (n.bmin.z + n.bmax.z);
     const float off2 = ox * ox + oy * oy + oz * oz;
-    const float inv_off = rsqrtf(fmaxf(off2, 1e-36f));
+    const float inv_off = rsqrt_normal(fmaxf(off2, 1e-36f));
     const float inv_emax = emax > 0.f ? __fdividef(1.0f, emax) : 0.f;
     const float gap2 = box_gap2(g, n);
     f[0] = clampf(l_h - l_d, -24.f, 8.f) * 0.125f;
     f[1] = clampf(l_R - l_d, -24.f, 8.f) * 0.125f;
-    f[2] = __log2f(clampf(1.0f - R * inv_d, 1e-4f, 1.0f)) * 0.125f;
+    f[2] = log2_normal(clampf(1.0f - R * inv_d, 1e-4f, 1.0f)) * 0.125f;
     f[3] = clampf(off2 * inv_off * inv_h, 0.f, 2.f);
     f[4] = emax > 0.f ? emin * inv_emax : 1.f;
     f[5] = emax > 0.f ? emid * inv_emax : 1.f;
-    f[6] = __log2f((float)min(max(n.count, 1u), 1u << 16)) * (1.0f / 16.0f);
+    f[6] = log2_normal((float)min(max(n.count, 1u), 1u << 16)) * (1.0f / 16.0f);
     f[7] = off2 > 1e-36f ? clampf((ox * dx + oy * dy + oz * dz) * inv_off * inv_d, -1.f, 1.f) : 0.f;
-    f[8] = clampf(g.l_g_aref + __log2f(n.cm.w) - __log2f(d2 + g.soft), -32.f, 32.f) * (1.0f / 16.0f);
+    f[8] = clampf(g.l_g_aref + __log2f(n.cm.w) - log2_normal(d2 + g.soft), -32.f, 32.f) * (1.0f / 16.0f);
     f[9] = clampf(g.l_soft - l_d2, -48.f, 8.f) * (1.0f / 16.0f);
     f[10] = clampf(l_h - l_R, -16.f, 16.f) * 0.125f;
     f[11] = clampf(0.5f * __log2f(fmaxf(gap2, 1e-12f * h * h)) - l_h, -20.f, 8.f) * 0.125f;
@@ -235,22 +236,21 @@ struct MacActs {
 // The two 16-row m-tiles go through all three layers one after the other,
 // which keeps the live accumulators to one tile's.  KEEP also returns the
 // FP32 activations (training); inference fuses ReLU into the BF16 packing.
-template <bool KEEP>
-__device__ __forceinline__ float mac_forward_warp(const MacDeviceWeights& mw, uint32_t warp, uint32_t lane,
-                                                  MacActs* acts) {
+// `rows(r, k)` gives word k (features 2 k and 2 k + 1, BF16) of staged row r.
+template <bool KEEP, class Rows>
+__device__ __forceinline__ float mac_forward_rows(const MacDeviceWeights& mw, uint32_t lane, Rows rows, MacActs* acts) {
     __syncwarp();
     const uint32_t gid = lane >> 2, tig = lane & 3;
     const uint4* F4 = reinterpret_cast<const uint4*>(mw.smem_frag) + lane;  // chunk c at F4[32 c]
-    const uint32_t* X = reinterpret_cast<const uint32_t*>(mw.smem_x + (size_t)warp * mw.x_rows * 16);
     auto act = [&](float x0, float x1) { return KEEP ? pack_bf16x2(x0, x1) : pack_bf16x2_relu(x0, x1); };
     float out[2][2];
 #pragma unroll
     for (int mt = 0; mt < 2; ++mt) {
         uint32_t a[4];
-        a[0] = X[(16 * mt + gid) * 8 + tig];
-        a[1] = X[(16 * mt + gid + 8) * 8 + tig];
-        a[2] = X[(16 * mt + gid) * 8 + tig + 4];
-        a[3] = X[(16 * mt + gid + 8) * 8 + tig + 4];
+        a[0] = rows(16 * mt + gid, tig);
+        a[1] = rows(16 * mt + gid + 8, tig);
+        a[2] = rows(16 * mt + gid, tig + 4);
+        a[3] = rows(16 * mt + gid + 8, tig + 4);
         // layer 1: 16 x 12(16) by 12(16) x 32, ReLU; n-tiles 2 ks, 2 ks + 1
         uint32_t a2[2][4];  // layer-2 A fragments [k-step]
 #pragma unroll
@@ -318,6 +318,14 @@ __device__ __forceinline__ float mac_forward_warp(const MacDeviceWeights& mw, ui
     const float v = sel == 0 ? v00 : sel == 1 ? v01 : sel == 2 ? v10 : v11;
     const float b3 = __uint_as_float(mw.smem_frag[(11 * 32 + lane) * 4]);
     return v + b3;
+}
+
+// the same on the rows that mac_stage_features staged
+template <bool KEEP>
+__device__ __forceinline__ float mac_forward_warp(const MacDeviceWeights& mw, uint32_t warp, uint32_t lane,
+                                                  MacActs* acts) {
+    const uint32_t* X = reinterpret_cast<const uint32_t*>(mw.smem_x + (size_t)warp * mw.x_rows * 16);
+    return mac_forward_rows<KEEP>(mw, lane, [X](uint32_t r, uint32_t k) { return X[r * 8 + k]; }, acts);
 }
 
 __device__ __forceinline__ float mac_infer_warp(const MacDeviceWeights& mw, uint32_t warp, uint32_t lane) {
