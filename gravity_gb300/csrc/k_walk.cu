@@ -37,35 +37,49 @@
 // two thirds are accepted or opened by all of the warp's bodies alike, which
 // one lane can tell from the box of the 32 bodies.  So a round pops up to 16
 // opened nodes and classifies their 32 children, one per lane (about 60
-// instructions for all of them); the force of a node on the bodies of its
-// mask then takes 17 instructions, and a node that the box leaves undecided
-// 23, force included.  A finer box (per 16, 8 or 4 bodies) leaves 309, 290 or
+// instructions for all of them); the force of a node on the bodies of its mask
+// and the test of a node that the box leaves undecided, force included, take
+// two nodes per packed FP32 instruction (17 and 23 instructions per node one
+// by one, about 9 and 14 in pairs).  A finer box (per 16, 8 or 4 bodies) leaves 309, 290 or
 // 267 of the 327 undecided nodes of a warp and was not worth its tests; 64
 // bodies per warp leave more undecided tests per body (485 against 654 for two
 // warps of 32, at twice the work each).
-// Walk stage, ms, before and after: 4,194,301-body mixture at theta 0.5 8.04 ->
-// 3.14; 2,097,152-body galaxy pair, precision form, 6.43 -> 2.50; 65,536-body
-// Plummer sphere 0.289 -> 0.092; 1,024 bodies 0.131 -> 0.045; 1,048,576-body
-// merge state at theta 0.7 0.457 -> 0.352.  Popping 32 nodes and classifying
-// both children of each in turn: 4.12 ms on the mixture.
+// Walk stage, ms, one node at a time -> classified in batches -> in pairs:
+// 4,194,301-body mixture at theta 0.5 8.04 -> 3.14 -> 2.88; 2,097,152-body
+// galaxy pair, precision form, 6.43 -> 2.50 -> 2.08; 1,048,576-body merge state
+// at theta 0.7 0.457 -> 0.352 -> 0.338; 65,536-body Plummer sphere 0.289 ->
+// 0.092 -> 0.080; 1,024 bodies 0.131 -> 0.045 -> 0.041.  Popping 32 nodes and
+// classifying both children of each in turn: 4.12 ms on the mixture.
 
 #define PW_THREADS 128
 #define PW_WARPS (PW_THREADS / 32)
 #define PW_LIST 64     // below 32 entries wait, one append adds up to 32
 #define PW_LOW 120     // above this many stack entries the walk turns depth-first
 #define PW_STACK 288   // PW_LOW + 63 (one batch) + 96 (a depth-first descent: 63 key + 30 tie-break levels)
-#define PW_BLOCKS 8     // resident blocks per SM (64 registers): 3.14 ms where 6 take 3.28, 5 3.62, 10 3.20
 
 enum PlainForm { PF_FP32 = 0, PF_PREC = 1, PF_MERGE = 2 };
+
+// Resident blocks per SM: seven (72 registers, 28 warps) where 8 and 6 take
+// 2.91 and 3.00 ms (4.2M mixture), 2.20 and 2.17 against 2.08 ms in the
+// precision form; eight in the merge form (0.338 against 0.346 ms).
+template <int FORM>
+struct PlainBlocks {
+    static constexpr int value = FORM == PF_MERGE ? 8 : 7;
+};
 
 // per-warp shared memory
 template <int FORM>
 struct PlainSmem {
-    float4 a_cm[PW_LIST];     // entries every lane of the mask interacts with: centre of mass, G x mass
-    float4 x_cm[PW_LIST];     // nodes to test body by body
-    uint2 x_half_mask[PW_LIST];
-    uint32_t x_id[PW_LIST];
+    // entries every lane of the mask interacts with, by component (the force
+    // loop takes two per packed instruction): centre of mass, G x mass
+    alignas(16) float a_x[PW_LIST], a_y[PW_LIST], a_z[PW_LIST], a_w[PW_LIST];
     uint32_t a_mask[PW_LIST];
+    // nodes to test body by body, with their half sides; the lanes of the mask
+    // that accepted an entry
+    float x_x[PW_LIST], x_y[PW_LIST], x_z[PW_LIST], x_w[PW_LIST], x_half[PW_LIST];
+    uint32_t x_mask[PW_LIST];
+    uint32_t x_id[PW_LIST];
+    uint32_t x_accept[32];
     uint2 stack[PW_STACK];    // (opened node's internal index, lanes that opened it)
     // merge and precision forms: leaves apart (mask; radius and slot, or residual)
     float4 l_cm[FORM == PF_FP32 ? 1 : PW_LIST];
@@ -80,7 +94,7 @@ struct PlainSmem {
 // (com - x_b) - lo_b for a node, and the leaf terms are summed with Kahan
 // compensation apart from the node terms.  Gravity only.
 template <int FORM>
-__global__ __launch_bounds__(PW_THREADS, PW_BLOCKS) void k_walk_plain(StepBuffers b) {
+__global__ __launch_bounds__(PW_THREADS, PlainBlocks<FORM>::value) void k_walk_plain(StepBuffers b) {
     constexpr bool PREC = FORM == PF_PREC;
     constexpr bool MERGE = FORM == PF_MERGE;
     __shared__ PlainSmem<FORM> s_warp[PW_WARPS];
@@ -162,6 +176,9 @@ __global__ __launch_bounds__(PW_THREADS, PW_BLOCKS) void k_walk_plain(StepBuffer
     uint32_t inter = 0, opened = 0;  // this lane's share of the warp's counts
     uint32_t sp = 0, max_sp = 0, an = 0, xn = 0, ln = 0;
     bool overflow = false;
+    // a candidate of this lane was not finite (or far out of range), or the
+    // softening does not keep the squared distances normal numbers
+    bool wild = !boxed || soft < GBH_MIN_NORMAL;
 
     // push the opened nodes of the lanes with mask != 0 (warp-collective)
     auto push = [&](uint32_t id, uint32_t mask) {
@@ -175,42 +192,53 @@ __global__ __launch_bounds__(PW_THREADS, PW_BLOCKS) void k_walk_plain(StepBuffer
         opened += __popc(mask & owners);
         sp += cnt;
     };
-    // forces of list A's last `cnt` entries on the lanes of each entry's mask
-    auto flush_a = [&](uint32_t cnt) {
-        __syncwarp();
-        an -= cnt;
-        const float4* cmv = S.a_cm + an;
-        const uint32_t* mv = S.a_mask + an;
-        if (want_pot) {
-            for (uint32_t j = 0; j < cnt; ++j) {
-                const float4 c = cmv[j];
-                float rx = c.x - pm.x, ry = c.y - pm.y, rz = c.z - pm.z;
-                if (PREC) rx = rx - lo_b.x, ry = ry - lo_b.y, rz = rz - lo_b.z;
-                const float inv = rsqrtf(__fmaf_rn(rz, rz, __fmaf_rn(ry, ry, __fmaf_rn(rx, rx, soft))));
-                if (mv[j] & bit) {
-                    const float f = c.w * (inv * inv * inv);
-                    ax = __fmaf_rn(f, rx, ax);
-                    ay = __fmaf_rn(f, ry, ay);
-                    az = __fmaf_rn(f, rz, az);
-                    pot = __fmaf_rn(-c.w, inv, pot);
-                }
-            }
-        } else {
-#pragma unroll 4
-            for (uint32_t j = 0; j < cnt; ++j) {
-                const float4 c = cmv[j];
-                float rx = c.x - pm.x, ry = c.y - pm.y, rz = c.z - pm.z;
-                if (PREC) rx = rx - lo_b.x, ry = ry - lo_b.y, rz = rz - lo_b.z;
-                const float inv = rsqrtf(__fmaf_rn(rz, rz, __fmaf_rn(ry, ry, __fmaf_rn(rx, rx, soft))));
-                const float f = c.w * (inv * inv * inv);
-                if (mv[j] & bit) {
-                    ax = __fmaf_rn(f, rx, ax);
-                    ay = __fmaf_rn(f, ry, ay);
-                    az = __fmaf_rn(f, rz, az);
-                }
+    // forces of list A's entries [0, cnt) on the lanes of each entry's mask, one
+    // by one: with the potential, or where an entry's offset may not be finite
+    // (times the zero of a masked lane it would not vanish)
+    auto flush_a_single = [&](uint32_t cnt) {
+        for (uint32_t j = 0; j < cnt; ++j) {
+            float rx = S.a_x[j] - pm.x, ry = S.a_y[j] - pm.y, rz = S.a_z[j] - pm.z;
+            const float m = S.a_w[j];
+            if (PREC) rx = rx - lo_b.x, ry = ry - lo_b.y, rz = rz - lo_b.z;
+            const float inv = rsqrtf(__fmaf_rn(rz, rz, __fmaf_rn(ry, ry, __fmaf_rn(rx, rx, soft))));
+            const float f = m * (inv * inv * inv);
+            if (S.a_mask[j] & bit) {
+                ax = __fmaf_rn(f, rx, ax);
+                ay = __fmaf_rn(f, ry, ay);
+                az = __fmaf_rn(f, rz, az);
+                if (want_pot) pot = __fmaf_rn(-m, inv, pot);
             }
         }
-        __syncwarp();
+    };
+    // the same, cnt a multiple of four, two entries per packed instruction
+    auto flush_a = [&](uint32_t cnt) {
+        const float2 px = make_float2(-pm.x, -pm.x), py = make_float2(-pm.y, -pm.y), pz = make_float2(-pm.z, -pm.z);
+        const float2 lx = make_float2(-lo_b.x, -lo_b.x), ly = make_float2(-lo_b.y, -lo_b.y), lz = make_float2(-lo_b.z, -lo_b.z);
+        const float2 soft2 = make_float2(soft, soft);
+        float2 sx = make_float2(0.f, 0.f), sy = sx, sz = sx;
+        auto two = [&](float2 x, float2 y, float2 z, float2 m, uint32_t m0, uint32_t m1) {
+            float2 rx = __fadd2_rn(x, px), ry = __fadd2_rn(y, py), rz = __fadd2_rn(z, pz);
+            if (PREC) rx = __fadd2_rn(rx, lx), ry = __fadd2_rn(ry, ly), rz = __fadd2_rn(rz, lz);
+            const float2 rr = __ffma2_rn(rz, rz, __ffma2_rn(ry, ry, __ffma2_rn(rx, rx, soft2)));
+            const float2 inv = make_float2(rsqrt_normal(rr.x), rsqrt_normal(rr.y));
+            float2 f = __fmul2_rn(m, __fmul2_rn(__fmul2_rn(inv, inv), inv));
+            f.x = (m0 & bit) ? f.x : 0.0f;
+            f.y = (m1 & bit) ? f.y : 0.0f;
+            sx = __ffma2_rn(f, rx, sx);
+            sy = __ffma2_rn(f, ry, sy);
+            sz = __ffma2_rn(f, rz, sz);
+        };
+#pragma unroll 2
+        for (uint32_t j = 0; j < cnt; j += 4) {
+            const float4 x = *reinterpret_cast<const float4*>(S.a_x + j), y = *reinterpret_cast<const float4*>(S.a_y + j),
+                         z = *reinterpret_cast<const float4*>(S.a_z + j), m = *reinterpret_cast<const float4*>(S.a_w + j);
+            const uint4 mk = *reinterpret_cast<const uint4*>(S.a_mask + j);
+            two(make_float2(x.x, x.y), make_float2(y.x, y.y), make_float2(z.x, z.y), make_float2(m.x, m.y), mk.x, mk.y);
+            two(make_float2(x.z, x.w), make_float2(y.z, y.w), make_float2(z.z, z.w), make_float2(m.z, m.w), mk.z, mk.w);
+        }
+        ax += sx.x + sx.y;
+        ay += sy.x + sy.y;
+        az += sz.x + sz.y;
     };
     // the same for the leaves of the merge and precision forms
     auto flush_l = [&](uint32_t cnt) {
@@ -282,40 +310,62 @@ __global__ __launch_bounds__(PW_THREADS, PW_BLOCKS) void k_walk_plain(StepBuffer
         }
         __syncwarp();
     };
-    // list X's last `cnt` nodes, body by body: the accepting lanes take the
-    // force, the others' mask goes on the stack
-    auto test_x = [&](uint32_t cnt) {
-        __syncwarp();
-        xn -= cnt;
-        const float4* cmv = S.x_cm + xn;
-        const uint2* hv = S.x_half_mask + xn;
-        uint32_t mine = 0u;
-#pragma unroll 4
+    // list X's entries [0, cnt), body by body: the accepting lanes take the
+    // force, x_accept their mask; one by one as flush_a_single
+    auto test_x_single = [&](uint32_t cnt) {
         for (uint32_t j = 0; j < cnt; ++j) {
-            const float4 c = cmv[j];
-            const uint2 hm = hv[j];
-            float rx = c.x - pm.x, ry = c.y - pm.y, rz = c.z - pm.z;
+            float rx = S.x_x[j] - pm.x, ry = S.x_y[j] - pm.y, rz = S.x_z[j] - pm.z;
+            const float m = S.x_w[j];
             if (PREC) rx = rx - lo_b.x, ry = ry - lo_b.y, rz = rz - lo_b.z;
-            const float rr = __fmaf_rn(rz, rz, __fmaf_rn(ry, ry, rx * rx));
-            const float inv = rsqrtf(rr + soft);
-            const bool accept = __uint_as_float(hm.x) * inv < theta;
-            const bool me = hm.y & bit;
-            const float f = c.w * (inv * inv * inv);
-            if (me && accept) {
+            const float inv = rsqrtf(__fmaf_rn(rz, rz, __fmaf_rn(ry, ry, rx * rx)) + soft);
+            const bool accept = (S.x_mask[j] & bit) && S.x_half[j] * inv < theta;
+            const float f = m * (inv * inv * inv);
+            if (accept) {
                 ax = __fmaf_rn(f, rx, ax);
                 ay = __fmaf_rn(f, ry, ay);
                 az = __fmaf_rn(f, rz, az);
-                if (want_pot) pot = __fmaf_rn(-c.w, inv, pot);
+                if (want_pot) pot = __fmaf_rn(-m, inv, pot);
             }
-            const uint32_t om = __ballot_sync(0xffffffffu, me && !accept);
-            if (lane == j) mine = om;
+            const uint32_t am = __ballot_sync(0xffffffffu, accept);
+            if (lane == 0) S.x_accept[j] = am;
         }
-        uint32_t id = 0u;
-        if (lane < cnt) {
-            id = S.x_id[xn + lane];
-            inter += __popc(hv[lane].y & ~mine & owners);
+    };
+    // the same, cnt a multiple of four, two entries per packed instruction
+    auto test_x = [&](uint32_t cnt) {
+        const float2 px = make_float2(-pm.x, -pm.x), py = make_float2(-pm.y, -pm.y), pz = make_float2(-pm.z, -pm.z);
+        const float2 lx = make_float2(-lo_b.x, -lo_b.x), ly = make_float2(-lo_b.y, -lo_b.y), lz = make_float2(-lo_b.z, -lo_b.z);
+        const float2 soft2 = make_float2(soft, soft);
+        float2 sx = make_float2(0.f, 0.f), sy = sx, sz = sx;
+        auto two = [&](uint32_t j, float2 x, float2 y, float2 z, float2 m, float2 half, uint32_t m0, uint32_t m1) {
+            float2 rx = __fadd2_rn(x, px), ry = __fadd2_rn(y, py), rz = __fadd2_rn(z, pz);
+            if (PREC) rx = __fadd2_rn(rx, lx), ry = __fadd2_rn(ry, ly), rz = __fadd2_rn(rz, lz);
+            const float2 rr = __fadd2_rn(__ffma2_rn(rz, rz, __ffma2_rn(ry, ry, __fmul2_rn(rx, rx))), soft2);
+            const float2 inv = make_float2(rsqrt_normal(rr.x), rsqrt_normal(rr.y));
+            const float2 h = __fmul2_rn(half, inv);
+            const bool a0 = (m0 & bit) && h.x < theta, a1 = (m1 & bit) && h.y < theta;
+            float2 f = __fmul2_rn(m, __fmul2_rn(__fmul2_rn(inv, inv), inv));
+            f.x = a0 ? f.x : 0.0f;
+            f.y = a1 ? f.y : 0.0f;
+            sx = __ffma2_rn(f, rx, sx);
+            sy = __ffma2_rn(f, ry, sy);
+            sz = __ffma2_rn(f, rz, sz);
+            const uint32_t am0 = __ballot_sync(0xffffffffu, a0), am1 = __ballot_sync(0xffffffffu, a1);
+            if (lane == 0) *reinterpret_cast<uint2*>(S.x_accept + j) = make_uint2(am0, am1);
+        };
+#pragma unroll 2
+        for (uint32_t j = 0; j < cnt; j += 4) {
+            const float4 x = *reinterpret_cast<const float4*>(S.x_x + j), y = *reinterpret_cast<const float4*>(S.x_y + j),
+                         z = *reinterpret_cast<const float4*>(S.x_z + j), m = *reinterpret_cast<const float4*>(S.x_w + j),
+                         h = *reinterpret_cast<const float4*>(S.x_half + j);
+            const uint4 mk = *reinterpret_cast<const uint4*>(S.x_mask + j);
+            two(j, make_float2(x.x, x.y), make_float2(y.x, y.y), make_float2(z.x, z.y), make_float2(m.x, m.y),
+                make_float2(h.x, h.y), mk.x, mk.y);
+            two(j + 2, make_float2(x.z, x.w), make_float2(y.z, y.w), make_float2(z.z, z.w), make_float2(m.z, m.w),
+                make_float2(h.z, h.w), mk.z, mk.w);
         }
-        push(id, mine);
+        ax += sx.x + sx.y;
+        ay += sy.x + sy.y;
+        az += sz.x + sz.y;
     };
     // one candidate per lane (`m`: the lanes whose walk reached it): leaves
     // and nodes that every body of the box accepts to list A (leaves to L in
@@ -324,7 +374,7 @@ __global__ __launch_bounds__(PW_THREADS, PW_BLOCKS) void k_walk_plain(StepBuffer
     auto classify = [&](bool has, float4 cm, float half, uint32_t id, uint32_t m) {
         const bool leaf = has && id < N;
         bool accept = false, open = false;
-        if (has && !leaf) {
+        if (has) {
             const float ux = mnx - cm.x, uy = mny - cm.y, uz = mnz - cm.z;
             const float vx = cm.x - mxx, vy = cm.y - mxy, vz = cm.z - mxz;
             const float lx = fmaxf(fmaxf(ux, vx), 0.0f), ly = fmaxf(fmaxf(uy, vy), 0.0f), lz = fmaxf(fmaxf(uz, vz), 0.0f);
@@ -334,7 +384,8 @@ __global__ __launch_bounds__(PW_THREADS, PW_BLOCKS) void k_walk_plain(StepBuffer
             // a centre of mass that is not finite has no far2 below 1e30; the
             // small constants leave squares that lose bits to underflow to X
             const float h2 = half * half;
-            const bool ok = boxed && far2 < 1e30f;
+            const bool ok = !leaf && boxed && far2 < 1e30f;
+            wild = wild || !(far2 < 1e30f);
             accept = ok && h2 < __fmaf_rn(t2_accept, near2, -1e-33f);
             open = ok && h2 >= __fmaf_rn(t2_open, far2, 1e-33f);
         }
@@ -348,7 +399,10 @@ __global__ __launch_bounds__(PW_THREADS, PW_BLOCKS) void k_walk_plain(StepBuffer
         const uint32_t ba = __ballot_sync(0xffffffffu, to_a);
         if (to_a) {
             const uint32_t pos = an + __popc(ba & lanemask_lt());
-            S.a_cm[pos] = make_float4(cm.x, cm.y, cm.z, G * cm.w);
+            S.a_x[pos] = cm.x;
+            S.a_y[pos] = cm.y;
+            S.a_z[pos] = cm.z;
+            S.a_w[pos] = G * cm.w;
             S.a_mask[pos] = take;
         }
         an += __popc(ba);
@@ -356,8 +410,12 @@ __global__ __launch_bounds__(PW_THREADS, PW_BLOCKS) void k_walk_plain(StepBuffer
         const uint32_t bx = __ballot_sync(0xffffffffu, to_x);
         if (to_x) {
             const uint32_t pos = xn + __popc(bx & lanemask_lt());
-            S.x_cm[pos] = make_float4(cm.x, cm.y, cm.z, G * cm.w);
-            S.x_half_mask[pos] = make_uint2(__float_as_uint(half), m);
+            S.x_x[pos] = cm.x;
+            S.x_y[pos] = cm.y;
+            S.x_z[pos] = cm.z;
+            S.x_w[pos] = G * cm.w;
+            S.x_half[pos] = half;
+            S.x_mask[pos] = m;
             S.x_id[pos] = id;
         }
         xn += __popc(bx);
@@ -374,36 +432,113 @@ __global__ __launch_bounds__(PW_THREADS, PW_BLOCKS) void k_walk_plain(StepBuffer
                 }
             }
             ln += __popc(bl);
-            if (ln >= 32) flush_l(32);
         }
         push(id, open ? m : 0u);
-        if (an >= 32) flush_a(32);
-        if (xn >= 32) test_x(32);
     };
 
-    if (n > 1 && owners) {
-        const WalkRec root = *b.root_rec;  // bh_force.comp:53
-        classify(lane == 0, root.cm, root.half_side, N, everyone);
-        for (;;) {
-            // the undecided nodes before a pop when the stack is empty (the
-            // opened ones refill it) and, above PW_LOW entries, always: the
-            // walk then takes one node at a time, depth-first, so the stack
-            // holds what a tree of any height needs.  Testing them earlier,
-            // from 8 to 24 waiting ones at 8 to 48 stack entries, changed
-            // nothing (3.26 to 3.29 ms).
-            const bool low = sp > PW_LOW;
-            if (xn && (sp == 0 || low)) {
-                test_x(min(xn, 32u));
-                continue;
+    // one site for each of the parts above, so that the code stays in the
+    // instruction cache; every list holds fewer than 32 entries before an
+    // append, which adds up to 32
+    for (bool first = true; n > 1 && owners;) {
+        const bool end = !first && sp == 0 && xn == 0;
+        if (an >= 32 || (end && an)) {
+            __syncwarp();
+            const uint32_t cnt = min(an, 32u);
+            if (want_pot || __any_sync(0xffffffffu, wild)) {
+                flush_a_single(cnt);
+            } else {
+                // massless entries up to a multiple of four
+                const uint32_t pad = (4u - (cnt & 3u)) & 3u;
+                if (lane < pad) {
+                    S.a_x[cnt + lane] = S.a_x[0];
+                    S.a_y[cnt + lane] = S.a_y[0];
+                    S.a_z[cnt + lane] = S.a_z[0];
+                    S.a_w[cnt + lane] = 0.0f;
+                    S.a_mask[cnt + lane] = 0u;
+                }
+                __syncwarp();
+                flush_a(cnt + pad);
             }
-            if (sp == 0) break;
+            an -= cnt;
+            __syncwarp();
+            if (lane < an) {  // the remaining entries to the front
+                S.a_x[lane] = S.a_x[32 + lane];
+                S.a_y[lane] = S.a_y[32 + lane];
+                S.a_z[lane] = S.a_z[32 + lane];
+                S.a_w[lane] = S.a_w[32 + lane];
+                S.a_mask[lane] = S.a_mask[32 + lane];
+            }
+            __syncwarp();
+            continue;
+        }
+        if (FORM != PF_FP32 && (ln >= 32 || (end && ln))) {
+            flush_l(min(ln, 32u));
+            continue;
+        }
+        if (end) break;
+        // the undecided nodes when a full batch waits, when the stack is empty
+        // (the opened ones refill it) and, above PW_LOW entries, always: the
+        // walk then takes one node at a time, depth-first, so the stack holds
+        // what a tree of any height needs.  Testing them earlier, from 8 to 24
+        // waiting ones at 8 to 48 stack entries, changed nothing (3.26 to 3.29
+        // ms).
+        const bool low = sp > PW_LOW;
+        if (xn && (xn >= 32 || sp == 0 || low)) {
+            __syncwarp();
+            const uint32_t cnt = min(xn, 32u);
+            if (want_pot || __any_sync(0xffffffffu, wild)) {
+                test_x_single(cnt);
+            } else {
+                const uint32_t pad = (4u - (cnt & 3u)) & 3u;
+                if (lane < pad) {
+                    S.x_x[cnt + lane] = S.x_x[0];
+                    S.x_y[cnt + lane] = S.x_y[0];
+                    S.x_z[cnt + lane] = S.x_z[0];
+                    S.x_w[cnt + lane] = 0.0f;
+                    S.x_half[cnt + lane] = 0.0f;
+                    S.x_mask[cnt + lane] = 0u;
+                }
+                __syncwarp();
+                test_x(cnt + pad);
+            }
+            __syncwarp();
+            uint32_t id = 0u, opening = 0u;
+            if (lane < cnt) {
+                id = S.x_id[lane];
+                const uint32_t mask = S.x_mask[lane], accept = S.x_accept[lane];
+                opening = mask & ~accept;
+                inter += __popc(accept & owners);
+            }
+            push(id, opening);
+            xn -= cnt;
+            __syncwarp();
+            if (lane < xn) {  // the remaining entries to the front
+                S.x_x[lane] = S.x_x[32 + lane];
+                S.x_y[lane] = S.x_y[32 + lane];
+                S.x_z[lane] = S.x_z[32 + lane];
+                S.x_w[lane] = S.x_w[32 + lane];
+                S.x_half[lane] = S.x_half[32 + lane];
+                S.x_mask[lane] = S.x_mask[32 + lane];
+                S.x_id[lane] = S.x_id[32 + lane];
+            }
+            __syncwarp();
+            continue;
+        }
+        bool has;
+        uint32_t m = 0u;
+        float4 cm = make_float4(0.f, 0.f, 0.f, 0.f);
+        uint2 meta = make_uint2(0u, 0u);
+        if (first) {  // the root, bh_force.comp:53
+            has = lane == 0;
+            cm = b.root_rec->cm;
+            meta = make_uint2(__float_as_uint(b.root_rec->half_side), N);
+            m = everyone;
+            first = false;
+        } else {
             max_sp = max(max_sp, sp);
             const uint32_t k = low ? 1u : min(sp, 16u);
             sp -= k;
-            const bool has = lane < 2 * k;
-            uint32_t m = 0u;
-            float4 cm = make_float4(0.f, 0.f, 0.f, 0.f);
-            uint2 meta = make_uint2(0u, 0u);
+            has = lane < 2 * k;
             __syncwarp();
             if (has) {  // lane l: child l & 1 of popped node l / 2
                 const uint2 e = S.stack[sp + (lane >> 1)];
@@ -413,10 +548,8 @@ __global__ __launch_bounds__(PW_THREADS, PW_BLOCKS) void k_walk_plain(StepBuffer
                 meta = __ldg(reinterpret_cast<const uint2*>(q + 1));
             }
             __syncwarp();
-            classify(has, cm, __uint_as_float(meta.x), meta.y, m);
         }
-        if (an) flush_a(an);
-        if (FORM != PF_FP32 && ln) flush_l(ln);
+        classify(has, cm, __uint_as_float(meta.x), meta.y, m);
     }
     if (overflow && lane == 0) set_error(b.st, GBH_DEVERR_WALK_STACK);
 
