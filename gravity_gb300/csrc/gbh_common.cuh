@@ -139,8 +139,10 @@ struct StepBuffers {
     uint32_t* hist;         // [SORT_PASSES][SORT_RADIX]
     uint32_t* bucket_base;  // [SORT_PASSES][SORT_RADIX]
     uint32_t* lookback;     // [SORT_PASSES][sort_tiles_cap][SORT_RADIX]
+    uint32_t ticket_clear;  // 1: the build just cleared the group walk's ticket
     uint32_t N;
     uint32_t sort_tiles_cap;
+    uint32_t sort_items;  // items per thread of the sort's tiles (4, 8; else 16)
     uint32_t prep_tiles_cap;
     uint32_t num_sms;  // multiprocessors of the context's device (grid sizes of the persistent kernels)
     // sharded walk: this rank's share of the live bodies (world 1: all)
@@ -340,6 +342,7 @@ __device__ __forceinline__ void kahan_add(float& sum, float& c, float x) {
 void launch_reset(const StepBuffers& b, cudaStream_t s);
 void launch_prepare(const StepBuffers& b, cudaStream_t s);
 void launch_sort(const StepBuffers& b, cudaStream_t s);
+uint32_t sort_items_for(uint32_t n);
 // histograms for launch_sort when the keys come from elsewhere than the encode
 // pass (hist must be zero; also sets st->n_new = n)
 void launch_sort_hist(const uint64_t* keys, uint32_t n, uint32_t* hist, DevState* st, uint32_t num_sms,

@@ -99,6 +99,8 @@ StepBuffers ctx_buffers(const gbh_ctx* c) {
     b.lookback = c->lookback;
     b.N = c->N;
     b.sort_tiles_cap = c->sort_tiles_cap;
+    b.sort_items = c->sort_items;
+    b.ticket_clear = c->ticket_clear ? 1u : 0u;
     b.prep_tiles_cap = c->prep_tiles_cap;
     b.num_sms = c->num_sms;
     b.shard_rank = c->shard_rank;
@@ -123,17 +125,24 @@ int enqueue_reset(gbh_ctx* c) {
 int enqueue_prepare(gbh_ctx* c) {
     launch_prepare(ctx_buffers(c), c->stream);
     c->iin = 1 - c->iin;  // GPU.swapMortonAndIndexBuffers after the partition
+    c->lookback_clear = c->groups_clear = true;
     return check_launch(c, "prepare");
 }
 
 int enqueue_sort(gbh_ctx* c) {
-    CUDA_TRY(c, cudaMemsetAsync(c->lookback, 0, c->lookback_bytes, c->stream));
-    CUDA_TRY(c, cudaMemsetAsync(c->st->sort_tiles, 0, sizeof(c->st->sort_tiles), c->stream));
+    if (!c->lookback_clear) {
+        CUDA_TRY(c, cudaMemsetAsync(c->lookback, 0, c->lookback_bytes, c->stream));
+        CUDA_TRY(c, cudaMemsetAsync(c->st->sort_tiles, 0, sizeof(c->st->sort_tiles), c->stream));
+    }
+    c->lookback_clear = false;
     launch_sort(ctx_buffers(c), c->stream);
     return check_launch(c, "sort");
 }
 
 int enqueue_build(gbh_ctx* c) {
+    if (!c->groups_clear) CUDA_TRY(c, cudaMemsetAsync(&c->st->num_groups, 0, 4, c->stream));
+    c->groups_clear = false;
+    c->ticket_clear = true;
     launch_build(ctx_buffers(c), c->stream);
     // the group walks' start lists belong to the tree: built with it when a
     // group walk is selected (otherwise the group walk builds them itself)
@@ -152,6 +161,7 @@ int enqueue_walk(gbh_ctx* c) {
         launch_walk_plain(ctx_buffers(c), c->stream);
     } else {
         int rc = enqueue_walk_learned(c);
+        c->ticket_clear = false;
         if (rc) return rc;
     }
     return check_launch(c, "walk");
@@ -171,8 +181,15 @@ typedef int (*stage_fn)(gbh_ctx*);
 static const stage_fn k_stages[GBH_NUM_STAGES] = {enqueue_reset, enqueue_prepare, enqueue_sort, enqueue_build,
                                                   enqueue_fill,  enqueue_walk,    enqueue_merge, enqueue_swap};
 
+// A whole step's merge stage has nothing to do unless the step merges: its
+// reset emptied the queue and its walk emits no task.
+static bool stage_idle(const gbh_ctx* c, int stage) {
+    return k_stages[stage] == enqueue_merge && c->params_host.merging_collision_or_neither != GBH_MODE_MERGE;
+}
+
 static int enqueue_step(gbh_ctx* c) {
     for (int s = 0; s < GBH_NUM_STAGES; ++s) {
+        if (stage_idle(c, s)) continue;
         int rc = k_stages[s](c);
         if (rc) return rc;
     }
@@ -278,7 +295,8 @@ int gbh_create(gbh_ctx** out, uint32_t n, const float bounds[6], const gbh_units
     c->num_sms = (uint32_t)sms;
     c->N = n;
     c->prep_tiles_cap = (n + PREP_TILE - 1) / PREP_TILE;
-    c->sort_tiles_cap = (n + SORT_TILE - 1) / SORT_TILE;
+    c->sort_items = sort_items_for(n);
+    c->sort_tiles_cap = (n + SORT_THREADS * c->sort_items - 1) / (SORT_THREADS * c->sort_items);
     const uint32_t ni = n > 1 ? n - 1 : 1;
 
     ArenaPlan A;
@@ -351,7 +369,7 @@ int gbh_create(gbh_ctx** out, uint32_t n, const float bounds[6], const gbh_units
     c->bucket_base = (uint32_t*)(base + o_bbase);
     c->lookback = (uint32_t*)(base + o_lb);
 
-    sort_setup();
+    sort_setup(c->sort_items);
     group_walk_setup();
     fill_setup();
     e = cudaStreamCreateWithFlags(&c->stream, cudaStreamNonBlocking);
@@ -724,6 +742,7 @@ int gbh_step_n(gbh_ctx* c, const gbh_step_params* p, uint32_t count) {
             cudaError_t e = cudaStreamEndCapture(c->stream, &g);
             c->bin = bin0;
             c->iin = iin0;
+            c->lookback_clear = c->groups_clear = c->ticket_clear = false;  // captured, not run
             if (rc) {
                 if (g) cudaGraphDestroy(g);
                 return rc;
@@ -739,6 +758,7 @@ int gbh_step_n(gbh_ctx* c, const gbh_step_params* p, uint32_t count) {
         // the graph's build stage ran for this mode (the key holds it): the
         // start lists are current exactly when a group walk is selected
         c->paths_current = c->mac_mode != GBH_MAC_PLAIN;
+        c->lookback_clear = c->groups_clear = c->ticket_clear = false;
         // the step flips both the body buffers and the (morton, index) buffers
         c->bin = 1 - c->bin;
         c->iin = 1 - c->iin;
@@ -1035,7 +1055,7 @@ int gbh_step_profiled(gbh_ctx* c, const gbh_step_params* p, float ms_out[GBH_NUM
     for (int i = 0; i <= GBH_NUM_STAGES; ++i) CUDA_TRY(c, cudaEventCreate(&ev[i]));
     CUDA_TRY(c, cudaEventRecord(ev[0], c->stream));
     for (int s = 0; s < GBH_NUM_STAGES; ++s) {
-        rc = k_stages[s](c);
+        rc = stage_idle(c, s) ? GBH_OK : k_stages[s](c);
         if (rc) break;
         CUDA_TRY(c, cudaEventRecord(ev[s + 1], c->stream));
     }

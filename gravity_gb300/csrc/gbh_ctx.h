@@ -15,6 +15,7 @@ struct gbh_ctx {
     uint32_t N = 0;
     uint32_t prep_tiles_cap = 0;
     uint32_t sort_tiles_cap = 0;
+    uint32_t sort_items = 16;
     gbh_units units{};
     bool inited = false;
 
@@ -53,6 +54,11 @@ struct gbh_ctx {
     uint32_t* group_node = nullptr;
     uint32_t* group_path = nullptr;
     uint32_t group_path_cap = 0;
+    // cleared by the stage before, as every step leaves them: the sort's
+    // look-back words and tickets (compaction), the group count (compaction),
+    // the group walk's ticket (build).  A stage that finds its own not cleared
+    // (called again, or alone) clears it with a memset.
+    bool lookback_clear = false, groups_clear = false, ticket_clear = false;
     bool paths_current = false;  // the start lists describe the current tree (enqueue_build)
     uint32_t* tile_dead = nullptr;
     float* tile_aabb = nullptr;
@@ -111,6 +117,6 @@ struct gbh_ctx {
 StepBuffers ctx_buffers(const gbh_ctx* c);
 int enqueue_walk_learned(gbh_ctx* c);
 void mac_release(gbh_ctx* c);
-void sort_setup();
+void sort_setup(uint32_t items);
 void group_walk_setup();
 void fill_setup();

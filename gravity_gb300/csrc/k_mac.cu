@@ -439,6 +439,7 @@ static int mac_ensure_pairs(gbh_ctx* c, uint32_t cap) {
     MacState* m = c->mac;
     if (m->cap >= cap) return GBH_OK;
     mac_free_pairs(m);
+    sort_setup(SORT_ITEMS);  // the pairs' sort has tiles of its own
     const uint32_t tiles = (cap + SORT_TILE - 1) / SORT_TILE;
     MTRY(c, cudaMalloc(&m->feats, (size_t)cap * MAC_FEATURES * 4));
     MTRY(c, cudaMalloc(&m->labels, (size_t)cap * 4));
@@ -634,6 +635,7 @@ int gbh_mac_generate(gbh_ctx* c, const gbh_step_params* params, uint32_t max_pai
     if ((rc = enqueue_reset(c)) || (rc = enqueue_prepare(c)) || (rc = enqueue_sort(c)) || (rc = enqueue_build(c)) ||
         (rc = enqueue_fill(c)))
         return rc;
+    c->ticket_clear = false;  // the recording walks below run one after another
     launch_walk_plain(ctx_buffers(c), c->stream);
     MTRY(c, cudaGetLastError());
     // 2. record candidate pairs from a conservative and an aggressive group

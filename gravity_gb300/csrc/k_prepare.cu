@@ -25,7 +25,6 @@ __global__ void k_reset(StepBuffers b) {
     const gbh_step_params* p = b.params;
     DevState* st = b.st;
     for (uint32_t i = threadIdx.x; i < SORT_PASSES * SORT_RADIX; i += blockDim.x) b.hist[i] = 0;
-    if (threadIdx.x < SORT_PASSES) st->sort_tiles[threadIdx.x] = 0;
     if (threadIdx.x == 0) {
         b.mq->head = 0;
         b.mq->tail = 0;
@@ -81,6 +80,18 @@ __global__ __launch_bounds__(PREP_THREADS) void k_prep_count(StepBuffers b) {
     const uint32_t tile = blockIdx.x;
     const uint32_t base = tile * PREP_TILE;
     if (base >= n) return;
+    // clear the sort's look-back words of the tiles that begin in this block's
+    // slots, and its tickets: the sort then starts without a memset
+    {
+        const uint32_t tile_items = SORT_THREADS * b.sort_items;
+        const uint32_t t0 = (base + tile_items - 1) / tile_items;
+        const uint32_t t1 = min((min(base + PREP_TILE, n) + tile_items - 1) / tile_items, b.sort_tiles_cap);
+        for (uint32_t t = t0; t < t1; ++t)
+            for (uint32_t p = threadIdx.x / 64; p < SORT_PASSES; p += PREP_THREADS / 64)
+                reinterpret_cast<uint4*>(b.lookback + ((size_t)p * b.sort_tiles_cap + t) * SORT_RADIX)[threadIdx.x % 64] =
+                    make_uint4(0u, 0u, 0u, 0u);
+        if (tile == 0 && threadIdx.x < SORT_PASSES) b.st->sort_tiles[threadIdx.x] = 0;
+    }
     const bool dynamic = b.params->static_or_dynamic == GBH_BOUNDS_DYNAMIC;
     // positions in index order from the last walk when nothing changed them since
     const bool sorted = b.st->sorted_valid != 0u;
@@ -210,6 +221,7 @@ __global__ __launch_bounds__(1024) void k_prep_scan(StepBuffers b) {
         st->n_old = n;
         st->just_died = died;
         st->n_new = n - died;
+        st->num_groups = 0;  // the build counts them
         // decrementDeadBodies, bh_update.comp:29-34
         sim->num_bodies = n - died;
         sim->just_died = 0;

@@ -44,17 +44,15 @@ __global__ void k_sort_scan(StepBuffers b) {
     b.bucket_base[p * SORT_RADIX + d] = off + x - v;
 }
 
+template <int ITEMS>
 struct SortSmem {
     uint32_t warp_hist[SORT_THREADS / 32][SORT_RADIX + 1];  // +1: sentinel bucket of out-of-range items
-#ifdef SORT_RANK_MATCH
-    uint32_t match[SORT_THREADS / 32][SORT_RADIX + 1];       // per-warp digit masks of the ranking
-#endif
     uint32_t block_excl[SORT_RADIX + 1];
     uint32_t delta[SORT_RADIX];
     uint32_t warp_tot[SORT_THREADS / 32];
     uint32_t tile;
-    unsigned long long keys[SORT_TILE];
-    uint32_t vals[SORT_TILE];
+    unsigned long long keys[SORT_THREADS * ITEMS];
+    uint32_t vals[SORT_THREADS * ITEMS];
 };
 
 // Warp-level stable ranking of the items, item rounds in slot order: lanes
@@ -63,11 +61,11 @@ struct SortSmem {
 // leader reserves the group's ranks with a shared-memory atomic.  A warp's
 // shared memory atomics take effect in program order, so items stay in slot
 // order.
-template <uint32_t SHIFT, int BITS>
-__device__ __forceinline__ void rank_items(const uint64_t (&key)[SORT_ITEMS], uint32_t (&rank)[SORT_ITEMS],
+template <uint32_t SHIFT, int BITS, int ITEMS>
+__device__ __forceinline__ void rank_items(const uint64_t (&key)[ITEMS], uint32_t (&rank)[ITEMS],
                                            uint32_t* warp_hist, uint32_t lane, uint32_t seg, uint32_t n) {
 #pragma unroll
-    for (int i = 0; i < SORT_ITEMS; ++i) {
+    for (int i = 0; i < ITEMS; ++i) {
         uint32_t dig = (uint32_t)(key[i] >> SHIFT) & 0xFFu;
         if (BITS > 8 && seg + i * 32 + lane >= n) dig = SORT_RADIX;
         uint32_t peers = 0xffffffffu;
@@ -85,81 +83,50 @@ __device__ __forceinline__ void rank_items(const uint64_t (&key)[SORT_ITEMS], ui
     }
 }
 
-#ifdef SORT_RANK_MATCH
-// The same stable ranking with the peers found in shared memory: each lane
-// ORs its bit into its digit's word of a per-warp mask table, reads the word
-// back (the lanes with its digit), and the digit's lowest lane reserves the
-// group's ranks and clears the word.  One shared atomic per item instead of
-// eight ballots.
-template <uint32_t SHIFT, int BITS>
-__device__ __forceinline__ void rank_items_match(const uint64_t (&key)[SORT_ITEMS], uint32_t (&rank)[SORT_ITEMS],
-                                                 uint32_t* warp_hist, uint32_t* match, uint32_t lane, uint32_t seg,
-                                                 uint32_t n) {
-    const uint32_t bit = 1u << lane;
-#pragma unroll
-    for (int i = 0; i < SORT_ITEMS; ++i) {
-        uint32_t dig = (uint32_t)(key[i] >> SHIFT) & 0xFFu;
-        if (BITS > 8 && seg + i * 32 + lane >= n) dig = SORT_RADIX;
-        atomicOr(&match[dig], bit);
-        __syncwarp();
-        const uint32_t peers = match[dig];
-        const uint32_t leader = __ffs(peers) - 1;
-        const uint32_t before = __popc(peers & (bit - 1u));
-        uint32_t prev = 0;
-        __syncwarp();
-        if (lane == leader) {
-            prev = atomicAdd(&warp_hist[dig], (uint32_t)__popc(peers));
-            match[dig] = 0u;
-        }
-        rank[i] = __shfl_sync(0xffffffffu, prev, leader) + before;
-    }
-}
-#endif
-
 // One kernel instance per pass: the digit's bit offset is a constant.
-template <uint32_t PASS>
-__global__ __launch_bounds__(SORT_THREADS, 3) void k_sort_pass(StepBuffers b, const uint64_t* __restrict__ kin,
+// resident blocks per SM, by the shared memory of a tile
+template <int ITEMS>
+struct SortBlocks {
+    static constexpr int value = ITEMS == 16 ? 3 : ITEMS == 8 ? 5 : 6;
+};
+
+template <uint32_t PASS, int ITEMS>
+__global__ __launch_bounds__(SORT_THREADS, SortBlocks<ITEMS>::value) void k_sort_pass(StepBuffers b, const uint64_t* __restrict__ kin,
                                                                const uint32_t* __restrict__ vin, uint64_t* __restrict__ kout,
                                                                uint32_t* __restrict__ vout) {
     constexpr uint32_t pass = PASS;
+    constexpr uint32_t TILE = SORT_THREADS * ITEMS;
     extern __shared__ __align__(16) unsigned char smem_raw[];
-    SortSmem& S = *reinterpret_cast<SortSmem*>(smem_raw);
+    SortSmem<ITEMS>& S = *reinterpret_cast<SortSmem<ITEMS>*>(smem_raw);
     const uint32_t n = b.st->n_new;
     constexpr uint32_t shift = SORT_BITS * PASS;
     const uint32_t lane = lane_id(), w = threadIdx.x >> 5;
     if (threadIdx.x == 0) S.tile = atomicAdd(&b.st->sort_tiles[pass], 1u);
     for (uint32_t i = threadIdx.x; i < (SORT_THREADS / 32) * (SORT_RADIX + 1); i += SORT_THREADS) {
         (&S.warp_hist[0][0])[i] = 0;
-#ifdef SORT_RANK_MATCH
-        (&S.match[0][0])[i] = 0;
-#endif
     }
     __syncthreads();
     const uint32_t tile = S.tile;
-    const uint32_t base = tile * SORT_TILE;
+    const uint32_t base = tile * TILE;
     if (base >= n) return;
     uint32_t* lb = b.lookback + ((size_t)pass * b.sort_tiles_cap) * SORT_RADIX;
 
     // load: warp w owns slots [base + w*32*ITEMS, +32*ITEMS), item i of lane l at +i*32+l
-    const uint32_t seg = base + w * 32 * SORT_ITEMS;
-    const bool full = base + SORT_TILE <= n;  // uniform over the block
-    uint64_t key[SORT_ITEMS];
-    uint32_t val[SORT_ITEMS];
-    uint32_t rank[SORT_ITEMS];
+    const uint32_t seg = base + w * 32 * ITEMS;
+    const bool full = base + TILE <= n;  // uniform over the block
+    uint64_t key[ITEMS];
+    uint32_t val[ITEMS];
+    uint32_t rank[ITEMS];
     if (full) {
 #pragma unroll
-        for (int i = 0; i < SORT_ITEMS; ++i) {
+        for (int i = 0; i < ITEMS; ++i) {
             key[i] = kin[seg + i * 32 + lane];
             val[i] = vin[seg + i * 32 + lane];
         }
-#ifdef SORT_RANK_MATCH
-        rank_items_match<shift, 8>(key, rank, S.warp_hist[w], S.match[w], lane, seg, n);
-#else
         rank_items<shift, 8>(key, rank, S.warp_hist[w], lane, seg, n);
-#endif
     } else {
 #pragma unroll
-        for (int i = 0; i < SORT_ITEMS; ++i) {
+        for (int i = 0; i < ITEMS; ++i) {
             const uint32_t pos = seg + i * 32 + lane;
             if (pos < n) {
                 key[i] = kin[pos];
@@ -169,11 +136,7 @@ __global__ __launch_bounds__(SORT_THREADS, 3) void k_sort_pass(StepBuffers b, co
                 val[i] = 0;
             }
         }
-#ifdef SORT_RANK_MATCH
-        rank_items_match<shift, 9>(key, rank, S.warp_hist[w], S.match[w], lane, seg, n);
-#else
         rank_items<shift, 9>(key, rank, S.warp_hist[w], lane, seg, n);
-#endif
     }
     __syncthreads();
     // thread d: exclusive prefix of digit d over warps, tile total
@@ -212,7 +175,7 @@ __global__ __launch_bounds__(SORT_THREADS, 3) void k_sort_pass(StepBuffers b, co
     // the look-back: the items leave the registers, and the predecessors
     // have longer to publish their inclusive counts
 #pragma unroll
-    for (int i = 0; i < SORT_ITEMS; ++i) {
+    for (int i = 0; i < ITEMS; ++i) {
         const uint32_t pos = seg + i * 32 + lane;
         if (pos < n) {
             const uint32_t dg = (uint32_t)(key[i] >> shift) & 0xFFu;
@@ -266,7 +229,7 @@ __global__ __launch_bounds__(SORT_THREADS, 3) void k_sort_pass(StepBuffers b, co
     }
     S.delta[d] = b.bucket_base[pass * SORT_RADIX + d] + prefix - S.block_excl[d];
     __syncthreads();
-    const uint32_t valid = min((uint32_t)SORT_TILE, n - base);
+    const uint32_t valid = min((uint32_t)TILE, n - base);
     bool bad = false;
     for (uint32_t j = threadIdx.x; j < valid; j += SORT_THREADS) {
         const uint64_t k = S.keys[j];
@@ -305,32 +268,48 @@ void launch_sort_hist(const uint64_t* keys, uint32_t n, uint32_t* hist, DevState
     k_sort_hist<<<blocks > 0 ? blocks : 1, 256, 0, s>>>(keys, n, hist, st);
 }
 
-void sort_setup() {
-    cudaFuncSetAttribute(k_sort_pass<0>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(SortSmem));
-    cudaFuncSetAttribute(k_sort_pass<1>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(SortSmem));
-    cudaFuncSetAttribute(k_sort_pass<2>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(SortSmem));
-    cudaFuncSetAttribute(k_sort_pass<3>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(SortSmem));
-    cudaFuncSetAttribute(k_sort_pass<4>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(SortSmem));
-    cudaFuncSetAttribute(k_sort_pass<5>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(SortSmem));
-    cudaFuncSetAttribute(k_sort_pass<6>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(SortSmem));
-    cudaFuncSetAttribute(k_sort_pass<7>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(SortSmem));
+// Items per thread of a sort of up to `n` pairs.  A small sort is eight chains of
+// latency (load, rank item after item, look back, scatter), shorter with small
+// tiles, which also reach more SMs; a large one wants long runs per digit.
+// Sort stage of an eager step, us, with 4, 8 and 16 items per thread: 1,000
+// pairs 59, 58, 75; 16,000 64, 75, 91; 150,000 84, 87, 95; 300,000 105, 93, 108;
+// 600,000 140, 114, 110; 4.2M 518, 365, 326.
+uint32_t sort_items_for(uint32_t n) { return n <= 200000u ? 4u : n <= 500000u ? 8u : 16u; }
+
+typedef void (*sort_pass_fn)(StepBuffers, const uint64_t*, const uint32_t*, uint64_t*, uint32_t*);
+static_assert(SORT_PASSES == 8, "one kernel instance per pass");
+template <int ITEMS>
+struct SortPasses {
+    static constexpr sort_pass_fn fn[SORT_PASSES] = {k_sort_pass<0, ITEMS>, k_sort_pass<1, ITEMS>, k_sort_pass<2, ITEMS>,
+                                                     k_sort_pass<3, ITEMS>, k_sort_pass<4, ITEMS>, k_sort_pass<5, ITEMS>,
+                                                     k_sort_pass<6, ITEMS>, k_sort_pass<7, ITEMS>};
+};
+
+template <int ITEMS>
+static void setup_passes() {
+    for (sort_pass_fn f : SortPasses<ITEMS>::fn)
+        cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(SortSmem<ITEMS>));
 }
 
-void launch_sort(const StepBuffers& b, cudaStream_t s) {
-    const size_t smem = sizeof(SortSmem);
-    k_sort_scan<<<SORT_PASSES, SORT_RADIX, 0, s>>>(b);
+void sort_setup(uint32_t items) {
+    if (items == 4)
+        setup_passes<4>();
+    else if (items == 8)
+        setup_passes<8>();
+    else
+        setup_passes<16>();
+}
+
+template <int ITEMS>
+static void launch_passes(const StepBuffers& b, cudaStream_t s) {
     // keys/index of the live bodies are in the *_in buffers (the compaction
     // swap already happened); 8 ping-pong passes through *_out end there again
     const uint64_t* kin = b.keys_in;
     const uint32_t* vin = b.idx_in;
     uint64_t* kt = b.keys_out;
     uint32_t* vt = b.idx_out;
-    static_assert(SORT_PASSES == 8, "one kernel instance per pass");
-    void (*const kernels[SORT_PASSES])(StepBuffers, const uint64_t*, const uint32_t*, uint64_t*, uint32_t*) = {
-        k_sort_pass<0>, k_sort_pass<1>, k_sort_pass<2>, k_sort_pass<3>,
-        k_sort_pass<4>, k_sort_pass<5>, k_sort_pass<6>, k_sort_pass<7>};
-    for (uint32_t p = 0; p < SORT_PASSES; ++p) {
-        kernels[p]<<<b.sort_tiles_cap, SORT_THREADS, smem, s>>>(b, kin, vin, kt, vt);
+    for (sort_pass_fn f : SortPasses<ITEMS>::fn) {
+        f<<<b.sort_tiles_cap, SORT_THREADS, sizeof(SortSmem<ITEMS>), s>>>(b, kin, vin, kt, vt);
         const uint64_t* nk = kt;
         const uint32_t* nv = vt;
         kt = const_cast<uint64_t*>(kin);
@@ -338,4 +317,14 @@ void launch_sort(const StepBuffers& b, cudaStream_t s) {
         kin = nk;
         vin = nv;
     }
+}
+
+void launch_sort(const StepBuffers& b, cudaStream_t s) {
+    k_sort_scan<<<SORT_PASSES, SORT_RADIX, 0, s>>>(b);
+    if (b.sort_items == 4)
+        launch_passes<4>(b, s);
+    else if (b.sort_items == 8)
+        launch_passes<8>(b, s);
+    else
+        launch_passes<16>(b, s);
 }

@@ -29,7 +29,7 @@
 
 #include "gbh_common.cuh"
 
-void sort_setup();  // k_sort.cu
+void sort_setup(uint32_t items);  // k_sort.cu
 
 #define NOALLOC_MAX_PAIRS (1u << 20)
 #define NOALLOC_TILES ((NOALLOC_MAX_PAIRS + SORT_TILE - 1) / SORT_TILE)
@@ -71,7 +71,7 @@ static const NoAllocDevice* setup_current_device(int* status) {
             *status = GBH_ERR_CUDA;
             return nullptr;
         }
-        sort_setup();
+        sort_setup(SORT_ITEMS);
         d.num_sms = (uint32_t)sms;
         d.scratch = static_cast<NoAllocScratch*>(p);
     }

@@ -60,6 +60,7 @@ __global__ __launch_bounds__(256) void k_build(StepBuffers b) {
     const uint32_t N = b.N;
     const uint32_t gid = blockIdx.x * blockDim.x + threadIdx.x;
     const uint64_t* keys = b.keys_in;
+    if (gid == 0) b.st->group_next = 0;  // the group walk's ticket
     if (n <= 1) {
         if (n == 1 && gid == 0) {
             // single body, bh_tree.comp:46-62: root with one child, bodiesContained 0,
@@ -194,7 +195,6 @@ void launch_group_paths(const StepBuffers& b, cudaStream_t s) {
 
 void launch_build(const StepBuffers& b, cudaStream_t s) {
     const uint32_t nodes = b.N > 1 ? b.N - 1 : 1;
-    cudaMemsetAsync(&b.st->num_groups, 0, 4, s);
     k_build<<<(nodes + 255) / 256, 256, 0, s>>>(b);
 }
 

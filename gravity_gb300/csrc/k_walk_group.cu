@@ -671,7 +671,7 @@ static void launch_mode(const StepBuffers& b, const MacDeviceWeights& mw, cudaSt
     // the step's walks find the start lists built with the tree
     // (enqueue_build); the recording walk builds its own
     if (MODE == GM_RECORD) launch_group_paths(b, s);
-    cudaMemsetAsync(&b.st->group_next, 0, 4, s);
+    if (!b.ticket_clear) cudaMemsetAsync(&b.st->group_next, 0, 4, s);
     // persistent: the blocks that fit at once (no more than the groups need)
     constexpr uint32_t threads = GroupShape<MODE>::threads;
     const uint32_t need = (b.N + threads - 1) / threads + 1;
