@@ -37,18 +37,12 @@ __device__ __forceinline__ int safe_lcp(const uint64_t* __restrict__ keys, int n
 // counter update per warp.
 __device__ __forceinline__ void emit_groups(const StepBuffers& b, uint32_t k, const uint2 (&mine)[2],
                                             const uint32_t (&node)[2]) {
-    const uint32_t lane = lane_id();
-    uint32_t incl = k;
-#pragma unroll
-    for (int o = 1; o < 32; o <<= 1) {
-        const uint32_t y = __shfl_up_sync(0xffffffffu, incl, o);
-        if (lane >= (uint32_t)o) incl += y;
-    }
-    const uint32_t total = __shfl_sync(0xffffffffu, incl, 31);
+    const uint32_t one = __ballot_sync(0xffffffffu, k > 0), two = __ballot_sync(0xffffffffu, k > 1);
+    if (!one) return;
     uint32_t base = 0;
-    if (lane == 31 && total) base = atomicAdd(&b.st->num_groups, total);
-    base = __shfl_sync(0xffffffffu, base, 31);
-    const uint32_t first = base + incl - k;
+    if (lane_id() == 0) base = atomicAdd(&b.st->num_groups, (uint32_t)(__popc(one) + __popc(two)));
+    base = __shfl_sync(0xffffffffu, base, 0);
+    const uint32_t first = base + __popc(one & lanemask_lt()) + __popc(two & lanemask_lt());
     for (uint32_t q = 0; q < k; ++q) {
         b.groups[first + q] = mine[q];
         b.group_node[first + q] = node[q];
@@ -83,22 +77,37 @@ __global__ __launch_bounds__(256) void k_build(StepBuffers b) {
     uint32_t k = 0;
     if (gid < n - 1) {
     const int i = (int)gid, ni = (int)n;
+    const uint64_t ki = keys[i];
     const int lcp_r = safe_lcp(keys, ni, i, i + 1);
     const int lcp_l = safe_lcp(keys, ni, i, i - 1);
     const int d = (lcp_l > lcp_r) ? -1 : 1;
-    const int delta_min = safe_lcp(keys, ni, i, i - d);
+    // The searches ask whether lcp(i, j) > delta for a fixed delta: j lies in
+    // the range and the first delta + 1 bits of (key, index) agree with i's.
+    // As a mask that is 4 instructions where the prefix length itself takes a
+    // dozen; a warp runs as long as its longest search, about 40 probes.
+    // Build stage at 16.8M bodies (with the start lists, 0.07): 0.53 -> 0.42 ms;
+    // 4.2M bodies without them 0.128 -> 0.096.
+    auto longer_than = [&](int delta) {
+        const int bits = delta + 1;
+        const uint64_t key_mask = bits >= 64 ? ~0ull : bits <= 0 ? 0ull : ~0ull << (64 - bits);
+        const uint32_t idx_mask = bits <= 64 ? 0u : bits >= 96 ? ~0u : ~0u << (96 - bits);
+        return [=](int j) {
+            return (uint32_t)j < (uint32_t)ni && ((ki ^ keys[j]) & key_mask) == 0ull && (((uint32_t)i ^ (uint32_t)j) & idx_mask) == 0u;
+        };
+    };
+    const auto beyond = longer_than(min(lcp_r, lcp_l));
     int lmax = 2;
-    while (safe_lcp(keys, ni, i, i + d * lmax) > delta_min) lmax *= 2;
+    while (beyond(i + d * lmax)) lmax *= 2;
     int l = 0;
-    for (int t = lmax / 2; t > 0; t /= 2)
-        if (safe_lcp(keys, ni, i, i + d * (l + t)) > delta_min) l += t;
+    for (int t = lmax >> 1; t > 0; t >>= 1)
+        if (beyond(i + d * (l + t))) l += t;
     const int j = i + l * d;
-    const int delta_node = safe_lcp(keys, ni, i, j);
+    const auto within = longer_than(safe_lcp(keys, ni, i, j));
     int s = 0;
     int t = l;
     while (t > 1) {
-        t = (t + 1) / 2;
-        if (safe_lcp(keys, ni, i, i + (s + t) * d) > delta_node) s += t;
+        t = (t + 1) >> 1;
+        if (within(i + (s + t) * d)) s += t;
     }
     const int gamma = i + s * d + min(d, 0);
     const int mn = min(i, j), mx = max(i, j);
