@@ -213,6 +213,45 @@ __device__ __forceinline__ uint64_t morton_encode64(const double* p64, const flo
     return (expand_bits21(q[0]) << 2) | (expand_bits21(q[1]) << 1) | expand_bits21(q[2]);
 }
 
+// What the fixed-point form below needs of the box, once per block: min, max
+// (FP64) and 2097151 / extent per axis.
+struct MortonBox64 {
+    double lo[3], hi[3], scale[3];
+};
+
+__device__ __forceinline__ void morton_box64(MortonBox64& b, int k, const float* mn, const float* mx) {
+    b.lo[k] = mn[k];
+    b.hi[k] = mx[k];
+    b.scale[k] = 2097151.0 / fmax(b.hi[k] - b.lo[k], 1e-9);
+}
+
+// morton_encode64's key with 2 FP64 instructions per axis (its division and
+// the rest take about 20, at 64 cycles each per warp and scheduler).  (x - min)
+// times the rounded scale differs from the exact sequence by at most 2^21 x 2^-51
+// = 2^-30; added to 1.5 x 2^28 it stands in the low bits in units of 2^-24.
+// Unless the fraction lies within two units of a whole number, its floor is the
+// exact sequence's; otherwise, and outside the box, that sequence decides.
+// `pm` is the FP32 rounding of p64: strictly inside the box it needs no clamp.
+// Compaction and encode of 2.1M bodies in the precision form: 0.312 -> 0.090 ms.
+__device__ __forceinline__ uint64_t morton_encode64_fast(const double* p64, float4 pm, const MortonBox64& b,
+                                                         const float* mn, const float* mx) {
+    const double2 xy = *reinterpret_cast<const double2*>(p64);
+    const double p[3] = {xy.x, xy.y, p64[2]};
+    const float f[3] = {pm.x, pm.y, pm.z};
+    uint32_t q[3];
+    bool sure = true;
+#pragma unroll
+    for (int k = 0; k < 3; ++k) {
+        const long long fixed = __double_as_longlong(fma(p[k] - b.lo[k], b.scale[k], 402653184.0)) -
+                                __double_as_longlong(402653184.0);
+        const uint32_t frac = (uint32_t)fixed & 0xFFFFFFu;
+        q[k] = (uint32_t)(fixed >> 24);
+        sure = sure && f[k] > mn[k] && f[k] < mx[k] && frac >= 2u && frac <= 0xFFFFFDu;
+    }
+    if (!sure) return morton_encode64(p64, mn, mx);
+    return (expand_bits21(q[0]) << 2) | (expand_bits21(q[1]) << 1) | expand_bits21(q[2]);
+}
+
 // radius(Body), common.glsl:228-230
 __device__ __forceinline__ float body_radius(float body_len_const, float m, float rho) {
     return body_len_const * powf(m / rho, 1.0f / 3.0f);

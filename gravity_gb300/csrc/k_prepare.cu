@@ -281,10 +281,12 @@ __global__ __launch_bounds__(PREP_THREADS) void k_prep_scatter(StepBuffers b) {
     __shared__ uint32_t s_hist[SORT_PASSES * SORT_RADIX];
     __shared__ uint32_t s_cnt[PREP_ITEMS][PREP_THREADS / 32];
     __shared__ float s_mn[3], s_mx[3];
+    __shared__ MortonBox64 s_box64;
     for (uint32_t i = threadIdx.x; i < SORT_PASSES * SORT_RADIX; i += PREP_THREADS) s_hist[i] = 0;
     if (threadIdx.x < 3) {
         s_mn[threadIdx.x] = b.sim->bounds_min[threadIdx.x];
         s_mx[threadIdx.x] = b.sim->bounds_max[threadIdx.x];
+        if (b.prec) morton_box64(s_box64, threadIdx.x, b.sim->bounds_min, b.sim->bounds_max);
     }
     const uint32_t lane = lane_id(), w = threadIdx.x >> 5;
     uint32_t bidx[PREP_ITEMS];
@@ -336,7 +338,7 @@ __global__ __launch_bounds__(PREP_THREADS) void k_prep_scatter(StepBuffers b) {
         if (alive[it]) {
             const uint32_t dst = alive_before_tile + arank;
             b.idx_out[dst] = bidx[it];
-            const uint64_t key = b.prec ? morton_encode64(b.pos64_in + 4 * (size_t)bidx[it], s_mn, s_mx)
+            const uint64_t key = b.prec ? morton_encode64_fast(b.pos64_in + 4 * (size_t)bidx[it], pm[it], s_box64, s_mn, s_mx)
                                         : morton_encode(pm[it].x, pm[it].y, pm[it].z, s_mn, s_mx);
             b.keys_out[dst] = key;
 #pragma unroll
