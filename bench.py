@@ -451,11 +451,11 @@ def train_out_of_sample(bh, args, local, held: list) -> dict:
 
 def kernels_per_step(mac_mode: int, merging: bool) -> int:
     """Kernels of this library launched by one step (the CUDA graph's kernel
-    nodes): reset 1, prepare 3, sort 1 + 8 passes, build 1 (it also lists the
+    nodes): prepare 3 (the first also resets), sort 8 passes, build 1 (it also lists the
     group walks' body groups; with the group and learned walks 2: then the
     groups' start lists), fill 2, walk 1, merge resolution 4 (in steps that
     merge), swap 0 (a pointer swap)."""
-    return 1 + 3 + 9 + (1 if mac_mode == abi.MAC_PLAIN else 2) + 2 + 1 + (4 if merging else 0)
+    return 3 + 8 + (1 if mac_mode == abi.MAC_PLAIN else 2) + 2 + 1 + (4 if merging else 0)
 
 
 def measure_e2e(bh, p_head, n, e2e_steps, local, dist=None) -> dict:

@@ -137,7 +137,6 @@ struct StepBuffers {
     float* tile_aabb;
     // sort scratch
     uint32_t* hist;         // [SORT_PASSES][SORT_RADIX]
-    uint32_t* bucket_base;  // [SORT_PASSES][SORT_RADIX]
     uint32_t* lookback;     // [SORT_PASSES][sort_tiles_cap][SORT_RADIX]
     uint32_t ticket_clear;  // 1: the build just cleared the group walk's ticket
     uint32_t N;
@@ -379,7 +378,7 @@ __device__ __forceinline__ void kahan_add(float& sum, float& c, float x) {
 
 // ---- launchers (host), one translation unit each -----------------------------
 void launch_reset(const StepBuffers& b, cudaStream_t s);
-void launch_prepare(const StepBuffers& b, cudaStream_t s);
+void launch_prepare(const StepBuffers& b, bool reset, cudaStream_t s);  // reset: launch_reset's work too
 void launch_sort(const StepBuffers& b, cudaStream_t s);
 uint32_t sort_items_for(uint32_t n);
 // histograms for launch_sort when the keys come from elsewhere than the encode

@@ -95,7 +95,6 @@ StepBuffers ctx_buffers(const gbh_ctx* c) {
     b.tile_dead = c->tile_dead;
     b.tile_aabb = c->tile_aabb;
     b.hist = c->hist;
-    b.bucket_base = c->bucket_base;
     b.lookback = c->lookback;
     b.N = c->N;
     b.sort_tiles_cap = c->sort_tiles_cap;
@@ -122,12 +121,14 @@ int enqueue_reset(gbh_ctx* c) {
     return check_launch(c, "reset");
 }
 
-int enqueue_prepare(gbh_ctx* c) {
-    launch_prepare(ctx_buffers(c), c->stream);
+static int enqueue_prepare_with(gbh_ctx* c, bool reset) {
+    launch_prepare(ctx_buffers(c), reset, c->stream);
     c->iin = 1 - c->iin;  // GPU.swapMortonAndIndexBuffers after the partition
     c->lookback_clear = c->groups_clear = true;
     return check_launch(c, "prepare");
 }
+
+int enqueue_prepare(gbh_ctx* c) { return enqueue_prepare_with(c, false); }
 
 int enqueue_sort(gbh_ctx* c) {
     if (!c->lookback_clear) {
@@ -187,13 +188,14 @@ static bool stage_idle(const gbh_ctx* c, int stage) {
     return k_stages[stage] == enqueue_merge && c->params_host.merging_collision_or_neither != GBH_MODE_MERGE;
 }
 
+// the step as one sequence: the reset runs inside the compaction's first kernel
 static int enqueue_step(gbh_ctx* c) {
-    for (int s = 0; s < GBH_NUM_STAGES; ++s) {
-        if (stage_idle(c, s)) continue;
-        int rc = k_stages[s](c);
-        if (rc) return rc;
+    int rc = enqueue_prepare_with(c, true);
+    for (int s = 0; s < GBH_NUM_STAGES && !rc; ++s) {
+        if (k_stages[s] == enqueue_reset || k_stages[s] == enqueue_prepare || stage_idle(c, s)) continue;
+        rc = k_stages[s](c);
     }
-    return GBH_OK;
+    return rc;
 }
 
 // FP64 positions (two, following the body buffers), leaf residuals and the
@@ -319,7 +321,7 @@ int gbh_create(gbh_ctx** out, uint32_t n, const float bounds[6], const gbh_units
     size_t o_tkids = A.add((size_t)ni * 8), o_tcnt = A.add((size_t)ni * 4), o_tready = A.add((size_t)ni * 4);
     size_t o_pint = A.add((size_t)ni * 4), o_pleaf = A.add((size_t)n * 4);
     size_t o_tdead = A.add((size_t)c->prep_tiles_cap * 4), o_taabb = A.add((size_t)c->prep_tiles_cap * 24);
-    size_t o_hist = A.add(SORT_PASSES * SORT_RADIX * 4), o_bbase = A.add(SORT_PASSES * SORT_RADIX * 4);
+    size_t o_hist = A.add(SORT_PASSES * SORT_RADIX * 4);
     c->lookback_bytes = (size_t)SORT_PASSES * c->sort_tiles_cap * SORT_RADIX * 4;
     size_t o_lb = A.add(c->lookback_bytes);
     e = cudaMalloc(&c->arena, A.total);
@@ -366,7 +368,6 @@ int gbh_create(gbh_ctx** out, uint32_t n, const float bounds[6], const gbh_units
     c->tile_dead = (uint32_t*)(base + o_tdead);
     c->tile_aabb = (float*)(base + o_taabb);
     c->hist = (uint32_t*)(base + o_hist);
-    c->bucket_base = (uint32_t*)(base + o_bbase);
     c->lookback = (uint32_t*)(base + o_lb);
 
     sort_setup(c->sort_items);

@@ -63,7 +63,6 @@ struct gbh_ctx {
     uint32_t* tile_dead = nullptr;
     float* tile_aabb = nullptr;
     uint32_t* hist = nullptr;
-    uint32_t* bucket_base = nullptr;
     uint32_t* lookback = nullptr;
     size_t lookback_bytes = 0;
 

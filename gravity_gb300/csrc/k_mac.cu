@@ -67,7 +67,6 @@ struct MacState {
     uint64_t* skeys[2] = {nullptr, nullptr};
     uint32_t* svals[2] = {nullptr, nullptr};
     uint32_t* shist = nullptr;
-    uint32_t* sbase = nullptr;
     uint32_t* slook = nullptr;
     DevState* sst = nullptr;
     uint32_t stiles = 0;
@@ -421,7 +420,7 @@ static int mac_ensure(gbh_ctx* c) {
 
 static void mac_free_pairs(MacState* m) {
     for (void* p : {(void*)m->feats, (void*)m->labels, (void*)m->pairs, (void*)m->skeys[0], (void*)m->skeys[1],
-                    (void*)m->svals[0], (void*)m->svals[1], (void*)m->shist, (void*)m->sbase, (void*)m->slook,
+                    (void*)m->svals[0], (void*)m->svals[1], (void*)m->shist, (void*)m->slook,
                     (void*)m->sst, (void*)m->feats_tmp, (void*)m->pairs_tmp})
         cudaFree(p);
     m->feats = m->feats_tmp = nullptr;
@@ -429,7 +428,7 @@ static void mac_free_pairs(MacState* m) {
     m->pairs = m->pairs_tmp = nullptr;
     m->skeys[0] = m->skeys[1] = nullptr;
     m->svals[0] = m->svals[1] = nullptr;
-    m->shist = m->sbase = m->slook = nullptr;
+    m->shist = m->slook = nullptr;
     m->sst = nullptr;
     m->cap = 0;
 }
@@ -451,7 +450,6 @@ static int mac_ensure_pairs(gbh_ctx* c, uint32_t cap) {
         MTRY(c, cudaMalloc(&m->svals[k], (size_t)cap * 4));
     }
     MTRY(c, cudaMalloc(&m->shist, SORT_PASSES * SORT_RADIX * 4));
-    MTRY(c, cudaMalloc(&m->sbase, SORT_PASSES * SORT_RADIX * 4));
     MTRY(c, cudaMalloc(&m->slook, (size_t)SORT_PASSES * tiles * SORT_RADIX * 4));
     MTRY(c, cudaMalloc(&m->sst, sizeof(DevState)));
     m->stiles = tiles;
@@ -483,7 +481,6 @@ static int mac_sort_pairs(gbh_ctx* c, uint32_t n) {
     sb.idx_out = m->svals[1];
     sb.st = m->sst;
     sb.hist = m->shist;
-    sb.bucket_base = m->sbase;
     sb.lookback = m->slook;
     sb.N = n;
     sb.sort_tiles_cap = m->stiles;

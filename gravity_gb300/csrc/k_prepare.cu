@@ -21,7 +21,7 @@
 #include "gbh_common.cuh"
 
 // ---------------------------------------------------------------------------
-__global__ void k_reset(StepBuffers b) {
+__device__ __forceinline__ void reset_step(const StepBuffers& b) {
     const gbh_step_params* p = b.params;
     DevState* st = b.st;
     for (uint32_t i = threadIdx.x; i < SORT_PASSES * SORT_RADIX; i += blockDim.x) b.hist[i] = 0;
@@ -60,6 +60,8 @@ __global__ void k_reset(StepBuffers b) {
     }
 }
 
+__global__ void k_reset(StepBuffers b) { reset_step(b); }
+
 void launch_reset(const StepBuffers& b, cudaStream_t s) { k_reset<<<1, 256, 0, s>>>(b); }
 
 // ---------------------------------------------------------------------------
@@ -74,7 +76,11 @@ __device__ __forceinline__ void warp_minmax(float v[6]) {
     }
 }
 
+// RESET: the step's reset too, by the first block (a whole step's reset and
+// compaction in one kernel; nothing below reads what the reset writes)
+template <bool RESET>
 __global__ __launch_bounds__(PREP_THREADS) void k_prep_count(StepBuffers b) {
+    if (RESET && blockIdx.x == 0) reset_step(b);
     const gbh_sim_values* sim = b.sim;
     const uint32_t n = sim->num_bodies;
     const uint32_t tile = blockIdx.x;
@@ -355,8 +361,11 @@ __global__ __launch_bounds__(PREP_THREADS) void k_prep_scatter(StepBuffers b) {
     }
 }
 
-void launch_prepare(const StepBuffers& b, cudaStream_t s) {
-    k_prep_count<<<b.prep_tiles_cap, PREP_THREADS, 0, s>>>(b);
+void launch_prepare(const StepBuffers& b, bool reset, cudaStream_t s) {
+    if (reset)
+        k_prep_count<true><<<b.prep_tiles_cap, PREP_THREADS, 0, s>>>(b);
+    else
+        k_prep_count<false><<<b.prep_tiles_cap, PREP_THREADS, 0, s>>>(b);
     k_prep_scan<<<1, 1024, 0, s>>>(b);
     k_prep_scatter<<<b.prep_tiles_cap, PREP_THREADS, 0, s>>>(b);
 }

@@ -7,7 +7,8 @@
 // keys yields the same permutation, so this is a onesweep sort (Adinets &
 // Merrill 2022): 8 passes of 8-bit digits, one kernel per pass.
 //   * The eight digit histograms are accumulated by the encode pass
-//     (k_prep_scatter) and scanned here once (k_sort_scan).
+//     (k_prep_scatter); every block scans its pass's histogram beside its own
+//     tile's digit counts, one kernel less than scanning them first.
 //   * Each pass kernel takes a tile ticket, ranks its keys per warp (digit
 //     peers from one ballot per digit bit, ranks reserved with shared-memory
 //     atomics in item order), publishes the tile's digit counts, resolves its global digit
@@ -24,32 +25,12 @@
 #define LB_WINDOW 4
 #endif
 
-__global__ void k_sort_scan(StepBuffers b) {
-    // one block per pass: exclusive scan of the 256 digit counts
-    const uint32_t p = blockIdx.x;
-    const uint32_t d = threadIdx.x;
-    const uint32_t v = b.hist[p * SORT_RADIX + d];
-    __shared__ uint32_t s_w[SORT_RADIX / 32];
-    const uint32_t lane = lane_id(), w = d >> 5;
-    uint32_t x = v;
-#pragma unroll
-    for (int o = 1; o < 32; o <<= 1) {
-        uint32_t y = __shfl_up_sync(0xffffffffu, x, o);
-        if (lane >= (uint32_t)o) x += y;
-    }
-    if (lane == 31) s_w[w] = x;
-    __syncthreads();
-    uint32_t off = 0;
-    for (uint32_t i = 0; i < w; ++i) off += s_w[i];
-    b.bucket_base[p * SORT_RADIX + d] = off + x - v;
-}
-
 template <int ITEMS>
 struct SortSmem {
     uint32_t warp_hist[SORT_THREADS / 32][SORT_RADIX + 1];  // +1: sentinel bucket of out-of-range items
     uint32_t block_excl[SORT_RADIX + 1];
     uint32_t delta[SORT_RADIX];
-    uint32_t warp_tot[SORT_THREADS / 32];
+    uint2 warp_tot[SORT_THREADS / 32];
     uint32_t tile;
     unsigned long long keys[SORT_THREADS * ITEMS];
     uint32_t vals[SORT_THREADS * ITEMS];
@@ -155,18 +136,30 @@ __global__ __launch_bounds__(SORT_THREADS, SortBlocks<ITEMS>::value) void k_sort
     } else {
         *my = LB_FLAG_AGG | total;
     }
-    // block exclusive scan of totals over digits -> block_excl
+    // block exclusive scans over the digits: of the tile's totals (block_excl)
+    // and of the pass's histogram (where each digit begins in the output)
+    const uint32_t digit_count = b.hist[pass * SORT_RADIX + d];
+    uint32_t bucket_base;
     {
-        uint32_t x = total;
+        uint32_t x = total, y = digit_count;
 #pragma unroll
         for (int o = 1; o < 32; o <<= 1) {
-            uint32_t y = __shfl_up_sync(0xffffffffu, x, o);
-            if (lane >= (uint32_t)o) x += y;
+            const uint32_t px = __shfl_up_sync(0xffffffffu, x, o), py = __shfl_up_sync(0xffffffffu, y, o);
+            if (lane >= (uint32_t)o) {
+                x += px;
+                y += py;
+            }
         }
-        if (lane == 31) S.warp_tot[w] = x;
+        if (lane == 31) S.warp_tot[w] = make_uint2(x, y);
         __syncthreads();
         uint32_t off = 0;
-        for (uint32_t i = 0; i < w; ++i) off += S.warp_tot[i];
+        bucket_base = 0;
+        for (uint32_t i = 0; i < w; ++i) {
+            const uint2 t = S.warp_tot[i];
+            off += t.x;
+            bucket_base += t.y;
+        }
+        bucket_base += y - digit_count;
         S.block_excl[d] = off + x - total;
         if (d == 0) S.block_excl[SORT_RADIX] = 0;
     }
@@ -227,7 +220,7 @@ __global__ __launch_bounds__(SORT_THREADS, SortBlocks<ITEMS>::value) void k_sort
         }
         *my = LB_FLAG_INC | (prefix + total);
     }
-    S.delta[d] = b.bucket_base[pass * SORT_RADIX + d] + prefix - S.block_excl[d];
+    S.delta[d] = bucket_base + prefix - S.block_excl[d];
     __syncthreads();
     const uint32_t valid = min((uint32_t)TILE, n - base);
     bool bad = false;
@@ -320,7 +313,6 @@ static void launch_passes(const StepBuffers& b, cudaStream_t s) {
 }
 
 void launch_sort(const StepBuffers& b, cudaStream_t s) {
-    k_sort_scan<<<SORT_PASSES, SORT_RADIX, 0, s>>>(b);
     if (b.sort_items == 4)
         launch_passes<4>(b, s);
     else if (b.sort_items == 8)

@@ -39,7 +39,6 @@ struct NoAllocScratch {
     unsigned long long keys_tmp[NOALLOC_MAX_PAIRS];
     uint32_t vals_tmp[NOALLOC_MAX_PAIRS];
     uint32_t hist[SORT_PASSES * SORT_RADIX];
-    uint32_t bucket_base[SORT_PASSES * SORT_RADIX];
     uint32_t lookback[SORT_PASSES * NOALLOC_TILES * SORT_RADIX];
     DevState st;
 };
@@ -122,7 +121,6 @@ extern "C" int gbh_sort_pairs_noalloc(const uint64_t* keys_in, const uint32_t* v
     b.idx_out = s->vals_tmp;
     b.st = &s->st;
     b.hist = s->hist;
-    b.bucket_base = s->bucket_base;
     b.lookback = s->lookback;
     b.N = n;
     b.sort_tiles_cap = NOALLOC_TILES;
