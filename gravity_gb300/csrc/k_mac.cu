@@ -21,9 +21,9 @@
 // Training (gbh_mac_train): minibatches drawn with a counter-based hash; the
 // forward pass is the inference code (BF16 mma.sync, FP32 accumulation), the
 // backward pass runs in FP32 on the CUDA cores (straight-through for the BF16
-// rounding), each warp writes its gradient sums, one kernel adds them in warp
-// order (no float atomics: training is bit-reproducible), then Adam updates
-// the FP32 master weights and rebuilds the BF16 fragment table.
+// rounding), each block writes its gradient sums, one kernel adds them in block
+// order (no float atomics: training is bit-reproducible) and updates the FP32
+// master weights (Adam); the BF16 fragment table follows from them.
 #include <cmath>
 #include <cstring>
 #include <string>
@@ -72,47 +72,44 @@ struct MacState {
     uint32_t stiles = 0;
     float* feats_tmp = nullptr;
     uint2* pairs_tmp = nullptr;
-    // per-warp gradient sums of one training step [warps][MAC_NPARAMS + 1]
+    // gradient sums of one training step's blocks [blocks][MAC_NPARAMS + 1]
     float* part = nullptr;
-    uint32_t part_warps = 0;
+    uint32_t part_blocks = 0;
 };
 
 #define MAC_PART_STRIDE (MAC_NPARAMS + 1)  // the parameters' gradients, then the loss
 
 // ---------------------------------------------------------------------------
-// fragment table from the FP32 parameters (layout in mac_mlp.cuh)
-__global__ void k_mac_build_frag(const float* __restrict__ p, uint32_t* __restrict__ frag) {
-    const uint32_t lane = threadIdx.x;
+// Word `word` of lane `lane` of the fragment table (layout in mac_mlp.cuh) from
+// the FP32 parameters.
+__device__ __forceinline__ uint32_t mac_frag_word(const float* p, uint32_t word, uint32_t lane) {
     const uint32_t gid = lane >> 2, tig = lane & 3;
-    const float* W1 = p + MAC_OFF_W1;
-    const float* W2 = p + MAC_OFF_W2;
-    const float* w3 = p + MAC_OFF_W3;
-    auto w1 = [&](uint32_t o, uint32_t k) { return k < MAC_FEATURES ? W1[o * MAC_FEATURES + k] : 0.0f; };
-    for (int nt = 0; nt < 4; ++nt) {
-        const uint32_t o = 8 * nt + gid;
-        frag[(2 * nt) * 32 + lane] = pack_bf16x2(w1(o, 2 * tig), w1(o, 2 * tig + 1));
-        frag[(2 * nt + 1) * 32 + lane] = pack_bf16x2(w1(o, 2 * tig + 8), w1(o, 2 * tig + 9));
-        for (int ks = 0; ks < 2; ++ks) {
-            const uint32_t k = 16 * ks + 2 * tig;
-            frag[(MAC_FRAG_W1 + (nt * 2 + ks) * 2) * 32 + lane] = pack_bf16x2(W2[o * 32 + k], W2[o * 32 + k + 1]);
-            frag[(MAC_FRAG_W1 + (nt * 2 + ks) * 2 + 1) * 32 + lane] =
-                pack_bf16x2(W2[o * 32 + k + 8], W2[o * 32 + k + 9]);
-        }
+    if (word < MAC_FRAG_W1) {  // 4 n-tiles x 2 registers
+        const float* row = p + MAC_OFF_W1 + (8 * (word >> 1) + gid) * MAC_FEATURES;
+        const uint32_t k = 2 * tig + 8 * (word & 1u);
+        return pack_bf16x2(k < MAC_FEATURES ? row[k] : 0.0f, k + 1 < MAC_FEATURES ? row[k + 1] : 0.0f);
     }
-    for (int ks = 0; ks < 2; ++ks) {
-        const uint32_t k = 16 * ks + 2 * tig;
-        const bool col0 = gid == 0;
-        frag[(MAC_FRAG_W1 + MAC_FRAG_W2 + 2 * ks) * 32 + lane] = col0 ? pack_bf16x2(w3[k], w3[k + 1]) : 0u;
-        frag[(MAC_FRAG_W1 + MAC_FRAG_W2 + 2 * ks + 1) * 32 + lane] = col0 ? pack_bf16x2(w3[k + 8], w3[k + 9]) : 0u;
+    word -= MAC_FRAG_W1;
+    if (word < MAC_FRAG_W2) {  // 4 n-tiles x 2 k-steps x 2 registers
+        const float* at = p + MAC_OFF_W2 + (8 * (word >> 2) + gid) * 32 + 16 * ((word >> 1) & 1u) + 2 * tig + 8 * (word & 1u);
+        return pack_bf16x2(at[0], at[1]);
     }
-    const int b1o = MAC_FRAG_W1 + MAC_FRAG_W2 + MAC_FRAG_W3;
-    const int b2o = b1o + MAC_FRAG_B1;
-    for (int nt = 0; nt < 4; ++nt)
-        for (int c = 0; c < 2; ++c) {
-            frag[(b1o + 2 * nt + c) * 32 + lane] = __float_as_uint(p[MAC_OFF_B1 + 8 * nt + 2 * tig + c]);
-            frag[(b2o + 2 * nt + c) * 32 + lane] = __float_as_uint(p[MAC_OFF_B2 + 8 * nt + 2 * tig + c]);
-        }
-    frag[(MAC_FRAG_WORDS - 1) * 32 + lane] = __float_as_uint(p[MAC_OFF_B3]);
+    word -= MAC_FRAG_W2;
+    if (word < MAC_FRAG_W3) {  // 2 k-steps x 2 registers, column 0 only
+        const float* at = p + MAC_OFF_W3 + 16 * (word >> 1) + 2 * tig + 8 * (word & 1u);
+        return gid == 0 ? pack_bf16x2(at[0], at[1]) : 0u;
+    }
+    word -= MAC_FRAG_W3;
+    if (word < MAC_FRAG_B1 + MAC_FRAG_B2) {  // 4 n-tiles x 2 columns of each bias
+        const float* bias = p + (word < MAC_FRAG_B1 ? MAC_OFF_B1 : MAC_OFF_B2);
+        const uint32_t t = word % MAC_FRAG_B1;
+        return __float_as_uint(bias[8 * (t >> 1) + 2 * tig + (t & 1u)]);
+    }
+    return __float_as_uint(p[MAC_OFF_B3]);
+}
+
+__global__ void k_mac_build_frag(const float* __restrict__ p, uint32_t* __restrict__ frag) {
+    for (uint32_t word = 0; word < MAC_FRAG_WORDS; ++word) frag[word * 32 + threadIdx.x] = mac_frag_word(p, word, threadIdx.x);
 }
 
 // ---------------------------------------------------------------------------
@@ -250,139 +247,207 @@ __global__ void k_mac_gather_pairs(const uint32_t* __restrict__ rows, uint32_t n
 }
 
 // ---------------------------------------------------------------------------
-// training: forward (tensor cores) + backward (FP32) of 32 samples per warp
+// training: forward (tensor cores) + backward (FP32), 32 samples per block
 struct TrainSmem {
     alignas(16) uint32_t frag[MAC_SMEM_FRAG_WORDS];
-    __nv_bfloat16 x[MAC_TRAIN_WARPS * 32 * 16];
-    float h1[MAC_TRAIN_WARPS][32][33];
-    float h2[MAC_TRAIN_WARPS][32][33];
-    float dz2[MAC_TRAIN_WARPS][32][33];
-    float dz1[MAC_TRAIN_WARPS][32][33];
-    float dy[MAC_TRAIN_WARPS][32];
+    alignas(16) float params[(MAC_NPARAMS + 3) / 4 * 4];
+    alignas(16) float h1[32][36];  // rows of four 16-byte words for each warp's outputs
+    alignas(16) float xf[32][16];  // features after the BF16 rounding, feature 3 w + c at 4 w + c
+    __nv_bfloat16 x[32 * 16];
+    float h2[32][33];
+    float dz2[32][33];
+    float dz1[32][33];
+    float dy[32];
 };
 
 __device__ __forceinline__ uint32_t sample_index(uint32_t seed, uint32_t step, uint32_t i, uint32_t n) {
     return hash32(hash32(seed * 0x9E3779B9u + step) ^ (i * 0x85EBCA6Bu)) % n;
 }
 
-// random = 1: sample indices with the hash; 0: rows [0, total) in order
-__global__ __launch_bounds__(MAC_TRAIN_WARPS * 32) void k_mac_train_step(
-    const float* __restrict__ feats, const float* __restrict__ labels, uint32_t n_pairs, uint32_t total,
-    int random, uint32_t seed, uint32_t step, MacDeviceWeights mw, const float* __restrict__ params,
-    float* __restrict__ part) {
+// One training step's gradient sums, one block per 32 samples (random = 1:
+// sample indices with the hash; 0: rows [0, total) in order).  Every sum runs
+// over the samples in order, whatever the block's shape.
+//
+// What bounds it: latency, a batch of 8,192 samples being 256 such chains.  A
+// warp per 32 samples in blocks of four used 64 SMs, and walked the whole
+// backward pass, about 5,000 instructions with W2 from global memory, alone.
+// Here four warps share the samples: the first runs the network, then each
+// takes 8 of the 32 hidden gradients and 11 of the 44 weight columns.  The
+// fragment table comes from the parameters in the same kernel, so a step is two
+// launches (with k_mac_update) instead of four.
+// One epoch over 524,288 pairs, batches of 8,192: 2.46 -> 1.28 ms.
+__global__ __launch_bounds__(128) void k_mac_train_step(
+    const float* __restrict__ feats, const float* __restrict__ labels, uint32_t n_pairs, uint32_t total, int random,
+    uint32_t seed, uint32_t step, const float* __restrict__ params, float* __restrict__ part) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
     TrainSmem& S = *reinterpret_cast<TrainSmem*>(smem_raw);
-    mac_load_frag(mw, S.frag, S.x);
     const uint32_t lane = lane_id(), w = threadIdx.x >> 5;
-    const uint32_t i = (blockIdx.x * MAC_TRAIN_WARPS + w) * 32 + lane;
+    const uint32_t i = blockIdx.x * 32 + lane;
     const bool valid = i < total;
     const uint32_t row = valid ? (random ? sample_index(seed, step, i, n_pairs) : i) : 0u;
     float f[MAC_FEATURES];
+    float y = 0.0f;
+    if (w == 0) {
 #pragma unroll
-    for (int k = 0; k < MAC_FEATURES; ++k) f[k] = valid ? feats[(size_t)row * MAC_FEATURES + k] : 0.0f;
-    const float y = valid ? labels[row] : 0.0f;
-    mac_stage_features(mw, w, lane, f);
-    MacActs acts;
-    const float pred = mac_forward_warp<true>(mw, w, lane, &acts);
-    // loss: mean squared error over `total` samples
-    const float e = pred - y;
-    float l = valid ? e * e : 0.0f;
-    const float d = valid ? 2.0f * e / (float)total : 0.0f;
-    // activations to shared memory, [sample][unit]
-    const uint32_t gid = lane >> 2, tig = lane & 3;
-#pragma unroll
-    for (int mt = 0; mt < 2; ++mt)
-#pragma unroll
-        for (int nt = 0; nt < 4; ++nt)
-#pragma unroll
-            for (int r = 0; r < 4; ++r) {
-                const uint32_t rr = 16 * mt + gid + 8 * (r >> 1), cc = 8 * nt + 2 * tig + (r & 1);
-                S.h1[w][rr][cc] = acts.h1[mt][nt][r];
-                S.h2[w][rr][cc] = acts.h2[mt][nt][r];
-            }
-    S.dy[w][lane] = d;
-    __syncwarp();
-    // lane = sample: dz2 = d * w3 * relu'(z2); dz1 = (dz2 . W2) * relu'(z1)
-    const float* W2 = params + MAC_OFF_W2;
-    const float* w3 = params + MAC_OFF_W3;
-    float dz2[32];
-#pragma unroll
-    for (int o = 0; o < 32; ++o) {
-        dz2[o] = S.h2[w][lane][o] > 0.0f ? d * w3[o] : 0.0f;
-        S.dz2[w][lane][o] = dz2[o];
+        for (int k = 0; k < MAC_FEATURES; ++k) f[k] = valid ? feats[(size_t)row * MAC_FEATURES + k] : 0.0f;
+        y = valid ? labels[row] : 0.0f;
     }
-    for (int k = 0; k < 32; ++k) {
-        float acc = 0.0f;
-#pragma unroll
-        for (int o = 0; o < 32; ++o) acc = fmaf(dz2[o], W2[o * 32 + k], acc);
-        S.dz1[w][lane][k] = S.h1[w][lane][k] > 0.0f ? acc : 0.0f;
+    for (uint32_t k = threadIdx.x; k < MAC_NPARAMS; k += 128) S.params[k] = params[k];
+    __syncthreads();
+    for (uint32_t k = threadIdx.x; k < MAC_FRAG_WORDS * 32; k += 128) {
+        const uint32_t word = k >> 5, l = k & 31;
+        S.frag[((word >> 2) * 32 + l) * 4 + (word & 3)] = mac_frag_word(S.params, word, l);
     }
-    __syncwarp();
-    // lane = output unit: weight gradients summed over the warp's samples
+    __syncthreads();
+    MacDeviceWeights mw;
+    mw.smem_frag = S.frag;
+    mw.smem_x = S.x;
+    mw.x_rows = 32;
+    float loss = 0.0f;
+    if (w == 0) {
+        mac_stage_features(mw, 0, lane, f);
+#pragma unroll
+        for (int k = 0; k < MAC_FEATURES; ++k) S.xf[lane][k / 3 * 4 + k % 3] = __bfloat162float(__float2bfloat16_rn(f[k]));
+        MacActs acts;
+        const float pred = mac_forward_warp<true>(mw, 0, lane, &acts);
+        // loss: mean squared error over `total` samples
+        const float e = pred - y;
+        loss = valid ? e * e : 0.0f;
+        S.dy[lane] = valid ? 2.0f * e / (float)total : 0.0f;
+        // activations to shared memory, [sample][unit]
+        const uint32_t gid = lane >> 2, tig = lane & 3;
+#pragma unroll
+        for (int mt = 0; mt < 2; ++mt)
+#pragma unroll
+            for (int nt = 0; nt < 4; ++nt)
+#pragma unroll
+                for (int r = 0; r < 4; ++r) {
+                    const uint32_t rr = 16 * mt + gid + 8 * (r >> 1), cc = 8 * nt + 2 * tig + (r & 1);
+                    S.h1[rr][cc] = acts.h1[mt][nt][r];
+                    S.h2[rr][cc] = acts.h2[mt][nt][r];
+                }
+    }
+    __syncthreads();
+    // lane = sample: dz2 = dy * w3 * relu'(z2) (in every warp), and this
+    // warp's units of dz1 = (dz2 . W2) * relu'(z1)
+    const float* W2 = S.params + MAC_OFF_W2;
+    const float* w3 = S.params + MAC_OFF_W3;
+    {
+        const float dy = S.dy[lane];
+        float acc[8];
+#pragma unroll
+        for (int k = 0; k < 8; ++k) acc[k] = 0.0f;
+#pragma unroll 8
+        for (int o = 0; o < 32; ++o) {
+            const float dz2 = S.h2[lane][o] > 0.0f ? dy * w3[o] : 0.0f;
+            if (w == 0) S.dz2[lane][o] = dz2;
+            const float4 a = *reinterpret_cast<const float4*>(W2 + o * 32 + 8 * w);
+            const float4 c = *reinterpret_cast<const float4*>(W2 + o * 32 + 8 * w + 4);
+            acc[0] = fmaf(dz2, a.x, acc[0]);
+            acc[1] = fmaf(dz2, a.y, acc[1]);
+            acc[2] = fmaf(dz2, a.z, acc[2]);
+            acc[3] = fmaf(dz2, a.w, acc[3]);
+            acc[4] = fmaf(dz2, c.x, acc[4]);
+            acc[5] = fmaf(dz2, c.y, acc[5]);
+            acc[6] = fmaf(dz2, c.z, acc[6]);
+            acc[7] = fmaf(dz2, c.w, acc[7]);
+        }
+#pragma unroll
+        for (int k = 0; k < 8; ++k) S.dz1[lane][8 * w + k] = S.h1[lane][8 * w + k] > 0.0f ? acc[k] : 0.0f;
+    }
+    __syncthreads();
+    // lane = output unit: weight gradients summed over the samples, this
+    // warp's columns: 8 of W2, 3 of W1; the vectors by one warp each
     const uint32_t o = lane;
-    float g_w3 = 0.f, g_b2 = 0.f, g_b1 = 0.f, g_b3 = 0.f;
-    float g_w2[32], g_w1[MAC_FEATURES];
+    float g_w2[8], g_w1[3], g_vec = 0.0f, g_b3 = 0.0f;
 #pragma unroll
-    for (int k = 0; k < 32; ++k) g_w2[k] = 0.f;
+    for (int k = 0; k < 8; ++k) g_w2[k] = 0.0f;
 #pragma unroll
-    for (int k = 0; k < MAC_FEATURES; ++k) g_w1[k] = 0.f;
-    const __nv_bfloat16* X = S.x + (size_t)w * 32 * 16;
+    for (int k = 0; k < 3; ++k) g_w1[k] = 0.0f;
+#pragma unroll 4
     for (int s = 0; s < 32; ++s) {
-        const float ds = S.dy[w][s];
-        g_w3 = fmaf(ds, S.h2[w][s][o], g_w3);
-        g_b3 += ds;
-        const float z2 = S.dz2[w][s][o];
-        g_b2 += z2;
-#pragma unroll
-        for (int k = 0; k < 32; ++k) g_w2[k] = fmaf(z2, S.h1[w][s][k], g_w2[k]);
-        const float z1 = S.dz1[w][s][o];
-        g_b1 += z1;
-#pragma unroll
-        for (int k = 0; k < MAC_FEATURES; ++k) g_w1[k] = fmaf(z1, __bfloat162float(X[s * 16 + k]), g_w1[k]);
+        const float z2 = S.dz2[s][o], z1 = S.dz1[s][o];
+        const float4 a = *reinterpret_cast<const float4*>(&S.h1[s][8 * w]);
+        const float4 c = *reinterpret_cast<const float4*>(&S.h1[s][8 * w + 4]);
+        const float4 x = *reinterpret_cast<const float4*>(&S.xf[s][4 * w]);
+        g_w2[0] = fmaf(z2, a.x, g_w2[0]);
+        g_w2[1] = fmaf(z2, a.y, g_w2[1]);
+        g_w2[2] = fmaf(z2, a.z, g_w2[2]);
+        g_w2[3] = fmaf(z2, a.w, g_w2[3]);
+        g_w2[4] = fmaf(z2, c.x, g_w2[4]);
+        g_w2[5] = fmaf(z2, c.y, g_w2[5]);
+        g_w2[6] = fmaf(z2, c.z, g_w2[6]);
+        g_w2[7] = fmaf(z2, c.w, g_w2[7]);
+        g_w1[0] = fmaf(z1, x.x, g_w1[0]);
+        g_w1[1] = fmaf(z1, x.y, g_w1[1]);
+        g_w1[2] = fmaf(z1, x.z, g_w1[2]);
+        if (w == 0) {
+            g_b3 += S.dy[s];
+        } else if (w == 1) {
+            g_vec = fmaf(S.dy[s], S.h2[s][o], g_vec);
+        } else {
+            g_vec += w == 2 ? z2 : z1;
+        }
     }
-    // this warp's sums: every parameter once (lane o: the weights of unit o)
-    float* gp = part + (size_t)(blockIdx.x * MAC_TRAIN_WARPS + w) * MAC_PART_STRIDE;
+    // every parameter once (lane o: the weights of unit o)
+    float* gp = part + (size_t)blockIdx.x * MAC_PART_STRIDE;
 #pragma unroll
-    for (int k = 0; k < MAC_FEATURES; ++k) gp[MAC_OFF_W1 + o * MAC_FEATURES + k] = g_w1[k];
-    gp[MAC_OFF_B1 + o] = g_b1;
+    for (int k = 0; k < 3; ++k) gp[MAC_OFF_W1 + o * MAC_FEATURES + 3 * w + k] = g_w1[k];
 #pragma unroll
-    for (int k = 0; k < 32; ++k) gp[MAC_OFF_W2 + o * 32 + k] = g_w2[k];
-    gp[MAC_OFF_B2 + o] = g_b2;
-    gp[MAC_OFF_W3 + o] = g_w3;
+    for (int k = 0; k < 8; ++k) gp[MAC_OFF_W2 + o * 32 + 8 * w + k] = g_w2[k];
+    if (w == 1) gp[MAC_OFF_W3 + o] = g_vec;
+    if (w == 2) gp[MAC_OFF_B2 + o] = g_vec;
+    if (w == 3) gp[MAC_OFF_B1 + o] = g_vec;
+    if (w == 0) {
 #pragma unroll
-    for (int s = 16; s > 0; s >>= 1) l += __shfl_xor_sync(0xffffffffu, l, s);
-    if (lane == 0) {
-        gp[MAC_OFF_B3] = g_b3;
-        gp[MAC_NPARAMS] = l;
+        for (int k = 16; k > 0; k >>= 1) loss += __shfl_xor_sync(0xffffffffu, loss, k);
+        if (lane == 0) {
+            gp[MAC_OFF_B3] = g_b3;
+            gp[MAC_NPARAMS] = loss;
+        }
     }
 }
 
-// The gradient of one step: the warps' sums added in warp order (the same
-// bits in every run); the loss slot adds into the epoch's running loss.
-__global__ void k_mac_reduce(const float* __restrict__ part, uint32_t warps, float* __restrict__ grad,
-                             float* __restrict__ loss) {
-    const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i > MAC_NPARAMS) return;
+// The gradient of one step: the blocks' sums added in block order (the same
+// bits in every run); the loss slot adds into the epoch's running loss.  ADAM:
+// then the update of the parameters, in the same kernel; otherwise the gradient
+// is stored.  A block takes 32 parameters: its 256 threads bring the sums of up
+// to 256 blocks into shared memory at once, one warp adds them.
+template <bool ADAM>
+__global__ __launch_bounds__(256) void k_mac_update(const float* __restrict__ part, uint32_t blocks,
+                                                    float* __restrict__ loss, float* __restrict__ grad,
+                                                    float* __restrict__ p, float* __restrict__ m, float* __restrict__ v,
+                                                    float lr, float bc1, float bc2) {
+    __shared__ float s_part[256][32];
+    const uint32_t lane = lane_id(), w = threadIdx.x >> 5;
+    const uint32_t i = blockIdx.x * 32 + lane;
     float sum = 0.0f;
-    for (uint32_t w = 0; w < warps; ++w) sum += part[(size_t)w * MAC_PART_STRIDE + i];
-    if (i < MAC_NPARAMS)
-        grad[i] = sum;
-    else
+    for (uint32_t b0 = 0; b0 < blocks; b0 += 256) {
+        const uint32_t cnt = min(256u, blocks - b0);
+        if (b0) __syncthreads();
+#pragma unroll 8
+        for (uint32_t k = w; k < cnt; k += 8)
+            s_part[k][lane] = i <= MAC_NPARAMS ? part[(size_t)(b0 + k) * MAC_PART_STRIDE + i] : 0.0f;
+        __syncthreads();
+        if (w == 0) {
+#pragma unroll 16
+            for (uint32_t k = 0; k < cnt; ++k) sum += s_part[k][lane];
+        }
+    }
+    if (w != 0 || i > MAC_NPARAMS) return;
+    if (i == MAC_NPARAMS) {
         loss[0] += sum;
+    } else if (ADAM) {
+        const float mi = 0.9f * m[i] + 0.1f * sum;
+        const float vi = 0.999f * v[i] + 0.001f * sum * sum;
+        m[i] = mi;
+        v[i] = vi;
+        p[i] -= lr * (mi / bc1) / (sqrtf(vi / bc2) + 1e-8f);
+    } else {
+        grad[i] = sum;
+    }
 }
-
-__global__ void k_mac_adam(float* __restrict__ p, float* __restrict__ g, float* __restrict__ m, float* __restrict__ v,
-                           float lr, float bc1, float bc2) {
-    const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= MAC_NPARAMS) return;
-    const float gi = g[i];
-    const float mi = 0.9f * m[i] + 0.1f * gi;
-    const float vi = 0.999f * v[i] + 0.001f * gi * gi;
-    m[i] = mi;
-    v[i] = vi;
-    p[i] -= lr * (mi / bc1) / (sqrtf(vi / bc2) + 1e-8f);
-    g[i] = 0.0f;
-}
+#define MAC_UPDATE_BLOCKS ((MAC_NPARAMS + 32) / 32)
 
 // ---------------------------------------------------------------------------
 // host
@@ -797,30 +862,29 @@ int gbh_mac_train(gbh_ctx* c, uint32_t epochs, uint32_t batch, float lr, uint64_
         m->adam_t = 0;
     }
     MTRY(c, cudaFuncSetAttribute(k_mac_train_step, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)train_smem()));
-    const uint32_t rows = MAC_TRAIN_WARPS * 32;
     const uint32_t steps = (m->num_pairs + batch - 1) / batch;
-    const uint32_t tblocks = (batch + rows - 1) / rows, warps = tblocks * MAC_TRAIN_WARPS;
-    if (m->part_warps < warps) {
+    const uint32_t tblocks = (batch + 31) / 32;
+    if (m->part_blocks < tblocks) {
         cudaFree(m->part);
         m->part = nullptr;
-        m->part_warps = 0;
-        MTRY(c, cudaMalloc(&m->part, (size_t)warps * MAC_PART_STRIDE * 4));
-        m->part_warps = warps;
+        m->part_blocks = 0;
+        MTRY(c, cudaMalloc(&m->part, (size_t)tblocks * MAC_PART_STRIDE * 4));
+        m->part_blocks = tblocks;
     }
     for (uint32_t ep = 0; ep < epochs; ++ep) {
         MTRY(c, cudaMemsetAsync(m->loss, 0, 16, c->stream));
         for (uint32_t s = 0; s < steps; ++s) {
             const uint32_t st = ep * steps + s;
-            k_mac_train_step<<<tblocks, rows, train_smem(), c->stream>>>(
-                m->feats, m->labels, m->num_pairs, batch, 1, (uint32_t)seed, st, mac_weights(c), m->params, m->part);
-            k_mac_reduce<<<(MAC_PART_STRIDE + 255) / 256, 256, 0, c->stream>>>(m->part, warps, m->grad, m->loss);
+            k_mac_train_step<<<tblocks, 128, train_smem(), c->stream>>>(m->feats, m->labels, m->num_pairs, batch, 1,
+                                                                        (uint32_t)seed, st, m->params, m->part);
             ++m->adam_t;
             const float bc1 = 1.0f - std::pow(0.9f, (float)m->adam_t);
             const float bc2 = 1.0f - std::pow(0.999f, (float)m->adam_t);
-            k_mac_adam<<<(MAC_NPARAMS + 255) / 256, 256, 0, c->stream>>>(m->params, m->grad, m->adam_m, m->adam_v, lr,
-                                                                        bc1, bc2);
-            k_mac_build_frag<<<1, 32, 0, c->stream>>>(m->params, m->frag);
+            k_mac_update<true><<<MAC_UPDATE_BLOCKS, 256, 0, c->stream>>>(m->part, tblocks, m->loss, nullptr, m->params,
+                                                                         m->adam_m, m->adam_v, lr, bc1, bc2);
         }
+        // the walk's fragment table of the parameters as they are now
+        k_mac_build_frag<<<1, 32, 0, c->stream>>>(m->params, m->frag);
         MTRY(c, cudaGetLastError());
         if (losses) {
             float l = 0.0f;
@@ -840,11 +904,10 @@ int gbh_mac_loss_grad(gbh_ctx* c, const float* features, const float* labels, ui
     MTRY(c, cudaSetDevice(c->device));
     MacState* m = c->mac;
     float *df = nullptr, *dl = nullptr, *dp = nullptr;
-    const uint32_t rows = MAC_TRAIN_WARPS * 32, tblocks = (count + rows - 1) / rows;
-    const uint32_t warps = tblocks * MAC_TRAIN_WARPS;
+    const uint32_t tblocks = (count + 31) / 32;
     MTRY(c, cudaMalloc(&df, (size_t)count * MAC_FEATURES * 4));
     MTRY(c, cudaMalloc(&dl, (size_t)count * 4));
-    MTRY(c, cudaMalloc(&dp, (size_t)warps * MAC_PART_STRIDE * 4));
+    MTRY(c, cudaMalloc(&dp, (size_t)tblocks * MAC_PART_STRIDE * 4));
     cudaError_t e = cudaMemcpyAsync(df, features, (size_t)count * MAC_FEATURES * 4, cudaMemcpyHostToDevice, c->stream);
     if (e == cudaSuccess) e = cudaMemcpyAsync(dl, labels, (size_t)count * 4, cudaMemcpyHostToDevice, c->stream);
     if (e == cudaSuccess) e = cudaMemsetAsync(m->grad, 0, MAC_NPARAMS * 4, c->stream);
@@ -852,9 +915,9 @@ int gbh_mac_loss_grad(gbh_ctx* c, const float* features, const float* labels, ui
     if (e == cudaSuccess)
         e = cudaFuncSetAttribute(k_mac_train_step, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)train_smem());
     if (e == cudaSuccess) {
-        k_mac_train_step<<<tblocks, rows, train_smem(), c->stream>>>(df, dl, count, count, 0, 0, 0, mac_weights(c),
-                                                                      m->params, dp);
-        k_mac_reduce<<<(MAC_PART_STRIDE + 255) / 256, 256, 0, c->stream>>>(dp, warps, m->grad, m->loss);
+        k_mac_train_step<<<tblocks, 128, train_smem(), c->stream>>>(df, dl, count, count, 0, 0, 0, m->params, dp);
+        k_mac_update<false><<<MAC_UPDATE_BLOCKS, 256, 0, c->stream>>>(dp, tblocks, m->loss, m->grad, nullptr, nullptr,
+                                                                      nullptr, 0.0f, 1.0f, 1.0f);
         e = cudaGetLastError();
     }
     if (e == cudaSuccess) e = cudaMemcpyAsync(grad, m->grad, MAC_NPARAMS * 4, cudaMemcpyDeviceToHost, c->stream);
