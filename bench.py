@@ -449,13 +449,14 @@ def train_out_of_sample(bh, args, local, held: list) -> dict:
             "weights_sha256": __import__("hashlib").sha256(w.tobytes()).hexdigest()[:16]}
 
 
-def kernels_per_step(mac_mode: int, merging: bool) -> int:
+def kernels_per_step(mac_mode: int, merging: bool, capacity: int) -> int:
     """Kernels of this library launched by one step (the CUDA graph's kernel
     nodes): prepare 3 (the first also resets), sort 8 passes, build 1 (it also lists the
     group walks' body groups; with the group and learned walks 2: then the
-    groups' start lists), fill 2, walk 1, merge resolution 4 (in steps that
-    merge), swap 0 (a pointer swap)."""
-    return 3 + 8 + (1 if mac_mode == abi.MAC_PLAIN else 2) + 2 + 1 + (4 if merging else 0)
+    groups' start lists), fill 2 (3 with a capacity of 4,097 to 131,072 bodies),
+    walk 1, merge resolution 4 (in steps that merge), swap 0 (a pointer swap)."""
+    fill = 3 if 4096 < capacity <= 131072 else 2
+    return 3 + 8 + (1 if mac_mode == abi.MAC_PLAIN else 2) + fill + 1 + (4 if merging else 0)
 
 
 def measure_e2e(bh, p_head, n, e2e_steps, local, dist=None) -> dict:
@@ -825,7 +826,7 @@ def run_ours(args):
             "l2": "inputs larger than L2 (bodies 537 MB, tree + sort buffers ~5 GB)",
             "parallelism": f"replicas x{world}",
         },
-        "gpu_launches": kernels_per_step(p_head.mac_mode, p_head.merging_collision_or_neither == abi.MODE_MERGE) * args.steps,
+        "gpu_launches": kernels_per_step(p_head.mac_mode, p_head.merging_collision_or_neither == abi.MODE_MERGE, n) * args.steps,
         "interactions_per_step": interactions,
         "interactions_per_s": interactions * value / world,
         "comparison": compare,
@@ -846,7 +847,7 @@ def run_ours(args):
             "mlp_tflops": mlp_flop / (walk_ms / 1000.0) / 1e12,
         },
         "roofline_sort": {
-            "kernel": "k_sort_pass x8 + k_sort_scan",
+            "kernel": "k_sort_pass x8",
             "bound": "hbm",
             "achieved": sort_gbs,
             "peak": hbm_peak,

@@ -65,6 +65,7 @@ struct DevState {
     uint32_t merge_tasks;
     uint32_t sort_tiles[SORT_PASSES];  // onesweep tile tickets
     uint32_t num_groups;               // body groups of the group walk
+    uint32_t num_subtrees[2];          // the fill's subtrees above the groups, and the nodes above those
     uint32_t group_next;               // the next group a warp of the group walk takes (ticket)
     uint32_t frontier_saturated;       // group walks that accepted instead of opening (full stack)
     uint32_t sorted_valid;             // sorted_pm holds the current positions in index order
@@ -114,7 +115,8 @@ struct StepBuffers {
     // writes whole 80-byte nodes (no partial-sector writes to the node arrays)
     uint2* topo_kids;      // (childA, childB) per internal node
     uint32_t* topo_cnt;    // bodiesContained per internal node
-    uint32_t* fill_ready;  // arrival counters of the fill's climb above the groups
+    uint32_t* fill_ready;  // of the nodes above the groups: the climb's arrival counters, or places in a list
+    uint32_t* fill_subtrees[2];  // internal nodes: the fill's subtrees, and the nodes above those
     uint32_t* parent_int;  // parentId per internal node
     uint32_t* parent_leaf; // parentId per leaf
     uint2* groups;        // (first slot, body count) of the group walk's body groups

@@ -79,6 +79,10 @@ StepBuffers ctx_buffers(const gbh_ctx* c) {
     b.topo_kids = c->topo_kids;
     b.topo_cnt = c->topo_cnt;
     b.fill_ready = c->fill_ready;
+    // the build's lists for the fill live in the sort's spare key buffer (free
+    // once the sorted keys are back in keys_in, until the next step's encode)
+    b.fill_subtrees[0] = reinterpret_cast<uint32_t*>(c->keys[1 - c->iin]);
+    b.fill_subtrees[1] = b.fill_subtrees[0] + c->N;
     b.parent_int = c->parent_int;
     b.parent_leaf = c->parent_leaf;
     b.groups = c->groups;
@@ -141,7 +145,7 @@ int enqueue_sort(gbh_ctx* c) {
 }
 
 int enqueue_build(gbh_ctx* c) {
-    if (!c->groups_clear) CUDA_TRY(c, cudaMemsetAsync(&c->st->num_groups, 0, 4, c->stream));
+    if (!c->groups_clear) CUDA_TRY(c, cudaMemsetAsync(&c->st->num_groups, 0, 12, c->stream));
     c->groups_clear = false;
     c->ticket_clear = true;
     launch_build(ctx_buffers(c), c->stream);

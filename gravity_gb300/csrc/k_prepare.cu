@@ -227,7 +227,7 @@ __global__ __launch_bounds__(1024) void k_prep_scan(StepBuffers b) {
         st->n_old = n;
         st->just_died = died;
         st->n_new = n - died;
-        st->num_groups = 0;  // the build counts them
+        st->num_groups = st->num_subtrees[0] = st->num_subtrees[1] = 0;  // the build counts these
         // decrementDeadBodies, bh_update.comp:29-34
         sim->num_bodies = n - died;
         sim->just_died = 0;

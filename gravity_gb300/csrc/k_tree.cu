@@ -8,11 +8,12 @@
 //   written in part.  The stage entry point gbh_stage_build also writes the
 //   reference's intermediate topology words into the nodes (k_build_nodes).
 // Fill: treeInitLeafNodesKernel (bh_tree.comp:140-175) + 64 launches of
-//   treePropagateNodesKernel (bh_tree.comp:183-259) become two kernels: one
-//   warp per body group (a subtree of at most 96 bodies) initialises its
-//   leaves and finishes its nodes, and one thread per group climbs above the
-//   groups, where an atomic on an arrival counter lets the second child finish
-//   a node (Karras 2012 / Apetrei 2014).  There is no pass limit, so trees taller
+//   treePropagateNodesKernel (bh_tree.comp:183-259) become two kernels or three:
+//   one warp per body group (a subtree of at most 96 bodies) initialises its
+//   leaves and finishes its nodes; above the groups small trees are finished by
+//   a block per subtree and one for the rest, larger ones by a thread per group
+//   that climbs, where an atomic on an arrival counter lets the second child
+//   finish a node (Karras 2012 / Apetrei 2014).  There is no pass limit, so trees taller
 //   than 64 levels are filled completely, and the queue-reset race of the
 //   reference (bh_tree.comp:188-193) does not exist.
 #include "gbh_common.cuh"
@@ -49,6 +50,11 @@ __device__ __forceinline__ void emit_groups(const StepBuffers& b, uint32_t k, co
     }
 }
 
+// bodies in a subtree that one block of k_fill_above fills above its groups;
+// the largest capacity filled that way
+#define FILL_SUBTREE 4096u
+#define FILL_ABOVE_MAX 131072u
+
 __global__ __launch_bounds__(256) void k_build(StepBuffers b) {
     const uint32_t n = b.st->n_new;
     const uint32_t N = b.N;
@@ -75,6 +81,7 @@ __global__ __launch_bounds__(256) void k_build(StepBuffers b) {
     uint2 mine[2];
     uint32_t mine_node[2] = {0u, 0u};
     uint32_t k = 0;
+    uint32_t bodies = 0, kid[2] = {0u, 0u}, kid_bodies[2] = {0u, 0u};
     if (gid < n - 1) {
     const int i = (int)gid, ni = (int)n;
     const uint64_t ki = keys[i];
@@ -124,6 +131,11 @@ __global__ __launch_bounds__(256) void k_build(StepBuffers b) {
     const uint32_t cnt = (uint32_t)(mx - mn + 1);
     if (cnt > GBH_GROUP_MAX) {
         const uint32_t cl = (uint32_t)(gamma - mn + 1), cr = (uint32_t)(mx - gamma);
+        bodies = cnt;
+        kid[0] = left - N;
+        kid[1] = right - N;
+        kid_bodies[0] = cl;
+        kid_bodies[1] = cr;
         if (cl <= GBH_GROUP_MAX) {
             mine_node[k] = left;
             mine[k++] = make_uint2((uint32_t)mn, cl);
@@ -138,6 +150,19 @@ __global__ __launch_bounds__(256) void k_build(StepBuffers b) {
     }
     }
     emit_groups(b, k, mine, mine_node);
+    // the subtrees whose nodes above the groups a block fills, and the nodes
+    // above the subtrees (k_fill_above): rare
+    if (N <= FILL_ABOVE_MAX) {
+        if (bodies > FILL_SUBTREE) {
+#pragma unroll
+            for (int q = 0; q < 2; ++q)
+                if (kid_bodies[q] > GBH_GROUP_MAX && kid_bodies[q] <= FILL_SUBTREE)
+                    b.fill_subtrees[0][atomicAdd(&b.st->num_subtrees[0], 1u)] = kid[q];
+            b.fill_subtrees[1][atomicAdd(&b.st->num_subtrees[1], 1u)] = gid;
+        } else if (gid == 0 && bodies > 0) {
+            b.fill_subtrees[0][atomicAdd(&b.st->num_subtrees[0], 1u)] = 0u;  // the whole tree
+        }
+    }
 }
 
 // The reference's Node topology words after buildBinaryRadixTree (childA/B,
@@ -263,6 +288,24 @@ __device__ __forceinline__ NodeVals load_node_cg(const gbh_node* nd) {
     const float2 c = __ldcg(reinterpret_cast<const float2*>(p + 2));  // aabb4, aabb5
     v.depth = __ldcg(reinterpret_cast<const uint32_t*>(p + 3));
     v.col = __ldcg(p + 4);
+    v.box[0] = a.x;
+    v.box[1] = a.y;
+    v.box[2] = a.z;
+    v.box[3] = a.w;
+    v.box[4] = c.x;
+    v.box[5] = c.y;
+    return v;
+}
+
+// the fields of a finished node
+__device__ __forceinline__ NodeVals load_node(const gbh_node* nd) {
+    NodeVals v;
+    const float4* p = reinterpret_cast<const float4*>(nd);
+    v.cm = p[0];
+    const float4 a = p[1];
+    const float2 c = *reinterpret_cast<const float2*>(p + 2);  // aabb4, aabb5
+    v.depth = *reinterpret_cast<const uint32_t*>(p + 3);
+    v.col = p[4];
     v.box[0] = a.x;
     v.box[1] = a.y;
     v.box[2] = a.z;
@@ -444,7 +487,8 @@ __device__ __forceinline__ NodeVals fill_vals(const FillSmem& S, uint32_t kid) {
 // plain divisions inlined.
 // Fill stage, ms, before (512-slot tiles, threads climbing from their leaves)
 // and after: 16,777,216-body mixture 1.99 -> 1.43; 8,388,608 bodies in clusters 1.12 -> 0.78; 4,194,301
-// bodies with the plain walk's records 0.63 -> 0.46; 65,536 bodies 0.094 -> 0.070.
+// bodies with the plain walk's records 0.63 -> 0.46; 65,536 bodies 0.094 -> 0.070 (0.059 with
+// k_fill_above).
 __global__ __launch_bounds__(FILL_THREADS, FILL_BLOCKS) void k_fill(StepBuffers b) {
     extern __shared__ __align__(16) unsigned char fill_smem[];
     const uint32_t lane = lane_id(), w = threadIdx.x >> 5;
@@ -677,8 +721,8 @@ __device__ void climb_global(const StepBuffers& b, uint32_t self, uint32_t self_
     }
 }
 
-// Fill of the nodes above the body groups: one thread per group climbs from
-// its subtree's root.
+// Fill of the nodes above the body groups, capacities above FILL_ABOVE_MAX: one
+// thread per group climbs from its subtree's root.
 __global__ __launch_bounds__(256) void k_fill_top(StepBuffers b) {
     const uint32_t groups = b.st->num_groups;
     const uint32_t N = b.N;
@@ -694,13 +738,211 @@ __global__ __launch_bounds__(256) void k_fill_top(StepBuffers b) {
     }
 }
 
+// An internal node above the groups, with what its finishing needs.
+struct AboveNode {
+    uint32_t id, first, bodies, parent, left, right;  // left, right: the children's bodies
+    uint2 kids;
+};
+
+__device__ __forceinline__ AboveNode above_node(const StepBuffers& b, uint32_t i) {
+    AboveNode a;
+    a.id = i;
+    a.kids = b.topo_kids[i];
+    a.first = b.node_lo[i];
+    a.bodies = b.topo_cnt[i];
+    a.parent = b.parent_int[i];
+    // the left child ends at the split, where its index lies too
+    a.left = (a.kids.x < b.N ? a.kids.x : a.kids.x - b.N) - a.first + 1;
+    a.right = a.bodies - a.left;
+    return a;
+}
+
+__device__ __forceinline__ NodeVals load_child(const StepBuffers& b, uint32_t id) {
+    return load_node(id < b.N ? &b.leaf[id] : &b.internal[id - b.N]);
+}
+
+__device__ __forceinline__ void store_above(const StepBuffers& b, const AboveNode& a, const NodeVals& out,
+                                            const NodeVals& L, const NodeVals& R) {
+    store_internal(b, a.id, out, L, R, a.kids.x, a.kids.y, a.left, a.right, a.bodies, a.parent);
+    if (a.parent == GBH_NONE) {
+        b.st->tree_height = out.depth;
+        *b.root_rec = make_rec(out, a.id + b.N, a.bodies, false);
+    }
+}
+
+// Rounds over a list of any length, values and flags in global memory: lists
+// longer than a block has threads (trees far from the usual shapes).  The
+// block's barriers order a node's words and flag before the rounds that read
+// them.
+__device__ void fill_long_list(const StepBuffers& b, const uint32_t* list, uint32_t m, uint32_t floor) {
+    volatile uint32_t* flags = b.fill_ready;  // the round that finished the node
+    for (uint32_t k = threadIdx.x; k < m; k += blockDim.x) flags[list[k]] = 0u;
+    __syncthreads();
+    for (uint32_t round = 1;; ++round) {
+        bool progress = false;
+        for (uint32_t k = threadIdx.x; k < m; k += blockDim.x) {
+            const uint32_t i = list[k];
+            if (flags[i]) continue;
+            const AboveNode a = above_node(b, i);
+            const uint32_t fa = a.left > floor ? flags[a.kids.x - b.N] : 0u, fb = a.right > floor ? flags[a.kids.y - b.N] : 0u;
+            if ((a.left > floor && !(fa && fa < round)) || (a.right > floor && !(fb && fb < round))) continue;
+            const NodeVals L = load_child(b, a.kids.x), R = load_child(b, a.kids.y);
+            store_above(b, a, combine(L, R), L, R);
+            flags[i] = round;
+            progress = true;
+        }
+        if (!__syncthreads_or(progress)) return;
+    }
+}
+
+// The nodes of one list (more than `floor` bodies each, their smaller children
+// finished), a thread each.
+template <int THREADS>
+struct AboveSmem {
+    float4 cm[THREADS], box03[THREADS], box45[THREADS], col[THREADS];  // finished nodes' values
+    uint32_t ids[THREADS];
+    uint32_t round[THREADS];  // the round that finished the node, 0 before
+    uint32_t count;
+};
+
+template <int THREADS>
+__device__ void fill_list(const StepBuffers& b, AboveSmem<THREADS>& S, uint32_t m, uint32_t floor) {
+    const uint32_t t = threadIdx.x;
+    AboveNode a;
+    a.left = a.right = 0;
+    if (t < m) {
+        a = above_node(b, S.ids[t]);
+        b.fill_ready[a.id] = t;  // its place, for its parent
+    }
+    S.round[t] = 0;
+    __syncthreads();
+    // children in the list by their place, the others' values now
+    uint32_t at_l = GBH_NONE, at_r = GBH_NONE;
+    NodeVals L, R, out;
+    if (t < m) {
+        if (a.left > floor) at_l = *(volatile uint32_t*)&b.fill_ready[a.kids.x - b.N]; else L = load_child(b, a.kids.x);
+        if (a.right > floor) at_r = *(volatile uint32_t*)&b.fill_ready[a.kids.y - b.N]; else R = load_child(b, a.kids.y);
+    }
+    auto get = [&](uint32_t k) {
+        NodeVals v;
+        v.cm = S.cm[k];
+        const float4 p = S.box03[k], q = S.box45[k];
+        v.col = S.col[k];
+        v.box[0] = p.x;
+        v.box[1] = p.y;
+        v.box[2] = p.z;
+        v.box[3] = p.w;
+        v.box[4] = q.x;
+        v.box[5] = q.y;
+        v.depth = __float_as_uint(q.z);
+        return v;
+    };
+    bool pending = t < m;
+    for (uint32_t round = 1;; ++round) {
+        // only what an earlier round finished: its values are behind a barrier
+        auto finished = [&](uint32_t at) {
+            if (at == GBH_NONE) return true;
+            const uint32_t f = *(volatile uint32_t*)&S.round[at];
+            return f != 0u && f < round;
+        };
+        const bool ready = pending && finished(at_l) && finished(at_r);
+        if (ready) {
+            if (at_l != GBH_NONE) L = get(at_l);
+            if (at_r != GBH_NONE) R = get(at_r);
+            out = combine(L, R);
+            S.cm[t] = out.cm;
+            S.box03[t] = make_float4(out.box[0], out.box[1], out.box[2], out.box[3]);
+            S.box45[t] = make_float4(out.box[4], out.box[5], __uint_as_float(out.depth), 0.0f);
+            S.col[t] = out.col;
+            S.round[t] = round;
+            pending = false;
+        }
+        if (!__syncthreads_or(ready)) break;
+    }
+    if (t < m) store_above(b, a, out, L, R);
+}
+
+// Fill of the nodes above the body groups for capacities up to FILL_ABOVE_MAX:
+// first a block per subtree of at most FILL_SUBTREE bodies (it finds its nodes,
+// those with more bodies than a group, by their indices, which lie in the
+// subtree's slots), then (LISTED) one block for the nodes above the subtrees, as
+// the build listed them.
+//
+// What bounds it: the chain of heights.  A climb from every group with an
+// atomic per node (release its words, meet the sibling, read its words from L2)
+// takes 2.2 us per height, 45 us for the 20 heights above the groups of 65,536
+// bodies.  Here a round takes the children's values from shared memory or
+// registers and has one barrier; the nodes are written after the last one.
+// At larger capacities the climbs (k_fill_top) hide each other's latency.  Fill
+// stage, us, climb -> subtrees: 1,024 bodies 45 -> 35, 65,536 68 -> 59, 100,000
+// 51 -> 49, 300,000 84 -> 76, 1,048,576 150 -> 158, 4,194,304 463 -> 586; with
+// three contexts' steps in flight the chain is partly hidden, a step: 1,024
+// bodies 44.5 -> 41.7, 65,536 99.9 -> 95.1, 100,000 the same, 300,000 266.8 ->
+// 268.9.  A level between with subtrees of 131,072 bodies costs 35 us for the
+// scan that finds its nodes.
+template <int THREADS, bool LISTED>
+__global__ __launch_bounds__(THREADS) void k_fill_above(StepBuffers b) {
+    extern __shared__ __align__(16) unsigned char fill_smem[];
+    AboveSmem<THREADS>& S = *reinterpret_cast<AboveSmem<THREADS>*>(fill_smem);
+    const uint32_t n = b.st->n_new;
+    if (LISTED) {
+        const uint32_t m = b.st->num_subtrees[1];
+        if (m > THREADS) {
+            fill_long_list(b, b.fill_subtrees[1], m, FILL_SUBTREE);
+        } else {
+            if (threadIdx.x < m) S.ids[threadIdx.x] = b.fill_subtrees[1][threadIdx.x];
+            fill_list<THREADS>(b, S, m, FILL_SUBTREE);
+        }
+        return;
+    }
+    if (n == 1 && blockIdx.x == 0 && threadIdx.x == 0)
+        climb_global(b, 0u, 1u, load_node_cg(&b.leaf[0]), b.N);  // the root's one child
+    const uint32_t subtrees = b.st->num_subtrees[0];
+    for (uint32_t s = blockIdx.x; s < subtrees; s += gridDim.x) {
+        const uint32_t root = b.fill_subtrees[0][s];
+        const uint32_t lo = b.node_lo[root], bodies = b.topo_cnt[root];
+        uint32_t* list = b.idx_out + lo;  // the spare index buffer: free until the next compaction
+        __syncthreads();
+        if (threadIdx.x == 0) S.count = 0;
+        __syncthreads();
+#pragma unroll 8
+        for (uint32_t k = threadIdx.x; k < bodies; k += THREADS) {
+            const uint32_t i = lo + k;
+            // at most one index of the range belongs to an ancestor (more bodies)
+            const uint32_t c = i + 1 < n ? b.topo_cnt[i] : 0u;
+            if (c > GBH_GROUP_MAX && c <= bodies) {
+                const uint32_t at = atomicAdd(&S.count, 1u);
+                list[at] = i;
+                if (at < THREADS) S.ids[at] = i;
+            }
+        }
+        __syncthreads();
+        const uint32_t m = S.count;
+        if (m > THREADS)
+            fill_long_list(b, list, m, GBH_GROUP_MAX);
+        else
+            fill_list<THREADS>(b, S, m, GBH_GROUP_MAX);
+    }
+}
+
+#define ABOVE_THREADS 128  // a subtree: about 40 nodes
+#define TOPS_THREADS 512   // the nodes above: one per 2,700 bodies
+
 void fill_setup() {
     cudaFuncSetAttribute(k_fill, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)(FILL_WARPS * sizeof(FillSmem)));
+    static_assert(sizeof(AboveSmem<TOPS_THREADS>) <= 48 * 1024, "above the default limit");
 }
 
 void launch_fill(const StepBuffers& b, cudaStream_t s) {
     // persistent: the blocks that fit at once, no more than the groups need
     const uint32_t blocks = min(b.num_sms * FILL_BLOCKS, (b.N + FILL_WARPS - 1) / FILL_WARPS);
     k_fill<<<blocks, FILL_THREADS, FILL_WARPS * sizeof(FillSmem), s>>>(b);
-    k_fill_top<<<b.num_sms * 4, 256, 0, s>>>(b);
+    if (b.N > FILL_ABOVE_MAX) {
+        k_fill_top<<<b.num_sms * 4, 256, 0, s>>>(b);
+        return;
+    }
+    k_fill_above<ABOVE_THREADS, false>
+        <<<min(b.num_sms * 4, b.N / GBH_GROUP_MAX + 1), ABOVE_THREADS, sizeof(AboveSmem<ABOVE_THREADS>), s>>>(b);
+    if (b.N > FILL_SUBTREE)
+        k_fill_above<TOPS_THREADS, true><<<1, TOPS_THREADS, sizeof(AboveSmem<TOPS_THREADS>), s>>>(b);
 }

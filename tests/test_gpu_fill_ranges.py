@@ -59,3 +59,20 @@ def test_fill_of_coinciding_bodies(gbh_lib, oracle_mod, n):
     line = (0.5 ** (1 + k % 20)).astype(np.float32)
     b["pos_mass"][:, :3] = np.where((k % 2 == 0)[:, None], 0.0, line[:, None])
     _fill_both(oracle_mod, b)
+
+
+@pytest.mark.parametrize("clusters", [3, 30, 400, 1300])
+def test_fill_of_long_chains(gbh_lib, oracle_mod, clusters):
+    # points of 97 coinciding bodies, each with bodies at halving distances:
+    # some 15 nodes above the groups per 112 bodies, more than a block has
+    # threads; the largest has a capacity whose fill climbs
+    rng = np.random.default_rng(1)
+    cells = rng.choice(16**3, clusters, replace=False)
+    corner = np.stack([cells % 16, cells // 16 % 16, cells // 256], 1) / 16.0
+    k = np.arange(6, 21)
+    per = np.concatenate([np.zeros(97), 0.5**k])
+    pos = (corner[:, None, :] + per[None, :, None]).reshape(-1, 3)
+    pos = np.concatenate([pos, [[0.0] * 3, [1.0] * 3]]).astype(np.float32)
+    b = plummer_case(len(pos), seed=1)
+    b["pos_mass"][:, :3] = pos
+    _fill_both(oracle_mod, b)
