@@ -10,11 +10,20 @@
 //     (k_prep_scatter); every block scans its pass's histogram beside its own
 //     tile's digit counts, one kernel less than scanning them first.
 //   * Each pass kernel takes a tile ticket, ranks its keys per warp (digit
-//     peers from one ballot per digit bit, ranks reserved with shared-memory
-//     atomics in item order), publishes the tile's digit counts, resolves its global digit
+//     peers from one ballot per digit bit, counts per warp and digit in 16
+//     bits), publishes the tile's digit counts, resolves its global digit
 //     offsets with a decoupled look-back (bounded spin, error word on
-//     timeout), stages keys digit-ordered in shared memory and writes them out
-//     with coalesced runs.
+//     timeout), stages the pairs digit-ordered in shared memory (the indices are
+//     loaded only now, into the registers that the keys leave) and writes them
+//     out with coalesced runs.
+// What bounds a pass: no one thing; of 8,388,608 pairs it takes 62 us where its
+// 201 MB take 30.  The ballots' integer work holds the ALU pipe 55% busy, the
+// shared memory 50%, and the rest is the chain of a tile's phases over 3 to 4
+// waves of tiles.  Counts in 16 bits read by every lane (before: 32 bits, an
+// atomic by one lane and a shuffle), late index loads and 512 threads a tile:
+// 39 -> 31 million warp instructions; sort stage, us: 1,024 pairs 52 -> 48,
+// 16,000 60 -> 52, 1,048,576 133 -> 123, 8,388,608 559 ->
+// 506, 16,777,216 1,008 -> 934.
 #include "gbh_common.cuh"
 
 #define LB_FLAG_AGG 0x40000000u
@@ -25,26 +34,26 @@
 #define LB_WINDOW 4
 #endif
 
-template <int ITEMS>
+// A tile of THREADS x ITEMS pairs.
+template <int ITEMS, int THREADS>
 struct SortSmem {
-    uint32_t warp_hist[SORT_THREADS / 32][SORT_RADIX + 1];  // +1: sentinel bucket of out-of-range items
+    uint16_t warp_hist[THREADS / 32][SORT_RADIX + 2];  // [SORT_RADIX]: sentinel bucket of out-of-range items
     uint32_t block_excl[SORT_RADIX + 1];
     uint32_t delta[SORT_RADIX];
-    uint2 warp_tot[SORT_THREADS / 32];
+    uint2 warp_tot[SORT_RADIX / 32];
     uint32_t tile;
-    unsigned long long keys[SORT_THREADS * ITEMS];
-    uint32_t vals[SORT_THREADS * ITEMS];
+    unsigned long long keys[THREADS * ITEMS];
+    uint32_t vals[THREADS * ITEMS];
 };
 
 // Warp-level stable ranking of the items, item rounds in slot order: lanes
 // with the same digit from one ballot per digit bit (BITS = 9 in a partial
-// tile, whose out-of-range slots carry the sentinel digit 256); the digit's
-// leader reserves the group's ranks with a shared-memory atomic.  A warp's
-// shared memory atomics take effect in program order, so items stay in slot
-// order.
+// tile, whose out-of-range slots carry the sentinel digit 256).  All lanes
+// read their digit's count so far, then the lowest lane of each digit writes
+// the new one.
 template <uint32_t SHIFT, int BITS, int ITEMS>
 __device__ __forceinline__ void rank_items(const uint64_t (&key)[ITEMS], uint32_t (&rank)[ITEMS],
-                                           uint32_t* warp_hist, uint32_t lane, uint32_t seg, uint32_t n) {
+                                           uint16_t* warp_hist, uint32_t lane, uint32_t seg, uint32_t n) {
 #pragma unroll
     for (int i = 0; i < ITEMS; ++i) {
         uint32_t dig = (uint32_t)(key[i] >> SHIFT) & 0xFFu;
@@ -56,35 +65,36 @@ __device__ __forceinline__ void rank_items(const uint64_t (&key)[ITEMS], uint32_
             const uint32_t m = __ballot_sync(0xffffffffu, on);
             peers &= on ? m : ~m;
         }
-        const uint32_t leader = __ffs(peers) - 1;
         const uint32_t before = __popc(peers & lanemask_lt());
-        uint32_t prev = 0;
-        if (lane == leader) prev = atomicAdd(&warp_hist[dig], (uint32_t)__popc(peers));
-        rank[i] = __shfl_sync(0xffffffffu, prev, leader) + before;
+        const uint32_t prev = warp_hist[dig];
+        __syncwarp();
+        if (before == 0) warp_hist[dig] = (uint16_t)(prev + __popc(peers));
+        __syncwarp();
+        rank[i] = prev + before;
     }
 }
 
-// One kernel instance per pass: the digit's bit offset is a constant.
-// resident blocks per SM, by the shared memory of a tile
-template <int ITEMS>
+// resident blocks per SM, by the shared memory and registers of a tile
+template <int ITEMS, int THREADS>
 struct SortBlocks {
-    static constexpr int value = ITEMS == 16 ? 3 : ITEMS == 8 ? 5 : 6;
+    static constexpr int value = THREADS == 512 ? 3 : ITEMS == 8 ? 5 : 6;
 };
 
-template <uint32_t PASS, int ITEMS>
-__global__ __launch_bounds__(SORT_THREADS, SortBlocks<ITEMS>::value) void k_sort_pass(StepBuffers b, const uint64_t* __restrict__ kin,
-                                                               const uint32_t* __restrict__ vin, uint64_t* __restrict__ kout,
-                                                               uint32_t* __restrict__ vout) {
+// One kernel instance per pass: the digit's bit offset is a constant.
+template <uint32_t PASS, int ITEMS, int THREADS>
+__global__ __launch_bounds__(THREADS, SortBlocks<ITEMS, THREADS>::value) void k_sort_pass(
+    StepBuffers b, const uint64_t* __restrict__ kin, const uint32_t* __restrict__ vin, uint64_t* __restrict__ kout,
+    uint32_t* __restrict__ vout) {
     constexpr uint32_t pass = PASS;
-    constexpr uint32_t TILE = SORT_THREADS * ITEMS;
+    constexpr uint32_t TILE = THREADS * ITEMS;
     extern __shared__ __align__(16) unsigned char smem_raw[];
-    SortSmem<ITEMS>& S = *reinterpret_cast<SortSmem<ITEMS>*>(smem_raw);
+    SortSmem<ITEMS, THREADS>& S = *reinterpret_cast<SortSmem<ITEMS, THREADS>*>(smem_raw);
     const uint32_t n = b.st->n_new;
     constexpr uint32_t shift = SORT_BITS * PASS;
     const uint32_t lane = lane_id(), w = threadIdx.x >> 5;
     if (threadIdx.x == 0) S.tile = atomicAdd(&b.st->sort_tiles[pass], 1u);
-    for (uint32_t i = threadIdx.x; i < (SORT_THREADS / 32) * (SORT_RADIX + 1); i += SORT_THREADS) {
-        (&S.warp_hist[0][0])[i] = 0;
+    for (uint32_t i = threadIdx.x; i < (THREADS / 32) * (SORT_RADIX + 2) / 2; i += THREADS) {
+        reinterpret_cast<uint32_t*>(&S.warp_hist[0][0])[i] = 0;
     }
     __syncthreads();
     const uint32_t tile = S.tile;
@@ -96,52 +106,39 @@ __global__ __launch_bounds__(SORT_THREADS, SortBlocks<ITEMS>::value) void k_sort
     const uint32_t seg = base + w * 32 * ITEMS;
     const bool full = base + TILE <= n;  // uniform over the block
     uint64_t key[ITEMS];
-    uint32_t val[ITEMS];
     uint32_t rank[ITEMS];
     if (full) {
 #pragma unroll
-        for (int i = 0; i < ITEMS; ++i) {
-            key[i] = kin[seg + i * 32 + lane];
-            val[i] = vin[seg + i * 32 + lane];
-        }
+        for (int i = 0; i < ITEMS; ++i) key[i] = kin[seg + i * 32 + lane];
         rank_items<shift, 8>(key, rank, S.warp_hist[w], lane, seg, n);
     } else {
 #pragma unroll
         for (int i = 0; i < ITEMS; ++i) {
             const uint32_t pos = seg + i * 32 + lane;
-            if (pos < n) {
-                key[i] = kin[pos];
-                val[i] = vin[pos];
-            } else {
-                key[i] = ~0ull;
-                val[i] = 0;
-            }
+            key[i] = pos < n ? kin[pos] : ~0ull;
         }
         rank_items<shift, 9>(key, rank, S.warp_hist[w], lane, seg, n);
     }
     __syncthreads();
-    // thread d: exclusive prefix of digit d over warps, tile total
+    // thread d < 256: exclusive prefix of digit d over warps, tile total
     const uint32_t d = threadIdx.x;
-    uint32_t total = 0;
-#pragma unroll
-    for (int ww = 0; ww < SORT_THREADS / 32; ++ww) {
-        const uint32_t c = S.warp_hist[ww][d];
-        S.warp_hist[ww][d] = total;
-        total += c;
-    }
-    // publish this tile's count for digit d (inclusive when it is the first tile)
+    const bool digit = THREADS == SORT_RADIX || d < SORT_RADIX;  // uniform over a warp
+    uint32_t total = 0, digit_count = 0, x = 0, y = 0;
     volatile uint32_t* my = lb + (size_t)tile * SORT_RADIX + d;
-    if (tile == 0) {
-        *my = LB_FLAG_INC | total;
-    } else {
-        *my = LB_FLAG_AGG | total;
-    }
-    // block exclusive scans over the digits: of the tile's totals (block_excl)
-    // and of the pass's histogram (where each digit begins in the output)
-    const uint32_t digit_count = b.hist[pass * SORT_RADIX + d];
-    uint32_t bucket_base;
-    {
-        uint32_t x = total, y = digit_count;
+    if (digit) {
+        digit_count = b.hist[pass * SORT_RADIX + d];
+#pragma unroll
+        for (int ww = 0; ww < THREADS / 32; ++ww) {
+            const uint32_t c = S.warp_hist[ww][d];
+            S.warp_hist[ww][d] = (uint16_t)total;
+            total += c;
+        }
+        // publish this tile's count for digit d (inclusive when it is the first tile)
+        *my = (tile == 0 ? LB_FLAG_INC : LB_FLAG_AGG) | total;
+        // block exclusive scans over the digits: of the tile's totals (block_excl)
+        // and of the pass's histogram (where each digit begins in the output)
+        x = total;
+        y = digit_count;
 #pragma unroll
         for (int o = 1; o < 32; o <<= 1) {
             const uint32_t px = __shfl_up_sync(0xffffffffu, x, o), py = __shfl_up_sync(0xffffffffu, y, o);
@@ -151,9 +148,11 @@ __global__ __launch_bounds__(SORT_THREADS, SortBlocks<ITEMS>::value) void k_sort
             }
         }
         if (lane == 31) S.warp_tot[w] = make_uint2(x, y);
-        __syncthreads();
+    }
+    __syncthreads();
+    uint32_t bucket_base = 0;
+    if (digit) {
         uint32_t off = 0;
-        bucket_base = 0;
         for (uint32_t i = 0; i < w; ++i) {
             const uint2 t = S.warp_tot[i];
             off += t.x;
@@ -167,21 +166,27 @@ __global__ __launch_bounds__(SORT_THREADS, SortBlocks<ITEMS>::value) void k_sort
     // stage digit-ordered in shared memory (tile-local offsets only), before
     // the look-back: the items leave the registers, and the predecessors
     // have longer to publish their inclusive counts
+    {
+        uint32_t val[ITEMS];
 #pragma unroll
-    for (int i = 0; i < ITEMS; ++i) {
-        const uint32_t pos = seg + i * 32 + lane;
-        if (pos < n) {
+        for (int i = 0; i < ITEMS; ++i) {
+            const uint32_t pos = seg + i * 32 + lane;
             const uint32_t dg = (uint32_t)(key[i] >> shift) & 0xFFu;
-            const uint32_t local = S.block_excl[dg] + S.warp_hist[w][dg] + rank[i];
-            S.keys[local] = key[i];
-            S.vals[local] = val[i];
+            rank[i] += S.block_excl[dg] + S.warp_hist[w][dg];
+            if (full || pos < n) {
+                S.keys[rank[i]] = key[i];
+                val[i] = vin[pos];
+            }
         }
+#pragma unroll
+        for (int i = 0; i < ITEMS; ++i)
+            if (full || seg + i * 32 + lane < n) S.vals[rank[i]] = val[i];
     }
     // decoupled look-back for digit d, LB_WINDOW predecessors per round
     // trip; tile 0 always publishes an inclusive count, so the walk ends
     // there at the latest
     uint32_t prefix = 0;
-    if (tile > 0) {
+    if (digit && tile > 0) {
         int32_t j = (int32_t)tile - 1;
         uint32_t spins = 0;
         while (true) {
@@ -220,11 +225,13 @@ __global__ __launch_bounds__(SORT_THREADS, SortBlocks<ITEMS>::value) void k_sort
         }
         *my = LB_FLAG_INC | (prefix + total);
     }
-    S.delta[d] = bucket_base + prefix - S.block_excl[d];
+    if (digit) S.delta[d] = bucket_base + prefix - S.block_excl[d];
     __syncthreads();
-    const uint32_t valid = min((uint32_t)TILE, n - base);
     bool bad = false;
-    for (uint32_t j = threadIdx.x; j < valid; j += SORT_THREADS) {
+#pragma unroll
+    for (int i = 0; i < ITEMS; ++i) {
+        const uint32_t j = i * THREADS + threadIdx.x;
+        if (!full && base + j >= n) break;
         const uint64_t k = S.keys[j];
         const uint32_t dst = S.delta[(uint32_t)(k >> shift) & 0xFFu] + j;
         if (dst < n) {  // holds whenever the digit histograms describe these keys
@@ -261,39 +268,47 @@ void launch_sort_hist(const uint64_t* keys, uint32_t n, uint32_t* hist, DevState
     k_sort_hist<<<blocks > 0 ? blocks : 1, 256, 0, s>>>(keys, n, hist, st);
 }
 
-// Items per thread of a sort of up to `n` pairs.  A small sort is eight chains of
-// latency (load, rank item after item, look back, scatter), shorter with small
-// tiles, which also reach more SMs; a large one wants long runs per digit.
-// Sort stage of an eager step, us, with 4, 8 and 16 items per thread: 1,000
-// pairs 59, 58, 75; 16,000 64, 75, 91; 150,000 84, 87, 95; 300,000 105, 93, 108;
-// 600,000 140, 114, 110; 4.2M 518, 365, 326.
-uint32_t sort_items_for(uint32_t n) { return n <= 200000u ? 4u : n <= 500000u ? 8u : 16u; }
+// Pairs per tile of a sort of up to `n` pairs, in units of 256.  A small sort is
+// eight chains of latency (load, rank item after item, look back, scatter),
+// shorter with small tiles, which also reach more SMs; a large one wants long
+// runs per digit.  Sort stage of an eager step, us, with 256 threads of 4, 8 and
+// 16 items: 1,000 pairs 59, 58, 75; 16,000 64, 75, 91; 150,000 84, 87, 95;
+// 300,000 105, 93, 108; 600,000 140, 114, 110.  Tiles of 4,096 pairs are ranked
+// by 512 threads (16 items of 256 threads: 127 for 123 us at 1,048,576 pairs,
+// 531 for 506 at 8,388,608).  Tiles of 8,192 are faster alone where they fit the
+// SMs at once and tiles of 4,096 just do not (170 for 195 us at 2,000,000 pairs,
+// but 252 for 240 at 3,000,000), and slower where steps of several contexts
+// share the SMs (a 2,000,003-body step 1,610 for 1,587 us).
+uint32_t sort_items_for(uint32_t n) {
+    return n <= 200000u ? 4u : n <= 500000u ? 8u : 16u;
+}
 
 typedef void (*sort_pass_fn)(StepBuffers, const uint64_t*, const uint32_t*, uint64_t*, uint32_t*);
 static_assert(SORT_PASSES == 8, "one kernel instance per pass");
-template <int ITEMS>
+template <int ITEMS, int THREADS>
 struct SortPasses {
-    static constexpr sort_pass_fn fn[SORT_PASSES] = {k_sort_pass<0, ITEMS>, k_sort_pass<1, ITEMS>, k_sort_pass<2, ITEMS>,
-                                                     k_sort_pass<3, ITEMS>, k_sort_pass<4, ITEMS>, k_sort_pass<5, ITEMS>,
-                                                     k_sort_pass<6, ITEMS>, k_sort_pass<7, ITEMS>};
+    static constexpr sort_pass_fn fn[SORT_PASSES] = {
+        k_sort_pass<0, ITEMS, THREADS>, k_sort_pass<1, ITEMS, THREADS>, k_sort_pass<2, ITEMS, THREADS>,
+        k_sort_pass<3, ITEMS, THREADS>, k_sort_pass<4, ITEMS, THREADS>, k_sort_pass<5, ITEMS, THREADS>,
+        k_sort_pass<6, ITEMS, THREADS>, k_sort_pass<7, ITEMS, THREADS>};
 };
 
-template <int ITEMS>
+template <int ITEMS, int THREADS>
 static void setup_passes() {
-    for (sort_pass_fn f : SortPasses<ITEMS>::fn)
-        cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(SortSmem<ITEMS>));
+    for (sort_pass_fn f : SortPasses<ITEMS, THREADS>::fn)
+        cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(SortSmem<ITEMS, THREADS>));
 }
 
 void sort_setup(uint32_t items) {
     if (items == 4)
-        setup_passes<4>();
+        setup_passes<4, 256>();
     else if (items == 8)
-        setup_passes<8>();
+        setup_passes<8, 256>();
     else
-        setup_passes<16>();
+        setup_passes<8, 512>();
 }
 
-template <int ITEMS>
+template <int ITEMS, int THREADS>
 static void launch_passes(const StepBuffers& b, cudaStream_t s) {
     // keys/index of the live bodies are in the *_in buffers (the compaction
     // swap already happened); 8 ping-pong passes through *_out end there again
@@ -301,8 +316,8 @@ static void launch_passes(const StepBuffers& b, cudaStream_t s) {
     const uint32_t* vin = b.idx_in;
     uint64_t* kt = b.keys_out;
     uint32_t* vt = b.idx_out;
-    for (sort_pass_fn f : SortPasses<ITEMS>::fn) {
-        f<<<b.sort_tiles_cap, SORT_THREADS, sizeof(SortSmem<ITEMS>), s>>>(b, kin, vin, kt, vt);
+    for (sort_pass_fn f : SortPasses<ITEMS, THREADS>::fn) {
+        f<<<b.sort_tiles_cap, THREADS, sizeof(SortSmem<ITEMS, THREADS>), s>>>(b, kin, vin, kt, vt);
         const uint64_t* nk = kt;
         const uint32_t* nv = vt;
         kt = const_cast<uint64_t*>(kin);
@@ -314,9 +329,9 @@ static void launch_passes(const StepBuffers& b, cudaStream_t s) {
 
 void launch_sort(const StepBuffers& b, cudaStream_t s) {
     if (b.sort_items == 4)
-        launch_passes<4>(b, s);
+        launch_passes<4, 256>(b, s);
     else if (b.sort_items == 8)
-        launch_passes<8>(b, s);
+        launch_passes<8, 256>(b, s);
     else
-        launch_passes<16>(b, s);
+        launch_passes<8, 512>(b, s);
 }
