@@ -143,7 +143,7 @@ struct StepBuffers {
     uint32_t ticket_clear;  // 1: the build just cleared the group walk's ticket
     uint32_t N;
     uint32_t sort_tiles_cap;
-    uint32_t sort_items;  // pairs per tile of the sort, in units of 256 (4, 8; else 16)
+    uint32_t sort_items;  // pairs per tile of the sort, in units of 256 (4, 8; 32: one block sorts all; else 16)
     uint32_t prep_tiles_cap;
     uint32_t num_sms;  // multiprocessors of the context's device (grid sizes of the persistent kernels)
     // sharded walk: this rank's share of the live bodies (world 1: all)

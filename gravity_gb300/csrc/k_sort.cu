@@ -9,6 +9,7 @@
 //   * The eight digit histograms are accumulated by the encode pass
 //     (k_prep_scatter); every block scans its pass's histogram beside its own
 //     tile's digit counts, one kernel less than scanning them first.
+//   * Up to 4,096 pairs one block does all passes (k_sort_small); above:
 //   * Each pass kernel takes a tile ticket, ranks its keys per warp (digit
 //     peers from one ballot per digit bit, counts per warp and digit in 16
 //     bits), publishes the tile's digit counts, resolves its global digit
@@ -21,8 +22,8 @@
 // shared memory 50%, and the rest is the chain of a tile's phases over 3 to 4
 // waves of tiles.  Counts in 16 bits read by every lane (before: 32 bits, an
 // atomic by one lane and a shuffle), late index loads and 512 threads a tile:
-// 39 -> 31 million warp instructions; sort stage, us: 1,024 pairs 52 -> 48,
-// 16,000 60 -> 52, 1,048,576 133 -> 123, 8,388,608 559 ->
+// 39 -> 31 million warp instructions; sort stage, us: 16,000 pairs 60 ->
+// 52, 1,048,576 133 -> 123, 8,388,608 559 ->
 // 506, 16,777,216 1,008 -> 934.
 #include "gbh_common.cuh"
 
@@ -244,6 +245,133 @@ __global__ __launch_bounds__(THREADS, SortBlocks<ITEMS, THREADS>::value) void k_
     if (bad) set_error(b.st, GBH_DEVERR_SORT_LOOKBACK);
 }
 
+#define SMALL_THREADS 1024
+#define SMALL_MAX (SMALL_THREADS * 4u)
+
+// The whole sort of up to SMALL_THREADS x ITEMS pairs by one block, pairs in
+// registers and shared memory between the passes.
+template <int ITEMS>
+struct SmallSortSmem {
+    uint32_t warp_hist[2][SMALL_THREADS / 32][SORT_RADIX / 2 + 1];  // 16-bit counts, then positions; passes alternate
+    uint32_t warp_tot[SMALL_THREADS / 32];
+    unsigned long long keys[SMALL_THREADS * ITEMS];
+    uint32_t vals[SMALL_THREADS * ITEMS];
+};
+
+// What bounds it: the latency of a pass, the ranking and four barriers, 1.7 us
+// with one item per thread and 4.3 with four, where a kernel per pass takes 6.
+// Sort stage, us, eight kernels -> one: 1,000 pairs 48 -> 17, 2,000 50 -> 24,
+// 4,000 51 -> 37; with eight items per thread 6,000 51 -> 49, 8,000 52 -> 61: so
+// up to four.  A 1,024-body step with three contexts' steps in flight: 39.8 ->
+// 34.2 us.
+template <int ITEMS>
+__global__ __launch_bounds__(SMALL_THREADS) void k_sort_small(StepBuffers b, uint64_t* __restrict__ keys,
+                                                              uint32_t* __restrict__ vals) {
+    constexpr int PARTS = SMALL_THREADS / SORT_RADIX;  // threads per digit in the scan
+    extern __shared__ __align__(16) unsigned char smem_raw[];
+    SmallSortSmem<ITEMS>& S = *reinterpret_cast<SmallSortSmem<ITEMS>*>(smem_raw);
+    const uint32_t n = min(b.st->n_new, (uint32_t)(SMALL_THREADS * ITEMS));
+    const uint32_t lane = lane_id(), w = threadIdx.x >> 5;
+    const uint32_t rounds = (n + SMALL_THREADS - 1) / SMALL_THREADS;  // items of each thread in use
+    const uint32_t seg = w * 32 * rounds + lane;                      // item i of the thread at seg + 32 i
+    uint64_t key[ITEMS];
+    uint32_t val[ITEMS], rank[ITEMS];
+#pragma unroll
+    for (int i = 0; i < ITEMS; ++i)
+        if (i < rounds && seg + i * 32 < n) {
+            key[i] = keys[seg + i * 32];
+            val[i] = vals[seg + i * 32];
+        }
+    for (uint32_t i = threadIdx.x; i < sizeof(S.warp_hist) / 4; i += SMALL_THREADS) (&S.warp_hist[0][0][0])[i] = 0;
+    __syncthreads();
+#pragma unroll 1
+    for (uint32_t pass = 0; pass < SORT_PASSES; ++pass) {
+        uint16_t* hist = reinterpret_cast<uint16_t*>(S.warp_hist[pass & 1][w]);
+        const uint32_t shift = SORT_BITS * pass;
+#pragma unroll
+        for (int i = 0; i < ITEMS; ++i) {
+            if (i >= rounds) break;
+            const bool in = seg + i * 32 < n;
+            const uint32_t dig = (uint32_t)(key[i] >> shift) & 0xFFu;
+            uint32_t peers = __ballot_sync(0xffffffffu, in);
+#pragma unroll
+            for (int bit = 0; bit < SORT_BITS; ++bit) {
+                const bool on = (dig >> bit) & 1u;
+                const uint32_t m = __ballot_sync(0xffffffffu, on);
+                peers &= on ? m : ~m;
+            }
+            const uint32_t before = __popc(peers & lanemask_lt());
+            const uint32_t prev = hist[dig];
+            __syncwarp();
+            if (in && before == 0) hist[dig] = (uint16_t)(prev + __popc(peers));
+            __syncwarp();
+            rank[i] = prev + before;
+        }
+        __syncthreads();
+        // counts -> positions: one exclusive scan over (digit, warp); each
+        // thread holds the counts of a digit in some of the warps
+        {
+            constexpr int ROWS = SMALL_THREADS / 32 / PARTS;
+            const uint32_t d = threadIdx.x / PARTS, first = threadIdx.x % PARTS * ROWS;
+            uint32_t sum = 0, c[ROWS];
+#pragma unroll
+            for (int r = 0; r < ROWS; ++r) {
+                c[r] = reinterpret_cast<const uint16_t*>(S.warp_hist[pass & 1][first + r])[d];
+                sum += c[r];
+            }
+            uint32_t x = sum;
+#pragma unroll
+            for (int o = 1; o < 32; o <<= 1) {
+                const uint32_t p = __shfl_up_sync(0xffffffffu, x, o);
+                if (lane >= (uint32_t)o) x += p;
+            }
+            if (lane == 31) S.warp_tot[w] = x;
+            __syncthreads();
+            uint32_t t = lane < SMALL_THREADS / 32 ? S.warp_tot[lane] : 0u;
+            const uint32_t own = t;
+#pragma unroll
+            for (int o = 1; o < 32; o <<= 1) {
+                const uint32_t p = __shfl_up_sync(0xffffffffu, t, o);
+                if (lane >= (uint32_t)o) t += p;
+            }
+            uint32_t at = __shfl_sync(0xffffffffu, t - own, w) + x - sum;
+#pragma unroll
+            for (int r = 0; r < ROWS; ++r) {
+                reinterpret_cast<uint16_t*>(S.warp_hist[pass & 1][first + r])[d] = (uint16_t)at;
+                at += c[r];
+            }
+            // the next pass counts in the other buffer, last read a pass ago
+            for (uint32_t i = threadIdx.x; i < sizeof(S.warp_hist) / 8; i += SMALL_THREADS)
+                (&S.warp_hist[(pass + 1) & 1][0][0])[i] = 0;
+        }
+        __syncthreads();
+#pragma unroll
+        for (int i = 0; i < ITEMS; ++i) {
+            if (i >= rounds) break;
+            if (seg + i * 32 < n) {
+                const uint32_t pos = hist[(uint32_t)(key[i] >> shift) & 0xFFu] + rank[i];
+                if (pass + 1 == SORT_PASSES) {
+                    keys[pos] = key[i];
+                    vals[pos] = val[i];
+                } else {
+                    S.keys[pos] = key[i];
+                    S.vals[pos] = val[i];
+                }
+            }
+        }
+        if (pass + 1 == SORT_PASSES) break;
+        __syncthreads();
+#pragma unroll
+        for (int i = 0; i < ITEMS; ++i) {
+            if (i >= rounds) break;
+            if (seg + i * 32 < n) {
+                key[i] = S.keys[seg + i * 32];
+                val[i] = S.vals[seg + i * 32];
+            }
+        }
+    }
+}
+
 // The eight digit histograms of `n` keys (for a sort whose keys were not
 // written by the step's encode pass) and the live count the passes read.
 __global__ void k_sort_hist(const uint64_t* __restrict__ keys, uint32_t n, uint32_t* __restrict__ hist,
@@ -279,7 +407,9 @@ void launch_sort_hist(const uint64_t* keys, uint32_t n, uint32_t* hist, DevState
 // SMs at once and tiles of 4,096 just do not (170 for 195 us at 2,000,000 pairs,
 // but 252 for 240 at 3,000,000), and slower where steps of several contexts
 // share the SMs (a 2,000,003-body step 1,610 for 1,587 us).
+#define SORT_ONE_BLOCK 32u  // of sort_items: the whole sort by one block (one tile of 8,192 in the counts)
 uint32_t sort_items_for(uint32_t n) {
+    if (n <= SMALL_MAX) return SORT_ONE_BLOCK;
     return n <= 200000u ? 4u : n <= 500000u ? 8u : 16u;
 }
 
@@ -299,8 +429,19 @@ static void setup_passes() {
         cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(SortSmem<ITEMS, THREADS>));
 }
 
+static const void* small_sort(uint32_t n, uint32_t* smem) {
+    if (n <= SMALL_THREADS) return *smem = sizeof(SmallSortSmem<1>), (const void*)k_sort_small<1>;
+    return *smem = sizeof(SmallSortSmem<4>), (const void*)k_sort_small<4>;
+}
+
 void sort_setup(uint32_t items) {
-    if (items == 4)
+    if (items == SORT_ONE_BLOCK) {
+        for (uint32_t n : {SMALL_THREADS * 1u, SMALL_MAX}) {
+            uint32_t smem;
+            const void* f = small_sort(n, &smem);
+            cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+        }
+    } else if (items == 4)
         setup_passes<4, 256>();
     else if (items == 8)
         setup_passes<8, 256>();
@@ -328,7 +469,12 @@ static void launch_passes(const StepBuffers& b, cudaStream_t s) {
 }
 
 void launch_sort(const StepBuffers& b, cudaStream_t s) {
-    if (b.sort_items == 4)
+    if (b.sort_items == SORT_ONE_BLOCK) {
+        uint32_t smem;
+        const void* f = small_sort(b.N, &smem);
+        void* args[] = {(void*)&b, (void*)&b.keys_in, (void*)&b.idx_in};
+        cudaLaunchKernel(f, dim3(1), dim3(SMALL_THREADS), args, smem, s);
+    } else if (b.sort_items == 4)
         launch_passes<4, 256>(b, s);
     else if (b.sort_items == 8)
         launch_passes<8, 256>(b, s);

@@ -13,7 +13,8 @@ pytestmark = pytest.mark.gpu
 
 # capacity, live bodies: partial and full tiles of 1,024, 2,048 and 4,096 pairs,
 # one pair, none beyond the first tile
-@pytest.mark.parametrize("capacity, live", [(2, 1), (1024, 1024), (1025, 1025), (200000, 199681), (200001, 200001),
+@pytest.mark.parametrize("capacity, live", [(2, 1), (33, 33), (1024, 1024), (1025, 1025), (4096, 4095),
+                                            (4097, 4097), (8192, 8192), (8192, 0), (8193, 8193), (200000, 199681), (200001, 200001),
                                             (500000, 2048), (500001, 500001), (500001, 4097), (1867776, 1867776),
                                             (1867777, 1867777), (2490368, 2490368), (2490368, 8193), (2490369, 2490369)])
 @pytest.mark.parametrize("lattice", [False, True])
@@ -26,7 +27,7 @@ def test_sort_is_the_stable_sort(gbh_lib, capacity, live, lattice):
         b["pos_mass"][:, 2] = k % 2
     dead = np.random.default_rng(2).permutation(capacity)[live:]
     b["pos_mass"][dead, 3] = 0.0
-    sim = BarnesHut(capacity, ic.exact_bounds(b) if capacity > 2 else np.array([-1, -1, -1, 1, 1, 1], np.float32),
+    sim = BarnesHut(capacity, ic.exact_bounds(b) if live > 1 else np.array([-1, -1, -1, 1, 1, 1], np.float32),
                     abi.units(G=1.0))
     sim.upload_bodies(b)
     sim.init()
