@@ -451,14 +451,14 @@ def train_out_of_sample(bh, args, local, held: list) -> dict:
 
 def kernels_per_step(mac_mode: int, merging: bool, capacity: int) -> int:
     """Kernels of this library launched by one step (the CUDA graph's kernel
-    nodes): prepare 3 (the first also resets), sort 8 passes (1 kernel with a
-    capacity of up to 4,096 bodies), build 1 (it also lists the
+    nodes): prepare 3 (the first also resets; 1 with a capacity of up to 2,048
+    bodies), sort 8 passes (1 kernel up to 4,096), build 1 (it also lists the
     group walks' body groups; with the group and learned walks 2: then the
     groups' start lists), fill 2 (3 with a capacity of 4,097 to 131,072 bodies),
     walk 1, merge resolution 4 (in steps that merge), swap 0 (a pointer swap)."""
     fill = 3 if 4096 < capacity <= 131072 else 2
     sort = 1 if capacity <= 4096 else 8
-    return 3 + sort + (1 if mac_mode == abi.MAC_PLAIN else 2) + fill + 1 + (4 if merging else 0)
+    return (1 if capacity <= 2048 else 3) + sort + (1 if mac_mode == abi.MAC_PLAIN else 2) + fill + 1 + (4 if merging else 0)
 
 
 def measure_e2e(bh, p_head, n, e2e_steps, local, dist=None) -> dict:
