@@ -464,7 +464,8 @@ __device__ __forceinline__ NodeVals fill_vals(const FillSmem& S, uint32_t kid) {
 
 // Fill of the body groups, one warp each (persistent: each warp takes every
 // W-th group).  A group is a subtree, so no node of it depends on another
-// warp, and the nodes above the groups (one per group) are left to k_fill_top.
+// warp, and the nodes above the groups (one per group) are left to k_fill_above
+// or k_fill_top.
 //   1. Every lane initialises its leaves and keeps their values in shared
 //      memory, beside its nodes' children.
 //   2. Rounds: the nodes whose children are finished (masks of finished
