@@ -144,7 +144,10 @@ int enqueue_sort(gbh_ctx* c) {
     return check_launch(c, "sort");
 }
 
-int enqueue_build(gbh_ctx* c) {
+// `fork` (while a step's graph is captured): the start lists become a branch
+// that begins after the build, on the copy stream; the caller joins it before
+// the walk.
+static int enqueue_build_with(gbh_ctx* c, bool fork) {
     if (!c->groups_clear) CUDA_TRY(c, cudaMemsetAsync(&c->st->num_groups, 0, 12, c->stream));
     c->groups_clear = false;
     c->ticket_clear = true;
@@ -152,9 +155,15 @@ int enqueue_build(gbh_ctx* c) {
     // the group walks' start lists belong to the tree: built with it when a
     // group walk is selected (otherwise the group walk builds them itself)
     c->paths_current = c->mac_mode != GBH_MAC_PLAIN;
-    if (c->paths_current) launch_group_paths(ctx_buffers(c), c->stream);
+    if (c->paths_current && fork) {
+        CUDA_TRY(c, cudaEventRecord(c->fork_event, c->stream));
+        CUDA_TRY(c, cudaStreamWaitEvent(c->copy_stream, c->fork_event, 0));
+    }
+    if (c->paths_current) launch_group_paths(ctx_buffers(c), fork ? c->copy_stream : c->stream);
     return check_launch(c, "build");
 }
+
+int enqueue_build(gbh_ctx* c) { return enqueue_build_with(c, false); }
 
 int enqueue_fill(gbh_ctx* c) {
     launch_fill(ctx_buffers(c), c->stream);
@@ -192,12 +201,22 @@ static bool stage_idle(const gbh_ctx* c, int stage) {
     return k_stages[stage] == enqueue_merge && c->params_host.merging_collision_or_neither != GBH_MODE_MERGE;
 }
 
-// the step as one sequence: the reset runs inside the compaction's first kernel
+// the step as one graph, captured from c->stream: the reset runs inside the
+// compaction's first kernel, and the group walks' start lists beside the fill
+// (they need the topology only, and 128 threads of them fit on an SM beside the
+// fill's blocks).  Step with three contexts in flight, us, one after the other
+// -> beside: 299,993 bodies learned 260 -> 251, 2,000,003 group walk 1,567 ->
+// 1,556; from 8.4M bodies on the same.
 static int enqueue_step(gbh_ctx* c) {
+    const bool fork = c->mac_mode != GBH_MAC_PLAIN;
     int rc = enqueue_prepare_with(c, true);
     for (int s = 0; s < GBH_NUM_STAGES && !rc; ++s) {
         if (k_stages[s] == enqueue_reset || k_stages[s] == enqueue_prepare || stage_idle(c, s)) continue;
-        rc = k_stages[s](c);
+        rc = k_stages[s] == enqueue_build ? enqueue_build_with(c, fork) : k_stages[s](c);
+        if (!rc && fork && k_stages[s] == enqueue_fill) {  // join
+            CUDA_TRY(c, cudaEventRecord(c->fork_event, c->copy_stream));
+            CUDA_TRY(c, cudaStreamWaitEvent(c->stream, c->fork_event, 0));
+        }
     }
     return rc;
 }
@@ -381,6 +400,7 @@ int gbh_create(gbh_ctx** out, uint32_t n, const float bounds[6], const gbh_units
     if (e == cudaSuccess) e = cudaStreamCreateWithFlags(&c->copy_stream, cudaStreamNonBlocking);
     for (cudaEvent_t& ev : c->copy_events)
         if (e == cudaSuccess) e = cudaEventCreateWithFlags(&ev, cudaEventDisableTiming);
+    if (e == cudaSuccess) e = cudaEventCreateWithFlags(&c->fork_event, cudaEventDisableTiming);
     if (e == cudaSuccess) e = cudaMemsetAsync(c->arena, 0, A.total, c->stream);
     // SimulationValues as packed by GPU.packValues (GPU.java:1096-1143)
     gbh_sim_values sv;
@@ -429,7 +449,7 @@ int gbh_destroy(gbh_ctx* c) {
         cudaStreamSynchronize(c->copy_stream2);
         cudaStreamDestroy(c->copy_stream2);
     }
-    for (cudaEvent_t e : {c->ev_in_ready, c->ev_out_ready, c->ev_out_done})
+    for (cudaEvent_t e : {c->fork_event, c->ev_in_ready, c->ev_out_ready, c->ev_out_done})
         if (e) cudaEventDestroy(e);
     // the role pointers (state, output, stage_in, spare) may name any of the
     // four body buffers: free the allocations

@@ -84,6 +84,9 @@ struct gbh_ctx {
     // one event per chunk (created with the context)
     cudaStream_t copy_stream = nullptr;
     cudaEvent_t copy_events[16] = {};
+    // names the fork and the join of the step's graph while it is captured (the
+    // copy stream stands for the branch)
+    cudaEvent_t fork_event = nullptr;
 
     // gbh_step_streamed: two more body buffers (allocated on first use), one
     // taking the next input and one the result waiting for its read-back;

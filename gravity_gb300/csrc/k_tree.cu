@@ -190,6 +190,8 @@ void launch_build_nodes(const StepBuffers& b, cudaStream_t s) {
     k_build_nodes<<<(b.N + 255) / 256, 256, 0, s>>>(b);
 }
 
+#define PATHS_THREADS 128  // one block fits on an SM beside k_fill's five (4,096 registers left)
+
 // Where each group's walk starts: the group's own subtree and the sibling of
 // every ancestor of it, which together hold every body once.  A walk from the
 // root opens each ancestor of the group anyway (its box holds the group's
@@ -197,7 +199,7 @@ void launch_build_nodes(const StepBuffers& b, cudaStream_t s) {
 // the same accepted and listed nodes without those rounds.  One thread per
 // group climbs the parent links; a group deeper than GBH_PATH_WORDS - 2
 // levels, or past the list's capacity, starts from the root (count 0).
-__global__ __launch_bounds__(256) void k_group_paths(StepBuffers b) {
+__global__ __launch_bounds__(PATHS_THREADS) void k_group_paths(StepBuffers b) {
     const uint32_t gi = blockIdx.x * blockDim.x + threadIdx.x;
     const uint32_t ng = min(b.st->num_groups, b.group_path_cap);
     if (gi >= ng) return;
@@ -224,7 +226,7 @@ void launch_group_paths(const StepBuffers& b, cudaStream_t s) {
     // the groups of the step are counted on the device: enough threads for
     // the list's capacity, the surplus returns at once
     const uint32_t threads = min(b.N, b.group_path_cap);
-    k_group_paths<<<(threads + 255) / 256, 256, 0, s>>>(b);
+    k_group_paths<<<(threads + PATHS_THREADS - 1) / PATHS_THREADS, PATHS_THREADS, 0, s>>>(b);
 }
 
 void launch_build(const StepBuffers& b, cudaStream_t s) {
