@@ -6,9 +6,10 @@
 // visit and a global atomic per opened node.
 //
 // Both kernels here give a warp 32 consecutive bodies of the Morton order
-// (spatial neighbours) and ONE shared stack of (node, mask of the lanes whose
-// own walk opened the node), so every lane interacts with exactly the nodes
-// that its own reference walk would interact with.  The children of an opened
+// (spatial neighbours; k_walk_plain 4 or 8 in small states) and ONE shared stack
+// of (node, mask of the lanes whose own walk opened the node), so every lane
+// interacts with exactly the nodes that its own reference walk would interact
+// with.  The children of an opened
 // node come as one 64-byte ChildPair record.
 //
 //   k_walk_plain     gravity and merges, FP32 and the precision form.  Up to 16
@@ -48,7 +49,8 @@
 // 4,194,301-body mixture at theta 0.5 8.04 -> 3.14 -> 2.88; 2,097,152-body
 // galaxy pair, precision form, 6.43 -> 2.50 -> 2.08; 1,048,576-body merge state
 // at theta 0.7 0.457 -> 0.352 -> 0.338; 65,536-body Plummer sphere 0.289 ->
-// 0.092 -> 0.080; 1,024 bodies 0.131 -> 0.045 -> 0.041.  Popping 32 nodes and
+// 0.092 -> 0.080; 1,024 bodies 0.131 -> 0.045 -> 0.041 (0.035 with 4 bodies per
+// warp).  Popping 32 nodes and
 // classifying both children of each in turn: 4.12 ms on the mixture.
 
 #define PW_THREADS 128
@@ -94,7 +96,7 @@ struct PlainSmem {
 // (com - x_b) - lo_b for a node, and the leaf terms are summed with Kahan
 // compensation apart from the node terms.  Gravity only.
 template <int FORM>
-__global__ __launch_bounds__(PW_THREADS, PlainBlocks<FORM>::value) void k_walk_plain(StepBuffers b) {
+__global__ __launch_bounds__(PW_THREADS, PlainBlocks<FORM>::value) void k_walk_plain(StepBuffers b, uint32_t per_warp) {
     constexpr bool PREC = FORM == PF_PREC;
     constexpr bool MERGE = FORM == PF_MERGE;
     __shared__ PlainSmem<FORM> s_warp[PW_WARPS];
@@ -103,13 +105,13 @@ __global__ __launch_bounds__(PW_THREADS, PlainBlocks<FORM>::value) void k_walk_p
     const uint32_t n = b.st->n_new;
     const uint32_t N = b.N;
     const uint32_t lane = lane_id(), w = threadIdx.x >> 5;
-    const uint32_t base = (blockIdx.x * PW_WARPS + w) * 32;
+    const uint32_t base = (blockIdx.x * PW_WARPS + w) * per_warp;
     const uint32_t g = base + lane;
     if (blockIdx.x == 0 && threadIdx.x == 0) b.st->sorted_valid = 1u;  // the update below fills sorted_pm
     uint32_t s_lo, s_hi;
     shard_slots(b, n, s_lo, s_hi);
-    const uint32_t block_first = blockIdx.x * PW_THREADS;
-    if (block_first >= n || block_first + PW_THREADS <= s_lo || block_first >= s_hi) return;
+    const uint32_t per_block = PW_WARPS * per_warp, block_first = blockIdx.x * per_block;
+    if (block_first >= n || block_first + per_block <= s_lo || block_first >= s_hi) return;
     if (threadIdx.x == 0) {
         s_inter = s_opened = 0ull;
         s_depth = 0u;
@@ -117,7 +119,7 @@ __global__ __launch_bounds__(PW_THREADS, PlainBlocks<FORM>::value) void k_walk_p
     __syncthreads();
     // every live body of the warp walks, so that a body's sums do not depend on
     // the sharding; only the shard's own bodies count, merge and are updated
-    const bool active = g < n;
+    const bool active = lane < per_warp && g < n;
     const bool owned = active && g >= s_lo && g < s_hi;
     const uint32_t everyone = __ballot_sync(0xffffffffu, active);
     const uint32_t owners = __ballot_sync(0xffffffffu, owned);
@@ -746,14 +748,25 @@ __global__ __launch_bounds__(WALK_THREADS) void k_walk_collide(StepBuffers b) {
     walk_update(b, P, sim, g, bi, pm, vd, ax, ay, az);
 }
 
+// Bodies per warp.  A small state leaves most of the GPU idle, and its walk is
+// the longest warp's chain, shorter with fewer bodies (a smaller box opens fewer
+// nodes), until the warps need each other's issue slots.  Walk stage, us, 32, 16,
+// 8 and 4 bodies per warp, Plummer spheres at theta 0.5: 1,024 bodies 45, 41, 37,
+// 35; 4,096 53, 45, 41, 39; 8,192 55, 51, 47, 47; 16,384 61, 57, 59, 70; 32,768
+// 72, 66, 80, 119.  Steps with three contexts in flight: 1,024 bodies 34.1 ->
+// 31.0 us, 4,096 50.5 -> 47.6, 8,192 58.3 -> 57.8, 6,000 in the precision form
+// 66.1 -> 63.0, but 24,000 with 16 per warp 68.6 -> 69.9.
+static uint32_t bodies_per_warp(uint32_t n) { return n <= 4096u ? 4u : n <= 8192u ? 8u : 32u; }
+
 void launch_walk_plain(const StepBuffers& b, cudaStream_t s) {
-    const uint32_t blocks = (b.N + PW_THREADS - 1) / PW_THREADS;
+    const uint32_t per_warp = bodies_per_warp(b.N);
+    const uint32_t blocks = (b.N + PW_WARPS * per_warp - 1) / (PW_WARPS * per_warp);
     if (b.collide)
         k_walk_collide<<<(b.N + WALK_THREADS - 1) / WALK_THREADS, WALK_THREADS, 0, s>>>(b);
     else if (b.prec)
-        k_walk_plain<PF_PREC><<<blocks, PW_THREADS, 0, s>>>(b);
+        k_walk_plain<PF_PREC><<<blocks, PW_THREADS, 0, s>>>(b, per_warp);
     else if (b.merge)
-        k_walk_plain<PF_MERGE><<<blocks, PW_THREADS, 0, s>>>(b);
+        k_walk_plain<PF_MERGE><<<blocks, PW_THREADS, 0, s>>>(b, per_warp);
     else
-        k_walk_plain<PF_FP32><<<blocks, PW_THREADS, 0, s>>>(b);
+        k_walk_plain<PF_FP32><<<blocks, PW_THREADS, 0, s>>>(b, per_warp);
 }

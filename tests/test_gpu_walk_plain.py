@@ -64,3 +64,22 @@ def test_walk_of_a_tall_tree(gbh_lib, oracle_mod):
         assert abs(int(g.read_stats().interactions) - int(o.read_stats().interactions)) <= 2
         far = np.linalg.norm(ao, axis=1) > 0
         assert np.median(rel_err(ag[far], ao[far])) < 1e-5
+
+
+# capacities at the edges of the ranges with 4, 8 and 32 bodies per warp, live
+# bodies at the edges of a warp and of a block
+@pytest.mark.parametrize("capacity, live", [(4096, 4096), (4096, 5), (4097, 4096), (8192, 8191), (8192, 33), (8193, 31),
+                                            (8193, 32), (8193, 33), (8193, 129), (8193, 8193)])
+@pytest.mark.parametrize("theta", [0.0, 0.5])
+def test_walk_bodies_per_warp(gbh_lib, oracle_mod, capacity, live, theta):
+    b = plummer_case(capacity, seed=capacity)
+    alive = np.sort(np.random.default_rng(3).permutation(capacity)[:live])
+    dead = np.setdiff1d(np.arange(capacity), alive)
+    b["pos_mass"][dead, 3] = 0.0
+    g, o = make_pair(oracle_mod, BarnesHut, b, bounds_of(b))
+    ag, ao = _walk(g, o, abi.step_params(theta=theta, softening=1e-4, flags=abi.FLAG_STORE_ACCEL))
+    ig, io = g.read_stats().interactions, o.read_stats().interactions
+    assert abs(int(ig) - int(io)) <= 1e-4 * io
+    if theta == 0.0:
+        assert ig == live * (live - 1)
+    assert np.median(rel_err(ag[alive], ao[alive])) < 1e-5
