@@ -6,7 +6,7 @@
 // visit and a global atomic per opened node.
 //
 // Both kernels here give a warp 32 consecutive bodies of the Morton order
-// (spatial neighbours; k_walk_plain 4 or 8 in small states) and ONE shared stack
+// (spatial neighbours; 4, 8 or 16 in small states) and ONE shared stack
 // of (node, mask of the lanes whose own walk opened the node), so every lane
 // interacts with exactly the nodes that its own reference walk would interact
 // with.  The children of an opened
@@ -605,19 +605,19 @@ struct __align__(16) StackEntry {
     uint32_t pad;
 };
 
-__global__ __launch_bounds__(WALK_THREADS) void k_walk_collide(StepBuffers b) {
+__global__ __launch_bounds__(WALK_THREADS) void k_walk_collide(StepBuffers b, uint32_t per_warp) {
     __shared__ StackEntry s_stack[WALK_WARPS][WALK_STACK];
     const uint32_t n = b.st->n_new;
     const uint32_t N = b.N;
     const uint32_t lane = lane_id(), w = threadIdx.x >> 5;
-    const uint32_t warp_global = blockIdx.x * WALK_WARPS + w;
-    const uint32_t g = warp_global * 32 + lane;
+    const uint32_t base = (blockIdx.x * WALK_WARPS + w) * per_warp;
+    const uint32_t g = base + lane;
     if (blockIdx.x == 0 && threadIdx.x == 0) b.st->sorted_valid = 1u;  // the update below fills sorted_pm
-    if (warp_global * 32 >= n) return;
+    if (base >= n) return;
     uint32_t s_lo, s_hi;
     shard_slots(b, n, s_lo, s_hi);
-    if (warp_global * 32 + 32 <= s_lo || warp_global * 32 >= s_hi) return;
-    const bool active = g < n && g >= s_lo && g < s_hi;
+    if (base + per_warp <= s_lo || base >= s_hi) return;
+    const bool active = lane < per_warp && g < n && g >= s_lo && g < s_hi;
     const gbh_step_params* P = b.params;
     const gbh_sim_values* sim = b.sim;
     const float G = sim->gravitational_constant;
@@ -758,11 +758,22 @@ __global__ __launch_bounds__(WALK_THREADS) void k_walk_collide(StepBuffers b) {
 // 66.1 -> 63.0, but 24,000 with 16 per warp 68.6 -> 69.9.
 static uint32_t bodies_per_warp(uint32_t n) { return n <= 4096u ? 4u : n <= 8192u ? 8u : 32u; }
 
+// The same for the collision kernel, where one node at a time makes the chain
+// longer.  Walk stage, us, 32, 16, 8 and 4 bodies per warp, bodies in a box at
+// theta 0.7: 1,024 bodies 39, 31, 27, 21; 8,192 51, 39, 35, 31; 16,384 55, 41, 35,
+// 35; 32,768 59, 47, 47, 59; 65,536 68, 61, 78, 96; 100,003 72, 80, 98, 139.  Steps
+// with three contexts in flight: 1,024 bodies 34.1 -> 26.9 us, 8,192 56.0 -> 48.3,
+// 16,384 59.0 -> 53.6, 32,768 65.0 -> 62.2.
+static uint32_t collide_per_warp(uint32_t n) {
+    return n <= 8192u ? 4u : n <= 16384u ? 8u : n <= 32768u ? 16u : 32u;
+}
+
 void launch_walk_plain(const StepBuffers& b, cudaStream_t s) {
     const uint32_t per_warp = bodies_per_warp(b.N);
     const uint32_t blocks = (b.N + PW_WARPS * per_warp - 1) / (PW_WARPS * per_warp);
+    const uint32_t per_block = WALK_WARPS * collide_per_warp(b.N);
     if (b.collide)
-        k_walk_collide<<<(b.N + WALK_THREADS - 1) / WALK_THREADS, WALK_THREADS, 0, s>>>(b);
+        k_walk_collide<<<(b.N + per_block - 1) / per_block, WALK_THREADS, 0, s>>>(b, collide_per_warp(b.N));
     else if (b.prec)
         k_walk_plain<PF_PREC><<<blocks, PW_THREADS, 0, s>>>(b, per_warp);
     else if (b.merge)

@@ -83,3 +83,29 @@ def test_walk_bodies_per_warp(gbh_lib, oracle_mod, capacity, live, theta):
     if theta == 0.0:
         assert ig == live * (live - 1)
     assert np.median(rel_err(ag[alive], ao[alive])) < 1e-5
+
+
+# the collision walk's result does not depend on the bodies per warp (4, 8, 16
+# or 32 by capacity): the same live bodies in capacities of all four ranges
+@pytest.mark.parametrize("live", [1, 5, 33, 129, 8191])
+def test_collision_walk_bodies_per_warp(gbh_lib, live):
+    rng = np.random.default_rng(live)
+    pos = rng.uniform(-1, 1, (live, 3)).astype(np.float32)
+    results = []
+    for capacity in (8192, 8193, 16385, 32769):
+        b = np.zeros(capacity, abi.BODY_DTYPE)
+        b["pos_mass"][:live, :3] = pos
+        b["pos_mass"][:live, 3] = 1.0 / live
+        b["vel_density"][:live, :3] = 1.0 - 2.0 * pos[:, ::-1]
+        b["vel_density"][:live, 3] = 2.0  # radii of some percent of the box: contacts
+        sim = BarnesHut(capacity, np.array([-1, -1, -1, 1, 1, 1], np.float32), abi.units(G=1.0))
+        sim.upload_bodies(b)
+        sim.init()
+        p = abi.step_params(dt=1e-3, theta=0.7, softening=1e-4, mode=abi.MODE_COLLISION)
+        for _ in range(2):
+            sim.step(p)
+        results.append(sim.read_bodies()[:live].view(np.uint32).copy())
+        assert sim.read_stats().error_word == 0
+        sim.close()
+    for r in results[1:]:
+        assert np.array_equal(r, results[0])
