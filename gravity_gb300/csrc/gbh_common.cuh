@@ -279,10 +279,12 @@ __device__ __forceinline__ uint32_t atomic_add_acq_rel(uint32_t* p, uint32_t v) 
     return old;
 }
 
-// 1/sqrt(x) and log2(x) as the hardware gives them, one instruction each.
-// rsqrtf and __log2f are the same instruction between a test and two
-// multiplications for subnormal x, so for x that is not subnormal (NaN,
-// infinities and negative x included) the results are the same bits.
+// 1/sqrt(x) and log2(x) by one PTX instruction each, for x that is not
+// subnormal: the .ftz forms take a subnormal x as a zero of its sign.  The PTX
+// ISA bounds rsqrt.approx's relative error by 2^-22.9 and lg2.approx's error by
+// 2^-22, absolute for x in (0.5, 2) and relative elsewhere.  For every x that is
+// not subnormal they return the bits of rsqrtf and __log2f
+// (tests/test_gpu_rsqrt_bits.py compares all of them).
 __device__ __forceinline__ float rsqrt_normal(float x) {
     float y;
     asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
