@@ -39,6 +39,7 @@
 #define GW_LIST 64
 #define GW_QUEUE 64  // queued band candidates per warp: a full MLP batch + one pop
 #define GW_BPL (GBH_GROUP_MAX / 32)  // bodies per lane
+#define GW_SATURATED 0x80000000u     // of a walk's count of opened nodes: its stack was full (a flag of its own spills)
 
 // FORM: the arithmetic form and the step's extra work, fixed per instance so
 // that the common case keeps its registers: FORM_FP32, FORM_PREC (precision
@@ -250,7 +251,6 @@ __global__ __launch_bounds__(GroupShape<MODE>::threads, GroupMinBlocks<MODE, FOR
     }
     uint32_t inter = 0, evals = 0, opened = 0;
     uint32_t sp = 0, ln = 0, np = 0;
-    bool saturated = false;
     if (n > 1) {
         // the group's start list when it has one (k_group_paths: its own
         // subtree, then the siblings of its ancestors), else the root.  The
@@ -444,7 +444,7 @@ __global__ __launch_bounds__(GroupShape<MODE>::threads, GroupMinBlocks<MODE, FOR
         uint32_t bo = __ballot_sync(0xffffffffu, kind == 2);
         if (sp + 2 * __popc(bo) > (uint32_t)Cfg::stack) {
             // frontier full: accept instead of opening (less accurate, never wrong)
-            saturated = true;
+            opened |= GW_SATURATED;
             if (kind == 2) kind = 1;
             bo = 0;
         }
@@ -606,13 +606,13 @@ __global__ __launch_bounds__(GroupShape<MODE>::threads, GroupMinBlocks<MODE, FOR
         }
         commit(kind, id, cm, ca, cb, lo);
     }
-    (void)saturated;
 
     // counters: interactions count the group's bodies for every list entry
     if (lane == 0) {
+        if (opened & GW_SATURATED) atomicAdd(&b.st->frontier_saturated, 1u);
         atomicAdd(&b.st->interactions, (unsigned long long)inter * grp.y);
         atomicAdd(&b.st->mac_evals, (unsigned long long)evals);
-        atomicAdd(&b.st->opened, (unsigned long long)opened);
+        atomicAdd(&b.st->opened, (unsigned long long)(opened & ~GW_SATURATED));
     }
 #pragma unroll
     for (int q = 0; q < GW_BPL; ++q) {
