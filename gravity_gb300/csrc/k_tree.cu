@@ -336,7 +336,8 @@ __device__ __forceinline__ WalkRec make_rec(const NodeVals& v, uint32_t id, uint
 // a quotient within one unit in the last place, corrected by its exact
 // remainder times the correctly rounded reciprocal, rounds as a / m does.  The
 // first correction brings the product a inv within that unit, the second
-// applies the theorem.  Holds where no remainder underflows: see div3.
+// applies the theorem.  Holds where the quotient is a normal number away from
+// the largest and no remainder underflows: see div3.
 __device__ __forceinline__ float div_by(float a, float m, float inv) {
     float q = a * inv;
     q = __fmaf_rn(__fmaf_rn(-q, m, a), inv, q);
@@ -352,9 +353,13 @@ __device__ __noinline__ float3 div3_slow(float x, float y, float z, float m) {
 // divisions take most of its instructions.
 __device__ __forceinline__ void div3(float x, float y, float z, float m, float inv, float4& out) {
     const float lo = fminf(fabsf(x), fminf(fabsf(y), fabsf(z))), hi = fmaxf(fabsf(x), fmaxf(fabsf(y), fabsf(z)));
-    // numerators in [2^-80, 2^80] and m in [2^-60, 2^60]: quotients and
-    // remainders (above 2^-128) stay normal; NaN and zeros divide below
-    if (lo >= 8.2718061e-25f && hi <= 1.2089258e24f && m >= 8.6736174e-19f && m <= 1.1529215e18f) {
+    // numerators in [2^-80, 2^80] and m in [2^-60, 2^60]: remainders (above
+    // 2^-128) stay normal; quotients in [2^-125, 2^126] by the bounds with m,
+    // which are exact where they decide (a subnormal quotient is rounded twice,
+    // and beside the largest number a inv overflows first).  NaN and zeros
+    // divide below.
+    if (lo >= 8.2718061e-25f && hi <= 1.2089258e24f && m >= 8.6736174e-19f && m <= 1.1529215e18f &&
+        lo >= m * 2.3509887e-38f && hi <= m * 8.5070592e37f) {
         out.x = div_by(x, m, inv);
         out.y = div_by(y, m, inv);
         out.z = div_by(z, m, inv);
