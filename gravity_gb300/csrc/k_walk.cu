@@ -56,8 +56,9 @@
 #define PW_THREADS 128
 #define PW_WARPS (PW_THREADS / 32)
 #define PW_LIST 64     // below 32 entries wait, one append adds up to 32
-#define PW_LOW 120     // above this many stack entries the walk turns depth-first
-#define PW_STACK 288   // PW_LOW + 63 (one batch) + 96 (a depth-first descent: 63 key + 30 tie-break levels)
+#define PW_STACK 288
+#define PW_BATCH 64    // what one batch can add: 16 opened nodes and the undecided ones that wait (31)
+#define PW_LEVELS 96   // the tallest tree: 63 key and 32 tie-break levels
 
 enum PlainForm { PF_FP32 = 0, PF_PREC = 1, PF_MERGE = 2 };
 
@@ -178,6 +179,9 @@ __global__ __launch_bounds__(PW_THREADS, PlainBlocks<FORM>::value) void k_walk_p
     uint32_t inter = 0, opened = 0;  // this lane's share of the warp's counts
     uint32_t sp = 0, max_sp = 0, an = 0, xn = 0, ln = 0;
     bool overflow = false;
+    // above this many stack entries the walk turns depth-first: what is left holds
+    // one batch and then the descent through a tree of this height
+    const uint32_t low_at = PW_STACK - PW_BATCH - min(b.st->tree_height + 1u, (uint32_t)PW_LEVELS);
     // a candidate of this lane was not finite (or far out of range), or the
     // softening does not keep the squared distances normal numbers
     bool wild = !boxed || soft < GBH_MIN_NORMAL;
@@ -479,12 +483,15 @@ __global__ __launch_bounds__(PW_THREADS, PlainBlocks<FORM>::value) void k_walk_p
         }
         if (end) break;
         // the undecided nodes when a full batch waits, when the stack is empty
-        // (the opened ones refill it) and, above PW_LOW entries, always: the
+        // (the opened ones refill it) and, above low_at entries, always: the
         // walk then takes one node at a time, depth-first, so the stack holds
-        // what a tree of any height needs.  Testing them earlier, from 8 to 24
+        // what the tree needs.  With one line for every tree, 120 entries, walks
+        // at thetas below 0.05 ran depth-first most of the time (65,536-body
+        // Plummer sphere at theta 0.005 and 0.02: 32.6 and 24.7 ms, now 15.1 and
+        // 10.0).  Testing them earlier, from 8 to 24
         // waiting ones at 8 to 48 stack entries, changed nothing (3.26 to 3.29
         // ms).
-        const bool low = sp > PW_LOW;
+        const bool low = sp > low_at;
         if (xn && (xn >= 32 || sp == 0 || low)) {
             __syncwarp();
             const uint32_t cnt = min(xn, 32u);
