@@ -167,10 +167,14 @@ __global__ __launch_bounds__(PW_THREADS, PlainBlocks<FORM>::value) void k_walk_p
         mxz = mxz + pad;
     }
     const bool boxed = !__any_sync(0xffffffffu, active && !(finite3(pm.x, pm.y, pm.z) && finite3(lo_b.x, lo_b.y, lo_b.z))) &&
-                       theta >= 1e-3f && theta <= 1e3f && soft >= 0.0f && soft <= 1e30f;
+                       (theta >= 1e-18f || theta == 0.0f) && theta <= 1e3f && soft >= 0.0f && soft <= 1e30f;
     // theta^2 with margins of 1e-5: the body's own test (a reciprocal square
     // root of at most 2 ulp error and six more roundings, together below 1e-6)
-    // decides the same way wherever the box test decides
+    // decides the same way wherever the box test decides.  Holds down to 1e-18,
+    // where theta^2 is still a normal number; theta 0 (the exact sum) opens
+    // everything.  With thetas below 1e-3 left to the tests body by body, theta 0
+    // took 9.9 ms at 16,384 bodies and 43.2 at 65,536 (Plummer spheres), now 1.0 and
+    // 6.6.
     const float t2_accept = theta * theta * 0.99999f, t2_open = theta * theta * 1.00001f;
 
     float ax = 0.0f, ay = 0.0f, az = 0.0f, pot = 0.0f;
@@ -486,9 +490,9 @@ __global__ __launch_bounds__(PW_THREADS, PlainBlocks<FORM>::value) void k_walk_p
         // (the opened ones refill it) and, above low_at entries, always: the
         // walk then takes one node at a time, depth-first, so the stack holds
         // what the tree needs.  With one line for every tree, 120 entries, walks
-        // at thetas below 0.05 ran depth-first most of the time (65,536-body
-        // Plummer sphere at theta 0.005 and 0.02: 32.6 and 24.7 ms, now 15.1 and
-        // 10.0).  Testing them earlier, from 8 to 24
+        // at thetas from 0 to 0.05 ran depth-first most of the time (65,536-body
+        // Plummer sphere at theta 0, 0.005 and 0.02: 13.0, 32.6 and 24.7 ms, now
+        // 6.6, 15.1 and 10.0).  Testing them earlier, from 8 to 24
         // waiting ones at 8 to 48 stack entries, changed nothing (3.26 to 3.29
         // ms).
         const bool low = sp > low_at;
