@@ -12,7 +12,6 @@
 
 #define GBH_NONE 0xFFFFFFFFu
 #define GBH_WARP 32
-#define GBH_WALK_STACK 192     // per-warp walk stack entries (tree height + 1 needed)
 #ifndef GBH_GROUP_MAX
 #define GBH_GROUP_MAX 96       // bodies per group of the group walk (one warp, three per lane)
 #endif

@@ -51,10 +51,12 @@ extern "C" {
 /* ---- device error word bits (gbh_stats.error_word) ------------------------ */
 #define GBH_DEVERR_SORT_LOOKBACK 0x1u   /* onesweep look-back spin gave up (bounded wait) */
 #define GBH_DEVERR_FILL_SPIN 0x2u       /* bottom-up fill: reserved, no longer raised */
-#define GBH_DEVERR_WALK_STACK 0x4u      /* a tree walk needed more stack than GBH_WALK_STACK */
+#define GBH_DEVERR_WALK_STACK 0x4u      /* a walk's stack was full: 288 entries per warp in the plain walk, 128 in
+                                         collision mode (trees have up to 96 levels: neither happens) */
 #define GBH_DEVERR_MERGE_OVERFLOW 0x8u  /* merge resolution did not finish (cannot happen: each round runs a task) */
 #define GBH_DEVERR_TREE_HEIGHT 0x10u    /* tree height above 64 (the reference fills only 64 levels) */
-#define GBH_DEVERR_MAC_FRONTIER 0x20u   /* learned walk frontier overflow */
+#define GBH_DEVERR_MAC_FRONTIER 0x20u   /* reserved, never raised (a full stack of a group walk
+                                         counts in gbh_stats.frontier_saturated) */
 
 /* ---- enums mirroring the reference uniforms ------------------------------ */
 /* mergingCollisionOrNeither (common.glsl:133-140, defaultProperties.json order) */
@@ -175,7 +177,9 @@ typedef struct gbh_stats {
     uint32_t merge_conflicts;/* tasks that shared a body with another task */
     uint32_t out_of_bounds;  /* bodies killed out of bounds in this step */
     uint32_t tree_height;    /* height of the root */
-    uint32_t max_stack;      /* deepest walk stack seen */
+    uint32_t max_stack;      /* most nodes on a warp's stack, plus one.  Plain walk: nodes opened and
+                                waiting, whole batches of them (not the tree's depth); collision
+                                mode: the depth-first stack; 0 after a group or learned walk */
     uint32_t error_word;     /* GBH_DEVERR_* bits, sticky until gbh_clear_error */
     uint32_t frontier_saturated; /* group walks whose candidate stack filled up: nodes were
                                     accepted instead of opened (less accurate, still a valid sum) */
