@@ -39,7 +39,7 @@
 template <int ITEMS, int THREADS>
 struct SortSmem {
     uint16_t warp_hist[THREADS / 32][SORT_RADIX + 2];  // [SORT_RADIX]: sentinel bucket of out-of-range items
-    uint32_t block_excl[SORT_RADIX + 1];
+    uint32_t block_excl[SORT_RADIX];
     uint32_t delta[SORT_RADIX];
     uint2 warp_tot[SORT_RADIX / 32];
     uint32_t tile;
@@ -161,7 +161,6 @@ __global__ __launch_bounds__(THREADS, SortBlocks<ITEMS, THREADS>::value) void k_
         }
         bucket_base += y - digit_count;
         S.block_excl[d] = off + x - total;
-        if (d == 0) S.block_excl[SORT_RADIX] = 0;
     }
     __syncthreads();
     // stage digit-ordered in shared memory (tile-local offsets only), before

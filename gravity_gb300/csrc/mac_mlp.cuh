@@ -46,7 +46,6 @@
 //   chunk 6   w3                        chunk 11   b3 (word 0)
 #define MAC_FRAG_CHUNKS 12
 #define MAC_SMEM_FRAG_WORDS (MAC_FRAG_CHUNKS * 4 * 32)
-#define MAC_WALK_WARPS 8
 // the learned walk's default band: nodes that pass the group rule at
 // MAC_BAND_LO are accepted, nodes that fail it at MAC_BAND_HI opened
 #define MAC_BAND_LO 0.25f
