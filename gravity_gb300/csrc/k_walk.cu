@@ -774,7 +774,10 @@ static uint32_t bodies_per_warp(uint32_t n) { return n <= 4096u ? 4u : n <= 8192
 // theta 0.7: 1,024 bodies 39, 31, 27, 21; 8,192 51, 39, 35, 31; 16,384 55, 41, 35,
 // 35; 32,768 59, 47, 47, 59; 65,536 68, 61, 78, 96; 100,003 72, 80, 98, 139.  Steps
 // with three contexts in flight: 1,024 bodies 34.1 -> 26.9 us, 8,192 56.0 -> 48.3,
-// 16,384 59.0 -> 53.6, 32,768 65.0 -> 62.2.
+// 16,384 59.0 -> 53.6, 32,768 65.0 -> 62.2.  With 32 and 16 per warp, in flight
+// (alone): 40,000 bodies 63.8 (181) and 62.4 us (172), 65,536 79.8 (201) and 81.2
+// (193), 100,003 92.7 (214) and 109.2 (221): the two cross between 40,000 and
+// 65,536 bodies in flight, and above 65,536 alone.
 static uint32_t collide_per_warp(uint32_t n) {
     return n <= 8192u ? 4u : n <= 16384u ? 8u : n <= 32768u ? 16u : 32u;
 }

@@ -8,9 +8,9 @@
 //     lane evaluates the acceptance criterion of the group against its node;
 //   * accepted nodes and leaves are appended to an interaction list, opened
 //     nodes push their two children;
-//   * every 32 list entries, all lanes accumulate the forces of the whole
-//     list on their own bodies (dense FMA loop, node data broadcast from
-//     shared memory).
+//   * when 32 or more entries wait, all lanes accumulate the forces of the
+//     whole list (at most 63) on their own bodies (dense FMA loop, node data
+//     broadcast from shared memory).
 // Criteria (gbh_step_params.mac_mode):
 //   GBH_MAC_GROUP    accept when the boxes are disjoint and half_side < theta *
 //                    sqrt(d^2 + softening), d = max(|com - c_g| - R_g, 0), with
@@ -28,7 +28,7 @@
 // once, and each warp takes its next group from a ticket counter when it has
 // finished the last, so warps that meet short walks are not left idle while
 // the rest of their block finishes long ones.
-// Only gravity (merging_collision_or_neither == 0) runs here.
+// Gravity and merges run here; collision mode does not.
 #include <cstddef>
 #include <type_traits>
 
@@ -359,7 +359,8 @@ __global__ __launch_bounds__(GroupShape<MODE>::threads, GroupMinBlocks<MODE, FOR
             // Two entries per packed instruction, four per iteration; a partial
             // list is padded with massless copies of its first entry.  A packed
             // instruction occupies the FMA pipe for two cycles, so the loop's
-            // bound stays (63% of the pipe's cycles in the group-theta walk),
+            // bound stays (65% of the pipe's cycles in the group-theta walk of
+            // 2,000,003 bodies),
             // but it takes 14 issue slots per two entries where single
             // instructions take 26.  One loop per slot reads the list once per
             // slot: 7.59 against 7.35 ms (16.8M mixture, learned), and two
