@@ -295,7 +295,7 @@ PLAIN_THETAS = [0.3, 0.5, 0.7]
 # DRAM bytes per body of one learned-walk launch: ncu dram__bytes_read.sum +
 # dram__bytes_write.sum of k_walk_group<1> on the 4,194,304-body mixture,
 # divided by its bodies; the walk's traffic grows in proportion to the bodies
-WALK_LEARNED_DRAM_BYTES_PER_BODY = 289.5
+WALK_LEARNED_DRAM_BYTES_PER_BODY = 289.9
 
 
 def timed_steps(bh, p, steps, warmup, stream, dist, local, clocks=None):
