@@ -778,33 +778,6 @@ __device__ __forceinline__ void store_above(const StepBuffers& b, const AboveNod
     }
 }
 
-// Rounds over a list of any length, values and flags in global memory: lists
-// longer than a block has threads (trees far from the usual shapes).  The
-// block's barriers order a node's words and flag before the rounds that read
-// them.
-__device__ void fill_long_list(const StepBuffers& b, const uint32_t* list, uint32_t m, uint32_t floor) {
-    volatile uint32_t* flags = b.fill_ready;  // the round that finished the node
-    for (uint32_t k = threadIdx.x; k < m; k += blockDim.x) flags[list[k]] = 0u;
-    __syncthreads();
-    for (uint32_t round = 1;; ++round) {
-        bool progress = false;
-        for (uint32_t k = threadIdx.x; k < m; k += blockDim.x) {
-            const uint32_t i = list[k];
-            if (flags[i]) continue;
-            const AboveNode a = above_node(b, i);
-            const uint32_t fa = a.left > floor ? flags[a.kids.x - b.N] : 0u, fb = a.right > floor ? flags[a.kids.y - b.N] : 0u;
-            if ((a.left > floor && !(fa && fa < round)) || (a.right > floor && !(fb && fb < round))) continue;
-            const NodeVals L = load_child(b, a.kids.x), R = load_child(b, a.kids.y);
-            store_above(b, a, combine(L, R), L, R);
-            flags[i] = round;
-            progress = true;
-        }
-        if (!__syncthreads_or(progress)) return;
-    }
-}
-
-// The nodes of one list (more than `floor` bodies each, their smaller children
-// finished), a thread each.
 template <int THREADS>
 struct AboveSmem {
     float4 cm[THREADS], box03[THREADS], box45[THREADS], col[THREADS];  // finished nodes' values
@@ -813,6 +786,57 @@ struct AboveSmem {
     uint32_t count;
 };
 
+// A list longer than the block has threads (trees far from the usual shapes: long
+// chains).  A thread starts at every node with no child in the list and climbs, up
+// to the last node of at most `most` bodies: where the other child is not in the
+// list its words are there already, and the climb goes straight on; where it is,
+// the second to arrive goes on (`fill_ready`, as in climb_global).  The starts hold
+// more than `floor` bodies each and are disjoint, so there are fewer than THREADS.
+// A level takes one round trip to L2, the next node's words loaded beside the
+// arithmetic.  Steps of 56,800 and 113,600 bodies in clumps with chains along the
+// axes (46 nodes above the groups per 142 bodies), us: a climb from every group of
+// the state 296 and 318, rounds over the list 418 and 446, this 221 and 245.
+template <int THREADS>
+__device__ __noinline__ void fill_long_list(const StepBuffers& b, AboveSmem<THREADS>& S, const uint32_t* list,
+                                            uint32_t m, uint32_t floor, uint32_t most) {
+    const uint32_t t = threadIdx.x;
+    __syncthreads();  // every thread has read the count
+    if (t == 0) S.count = 0;
+    __syncthreads();
+    for (uint32_t k = t; k < m; k += THREADS) {
+        const AboveNode a = above_node(b, list[k]);
+        b.fill_ready[a.id] = 0u;
+        if (a.left > floor || a.right > floor) continue;
+        const uint32_t at = atomicAdd(&S.count, 1u);
+        if (at < THREADS) S.ids[at] = a.id;
+    }
+    __syncthreads();
+    const uint32_t start = t % 32 * (THREADS / 32) + t / 32;  // over all warps
+    if (start >= S.count) return;
+    AboveNode a = above_node(b, S.ids[start]);
+    NodeVals L = load_child(b, a.kids.x), R = load_child(b, a.kids.y);
+    for (;;) {
+        // the next node, and its other child's words if they are there, beside this one
+        const bool top = a.parent == GBH_NONE;
+        const AboveNode up = top ? a : above_node(b, a.parent - b.N);
+        const bool is_left = up.kids.x == a.id + b.N;
+        const uint32_t other = is_left ? up.kids.y : up.kids.x;
+        const gbh_node* words = other < b.N ? &b.leaf[other] : &b.internal[other - b.N];
+        const bool last = top || up.bodies > most, meets = (is_left ? up.right : up.left) > floor;
+        NodeVals v;
+        if (!last && !meets) v = load_node_cg(words);
+        const NodeVals out = combine(L, R);
+        store_above(b, a, out, L, R);
+        if (last || (meets && atomic_add_acq_rel(&b.fill_ready[up.id], 1u) == 0u)) return;
+        if (meets) v = load_node_cg(words);
+        L = is_left ? out : v;
+        R = is_left ? v : out;
+        a = up;
+    }
+}
+
+// The nodes of one list (more than `floor` bodies each, their smaller children
+// finished), a thread each.
 template <int THREADS>
 __device__ void fill_list(const StepBuffers& b, AboveSmem<THREADS>& S, uint32_t m, uint32_t floor) {
     const uint32_t t = threadIdx.x;
@@ -889,14 +913,14 @@ __device__ void fill_list(const StepBuffers& b, AboveSmem<THREADS>& S, uint32_t 
 // 268.9.  A level between with subtrees of 131,072 bodies costs 35 us for the
 // scan that finds its nodes.
 template <int THREADS, bool LISTED>
-__global__ __launch_bounds__(THREADS) void k_fill_above(StepBuffers b) {
+__global__ __launch_bounds__(THREADS, LISTED ? 1 : 4) void k_fill_above(StepBuffers b) {
     extern __shared__ __align__(16) unsigned char fill_smem[];
     AboveSmem<THREADS>& S = *reinterpret_cast<AboveSmem<THREADS>*>(fill_smem);
     const uint32_t n = b.st->n_new;
     if (LISTED) {
         const uint32_t m = b.st->num_subtrees[1];
         if (m > THREADS) {
-            fill_long_list(b, b.fill_subtrees[1], m, FILL_SUBTREE);
+            fill_long_list(b, S, b.fill_subtrees[1], m, FILL_SUBTREE, ~0u);
         } else {
             if (threadIdx.x < m) S.ids[threadIdx.x] = b.fill_subtrees[1][threadIdx.x];
             fill_list<THREADS>(b, S, m, FILL_SUBTREE);
@@ -927,7 +951,7 @@ __global__ __launch_bounds__(THREADS) void k_fill_above(StepBuffers b) {
         __syncthreads();
         const uint32_t m = S.count;
         if (m > THREADS)
-            fill_long_list(b, list, m, GBH_GROUP_MAX);
+            fill_long_list(b, S, list, m, GBH_GROUP_MAX, bodies);
         else
             fill_list<THREADS>(b, S, m, GBH_GROUP_MAX);
     }
